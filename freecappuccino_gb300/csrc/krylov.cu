@@ -14,15 +14,17 @@
 //  * One sweep is a fixed chain of kernels captured once into the body of a CUDA-graph
 //    WHILE node; the kernel that evaluates the stop test clears the node's condition.
 //    A whole solve is one graph launch.
-//  * The DIC/DILU triangular solves run level by level (rows of one level depend only
-//    on rows of earlier levels), one kernel per level inside the same graph; each row
-//    is computed with the reference's operand order, so the preconditioner is the
-//    reference's M = (D+L) D^-1 (D+U) exactly.
-// Deviations kept on purpose (FP64 division is slow on this part; each differs from the
-// reference's division by at most one ulp per entry): DPCG's z = r / a(diag) is computed
-// as r * (1/a(diag)), and the rescale zk/(d+small) between the DIC/DILU sweeps
-// (iccg.f90:102) as zk * (1/(d+small)), the reciprocal formed once per solve with the
-// factor.
+//  * The DIC/DILU triangular solves run in one launch each: on a lexicographic hex block
+//    as wavefront-tiled sweeps (wave_sweep.cuh), elsewhere with rows waiting on the rows
+//    they read; one launch per level (rows of one level depend only on rows of earlier
+//    levels) is kept behind FCG_SWEEP=levels.  Each row takes its entries in the
+//    reference's order: the reference's M = (D+L) D^-1 (D+U).
+// Deviations kept on purpose (FP64 division is slow on this part and every FP64
+// operation of a sweep lengthens its chain of dependent rows): DPCG's z = r / a(diag) is
+// computed as r * (1/a(diag)); a sweep's row (b - sum a_k z_k) d as b d - sum (a_k d) z_k
+// with fused multiply-adds; the rescale zk/(d+small) between the sweeps (iccg.f90:102)
+// as a product with d/(d+small), formed once per solve with the factor.  Each rounds an
+// entry by at most an ulp differently.
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
@@ -32,6 +34,7 @@
 #include "fcg_internal.h"
 #include "krylov_common.cuh"
 #include "launch.h"
+#include "wave_sweep.cuh"
 
 namespace fcg {
 
@@ -69,11 +72,11 @@ struct KrylovState {
   double *x = nullptr, *res = nullptr, *su = nullptr, *pk = nullptr, *zk = nullptr,
          *qk = nullptr, *invd = nullptr, *d = nullptr, *reso = nullptr, *uk = nullptr,
          *vk = nullptr, *a = nullptr, *sval = nullptr, *partials = nullptr, *rtmp = nullptr;
-  double *rdi = nullptr;  // 1/(d + small), the backward sweep's rescale (with the factor)
-  // coefficient planes of the wavefront-tiled sweeps on a hex block: lower entries in
-  // the order -nx ny, -nx, -1 and upper entries in the order +1, +nx, +nx ny, [3][n] each
-  DBuf wcoef;
-  double *wlo = nullptr, *wup = nullptr;
+  double *rdi = nullptr;  // d/(d + small), the backward sweep's rescale (with the factor)
+  // records and vectors of the wavefront-tiled sweeps on a hex block (wave_sweep.cuh),
+  // made at the first solve that sweeps
+  DBuf wbuf;
+  wave::Arrays<double> wv{};
   DBuf trace;
   // mixed precision: FP32 copy of D^-1/2 A D^-1/2 in the sliced layout, the scaling
   // D^-1/2 in FP64 and the FP32 inner vectors (correction y, residual r, direction p, Ap)
@@ -102,7 +105,6 @@ struct KrylovState {
   int sf_spin = 1 << 20;     // polls before a dependency wait gives up
   int sf_absent_row = -1;    // test hook: this row never publishes its flag
   bool wave_on = true;       // wavefront-tiled sweeps on lexicographic hex blocks
-  bool wave_wide = true;     // tiles of 16 x 8 columns rather than 8 x 8
 };
 
 void destroy_krylov(KrylovState *k) {
@@ -117,7 +119,7 @@ void destroy_krylov(KrylovState *k) {
   if (k->hS) cudaFreeHost(k->hS);
   if (k->S) cudaFree(k->S);
   k->vec.release();
-  k->wcoef.release();
+  k->wbuf.release();
   k->trace.release();
   k->mixed.release();
   k->sfb.release();
@@ -347,10 +349,10 @@ __global__ void __launch_bounds__(kTPB, 8) k_cg_dot(int n, const double *__restr
 }
 
 // --- triangular sweeps, one launch per level -----------------------------------
-// The row arithmetic of the sweeps and factors is written with __dmul_rn / __dsub_rn: a
-// multiply and a subtract each rounded, as the reference's loops evaluate them, and the
-// same bits whichever kernel form (per level or one launch) runs it.
-// forward: z_i = (b_i - sum_{k<diag} a_k z_{ja_k}) * d_i        (iccg.f90:248-254)
+// The row arithmetic is explicit -- the sweeps' coefficient a_k d_i rounded, then a fused
+// multiply-add per entry; the factors' products and differences each rounded -- so that
+// every kernel form (per level, one launch, wavefront tiles) gives the same bits.
+// forward: z_i = b_i d_i - sum_{k<diag} (a_k d_i) z_{ja_k}        (iccg.f90:248-254)
 __global__ void k_fwd_level(const int *__restrict__ rows, int count,
                             const int *__restrict__ ioffset, const int *__restrict__ ja,
                             const int *__restrict__ diag, const double *__restrict__ a,
@@ -360,13 +362,14 @@ __global__ void k_fwd_level(const int *__restrict__ rows, int count,
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= count) return;
   int i = rows[t];
-  double zi = b[i];
-  for (int k = ioffset[i]; k < diag[i]; ++k) zi = __dsub_rn(zi, __dmul_rn(a[k], z[ja[k]]));
-  z[i] = zi * d[i];
+  const double di = d[i];
+  double zi = b[i] * di;
+  for (int k = ioffset[i]; k < diag[i]; ++k) zi = __fma_rn(-(a[k] * di), z[ja[k]], zi);
+  z[i] = zi;
 }
 
 // backward with the reference's rescale zk/(d+small) folded in (iccg.f90:256-265), as a
-// product with rdi = 1/(d+small).
+// product with rdi = d/(d+small): z_i = y_i rdi_i - sum_{k>diag} (a_k d_i) z_{ja_k}.
 __global__ void k_bwd_level(const int *__restrict__ rows, int count,
                             const int *__restrict__ ioffset, const int *__restrict__ ja,
                             const int *__restrict__ diag, const double *__restrict__ a,
@@ -378,8 +381,8 @@ __global__ void k_bwd_level(const int *__restrict__ rows, int count,
   int i = rows[t];
   double di = d[i];
   double zi = z[i] * rdi[i];
-  for (int k = diag[i] + 1; k < ioffset[i + 1]; ++k) zi = __dsub_rn(zi, __dmul_rn(a[k], z[ja[k]]));
-  z[i] = zi * di;
+  for (int k = diag[i] + 1; k < ioffset[i + 1]; ++k) zi = __fma_rn(-(a[k] * di), z[ja[k]], zi);
+  z[i] = zi;
 }
 
 // --- sync-free triangular sweeps ---------------------------------------------------
@@ -451,8 +454,8 @@ __global__ void k_sf_fill(int n, double *__restrict__ o1, double *__restrict__ o
   }
 }
 
-// One row: acc - sum a_k v_{ja_k} over k in [k0, hi), the values awaited in batches.
-__device__ __forceinline__ double sf_row(double acc, int k0, int hi, const int *__restrict__ ja,
+// One row: acc - sum (a_k di) v_{ja_k} over k in [k0, hi), the values awaited in batches.
+__device__ __forceinline__ double sf_row(double acc, double di, int k0, int hi, const int *__restrict__ ja,
                                          const double *__restrict__ a, const double *v, int *ctl,
                                          Scal *S, int spin) {
   for (; k0 < hi; k0 += kSfBatch) {
@@ -474,12 +477,12 @@ __device__ __forceinline__ double sf_row(double acc, int k0, int hi, const int *
     if (!ok) sf_fail(&ctl[3], S);
 #pragma unroll
     for (int t = 0; t < kSfBatch; ++t)
-      if (k0 + t < hi) acc = __dsub_rn(acc, __dmul_rn(aa[t], vv[t]));
+      if (k0 + t < hi) acc = __fma_rn(-(aa[t] * di), vv[t], acc);
   }
   return acc;
 }
 
-// forward: y_i = (b_i - sum_{k<diag} a_k y_{ja_k}) * d_i        (iccg.f90:248-254)
+// forward: y_i = b_i d_i - sum_{k<diag} (a_k d_i) y_{ja_k}        (iccg.f90:248-254)
 __global__ void k_fwd_sf(const int *__restrict__ rows, int len, const int *__restrict__ ioffset,
                          const int *__restrict__ ja, const int *__restrict__ diag,
                          const double *__restrict__ a, const double *__restrict__ d,
@@ -494,14 +497,13 @@ __global__ void k_fwd_sf(const int *__restrict__ rows, int len, const int *__res
     if (base >= len) break;
     const int i = rows[base + lane];
     if (i < 0 || i == absent) continue;
-    const double zi = sf_row(b[i], ioffset[i], diag[i], ja, a, y, ctl, S, spin);
-    st_relaxed64(&y[i], zi * d[i]);
+    const double di = d[i];
+    st_relaxed64(&y[i], sf_row(b[i] * di, di, ioffset[i], diag[i], ja, a, y, ctl, S, spin));
   }
 }
 
 // backward from the forward result y with the reference's rescale zk/(d+small) folded
-// in (iccg.f90:256-265): z_i = (y_i rdi_i - sum_{k>diag} a_k z_{ja_k}) * d_i,
-// rdi = 1/(d+small)
+// in (iccg.f90:256-265): z_i = y_i rdi_i - sum_{k>diag} (a_k d_i) z_{ja_k}, rdi = d/(d+small)
 __global__ void k_bwd_sf(const int *__restrict__ rows, int len, const int *__restrict__ ioffset,
                          const int *__restrict__ ja, const int *__restrict__ diag,
                          const double *__restrict__ a, const double *__restrict__ d,
@@ -517,8 +519,8 @@ __global__ void k_bwd_sf(const int *__restrict__ rows, int len, const int *__res
     const int i = rows[base + lane];
     if (i < 0) continue;
     const double di = d[i];
-    const double zi = sf_row(y[i] * rdi[i], diag[i] + 1, ioffset[i + 1], ja, a, z, ctl, S, spin);
-    st_relaxed64(&z[i], zi * di);
+    st_relaxed64(&z[i], sf_row(y[i] * rdi[i], di, diag[i] + 1, ioffset[i + 1], ja, a, z, ctl, S,
+                               spin));
   }
 }
 
@@ -548,7 +550,7 @@ __global__ void k_factor_sf(const int *__restrict__ rows, int len, const int *__
     if (!ok) sf_fail(&ctl[3], S);
     const double inv = 1.0 / di;
     st_relaxed64(&d[i], inv);
-    rdi[i] = 1.0 / (inv + S->small);
+    rdi[i] = inv / (inv + S->small);
     if (!isfinite(inv) || di == 0.0) fail_status(S, FCG_ERR_PIVOT);
   }
 }
@@ -574,25 +576,16 @@ __global__ void k_factor_level(const int *__restrict__ rows, int count,
   }
   double inv = 1.0 / di;
   d[i] = inv;
-  rdi[i] = 1.0 / (inv + S->small);
+  rdi[i] = inv / (inv + S->small);
   if (!isfinite(inv) || di == 0.0) fail_status(S, FCG_ERR_PIVOT);
 }
 
-// --- wavefront-tiled sweeps on a lexicographic hex block ---------------------------
-// On a mesh whose cells form an nx x ny x nz block (c->hex), the lower entries of row r are
-// (when present, in CSR order) r - nx ny, r - nx, r - 1 and the upper ones r + 1, r + nx,
-// r + nx ny.  A block of TX x TY threads owns a tile of TX x TY (i, j) columns and walks
-// the tile's cells in the order of their wavefront (i - i0) + (j - j0) + k: at local step
-// L each thread computes the cell of its column with k = L - di - dj.  The cell's
-// upstream neighbour in k is the thread's own previous cell (a register); those in i and
-// j inside the tile were computed one step earlier by the neighbouring threads (shared
-// memory, double buffered, one barrier per step).  Only the tile's first row and column
-// read cells of another tile, from global memory through the value-as-flag wait of the
-// one-launch sweeps.  The backward sweep walks from the opposite corner over the upper
-// entries.  Tiles are claimed through an atomic counter in an order in which a tile's
-// upstream tiles come first, so a block only waits for blocks that are running.  Each
-// row uses the arithmetic of the level kernels with its entries in the same order: the
-// same bits.
+// --- wavefront-tiled factor on a lexicographic hex block --------------------------
+// The tiles and steps of wave_sweep.cuh, from the CSR and in the natural order (once per
+// solve): a tile's first row and column read the cells of other tiles from global memory
+// through the value-as-flag wait of the one-launch sweeps.  Tiles are claimed in an order
+// in which a tile's upstream tiles come first.  The level kernel's arithmetic: the same
+// bits.
 template <int TX, int TY>
 struct WaveTile {
   int ntx, nty, di, dj, p, q;
@@ -601,7 +594,7 @@ struct WaveTile {
 };
 
 // Claims a tile (thread 0, broadcast); false when every tile is taken.
-template <int TX, int TY, bool BWD>
+template <int TX, int TY>
 __device__ __forceinline__ bool wave_claim(int nx, int ny, int *counter, WaveTile<TX, TY> &t) {
   __shared__ int tile_sh;
   if (threadIdx.x == 0) tile_sh = atomicAdd(counter, 1);
@@ -612,18 +605,17 @@ __device__ __forceinline__ bool wave_claim(int nx, int ny, int *counter, WaveTil
   if (tile >= t.ntx * t.nty) return false;
   t.di = threadIdx.x % TX;
   t.dj = threadIdx.x / TX;
-  t.p = (tile % t.ntx) * TX + t.di;  // column, counted from the sweep's start corner
+  t.p = (tile % t.ntx) * TX + t.di;
   t.q = (tile / t.ntx) * TY + t.dj;
   t.col_ok = t.p < nx && t.q < ny;
-  const int i = BWD ? nx - 1 - t.p : t.p, j = BWD ? ny - 1 - t.q : t.q;
-  t.col0 = i + (long long)nx * j;
-  t.step_i = BWD ? 1 : -1;
-  t.step_j = BWD ? nx : -nx;
+  t.col0 = t.p + (long long)nx * t.q;
+  t.step_i = -1;
+  t.step_j = -nx;
   return true;
 }
 
 // DIC (DILU) factor d = 1/(a_ii - sum a_ik^2 d_k) (1/(a_ii - sum a_ik d_k a_ki)) in the
-// forward wavefront, reading the CSR directly (once per solve); also rdi = 1/(d + small).
+// forward wavefront, reading the CSR directly (once per solve); also rdi = d/(d + small).
 template <int TX, int TY, bool DILU>
 __global__ void __launch_bounds__(TX * TY)
     k_wave_factor(int nx, int ny, int nz, const int *__restrict__ ioffset,
@@ -632,7 +624,7 @@ __global__ void __launch_bounds__(TX * TY)
                   Scal *S, int spin) {
   __shared__ double sm[2][TY][TX];
   WaveTile<TX, TY> t;
-  if (!wave_claim<TX, TY, false>(nx, ny, &ctl[0], t)) return;
+  if (!wave_claim<TX, TY>(nx, ny, &ctl[0], t)) return;
   const long long nxy = (long long)nx * ny;
   const int nlev = TX + TY - 2 + nz;
   double prev = 0.0;
@@ -664,134 +656,12 @@ __global__ void __launch_bounds__(TX * TY)
       if (t.p > 0) term(vp);
       val = 1.0 / dd;
       st_relaxed64(&d[r], val);
-      rdi[r] = 1.0 / (val + S->small);
+      rdi[r] = val / (val + S->small);
       if (!isfinite(val) || dd == 0.0) fail_status(S, FCG_ERR_PIVOT);
       prev = val;
     }
     sm[L & 1][t.dj][t.di] = val;
     __syncthreads();
-  }
-}
-
-// Coefficient planes of the sweeps from the CSR values: lo[t][r] for the lower entries in
-// CSR order (-nx ny, -nx, -1) and up[t][r] for the upper ones (+1, +nx, +nx ny), 0 where the
-// row has no such entry (the sweeps skip those terms).
-__global__ void k_wave_coef(int nx, int ny, int nz, const int *__restrict__ ioffset,
-                            const int *__restrict__ diag, const double *__restrict__ a,
-                            double *__restrict__ lo, double *__restrict__ up) {
-  const long long nxy = (long long)nx * ny, n = nxy * nz;
-  FCG_GRID_STRIDE(r, n) {
-    const int i = (int)(r % nx), j = (int)((r / nx) % ny), k = (int)(r / nxy);
-    int e = ioffset[r];
-    lo[r] = k > 0 ? a[e++] : 0.0;
-    lo[n + r] = j > 0 ? a[e++] : 0.0;
-    lo[2 * n + r] = i > 0 ? a[e++] : 0.0;
-    e = diag[r] + 1;
-    up[r] = i < nx - 1 ? a[e++] : 0.0;
-    up[n + r] = j < ny - 1 ? a[e++] : 0.0;
-    up[2 * n + r] = k < nz - 1 ? a[e++] : 0.0;
-  }
-}
-
-// Forward sweep y = (b - L y) d (BWD false) or backward sweep z = (y rdi - U z) d (BWD
-// true).  The inputs of a cell (its three coefficients, right-hand side, d, rdi, and for a
-// column on the tile's first row or column the upstream value of the neighbouring tile)
-// are loaded kRing steps ahead into a register ring whose slot is the step modulo kRing,
-// so every slot index is a compile-time constant of the unrolled step loop.  An upstream
-// value that was still the sentinel when loaded is then waited for.
-//
-// The step is branch-free: a neighbour outside the block has coefficient +0 (k_wave_coef)
-// and value +0, and acc - (+0)(+0) is acc exactly, so every cell runs the same three
-// terms in CSR order and gives the bits of the level kernels.  On this part a dependent
-// FP64 operation takes about 64 cycles, so the step's length is its chain of FP64
-// operations: the term of the cell's own column (the previous step of the same thread)
-// is formed before the barrier, which leaves the two products and subtractions of the
-// in-tile neighbours and the scaling after it.
-template <int TX, int TY, bool BWD>
-__global__ void __launch_bounds__(TX * TY)
-    k_wave_sweep(int nx, int ny, int nz, const double *__restrict__ coef,
-                 const double *__restrict__ in, const double *__restrict__ d,
-                 const double *__restrict__ rdi, double *out, int *ctl, Scal *S, int spin) {
-  constexpr int kRing = 4;
-  if (solve_done(S)) return;
-  __shared__ double sm[2][TY][TX];
-  WaveTile<TX, TY> t;
-  if (!wave_claim<TX, TY, BWD>(nx, ny, &ctl[BWD ? 1 : 0], t)) return;
-  const long long nxy = (long long)nx * ny, n = nxy * nz;
-  const bool edge_q = t.q > 0 && t.dj == 0, edge_p = t.p > 0 && t.di == 0;
-  auto row_of = [&](int s) { return t.col0 + nxy * (BWD ? nz - 1 - s : s); };
-  // Only loads here: an instruction that used a loaded value would hold the warp's
-  // in-order issue until the load returned.
-  struct Cell {
-    double c0, c1, c2, x, dd, sc, eq, ep;
-  };
-  Cell ring[kRing];
-  auto load = [&](int s, Cell &cl) {
-    if (!t.col_ok || s < 0 || s >= nz) return;
-    const long long r = row_of(s);
-    cl.c0 = coef[r];
-    cl.c1 = coef[n + r];
-    cl.c2 = coef[2 * n + r];
-    cl.x = in[r];
-    cl.dd = d[r];
-    if (BWD) cl.sc = rdi[r];
-    if (edge_q) cl.eq = ld_relaxed64(&out[r + t.step_j]);
-    if (edge_p) cl.ep = ld_relaxed64(&out[r + t.step_i]);
-  };
-  // The terms of the next step's cell that do not need the neighbours' values, formed
-  // before the barrier: forward x - c0 prev (k first in CSR order); backward y rdi and the
-  // product c2 prev (k last).
-  double part = 0.0, part2 = 0.0;
-  auto own = [&](const Cell &cl, double prev) {
-    if (BWD) {
-      part = cl.x * cl.sc;
-      part2 = __dmul_rn(cl.c2, prev);
-    } else {
-      part = __dsub_rn(cl.x, __dmul_rn(cl.c0, prev));
-    }
-  };
-#pragma unroll
-  for (int u = 0; u < kRing; ++u) load(u - t.di - t.dj, ring[u]);
-  const int nlev = TX + TY - 2 + nz;
-  double prev = 0.0;  // +0: the first cell of a column has no own-column neighbour
-  own(ring[0], prev);
-  for (int L0 = 0; L0 < nlev; L0 += kRing) {
-#pragma unroll
-    for (int u = 0; u < kRing; ++u) {
-      const int L = L0 + u;
-      if (L < nlev) {  // the same for the whole block
-        const int s = L - t.di - t.dj;
-        double val = 0.0;
-        if (t.col_ok && s >= 0 && s < nz) {
-          const long long r = row_of(s);
-          const Cell cl = ring[u];
-          bool ok = true;
-          const double sq = sm[(L - 1) & 1][t.dj > 0 ? t.dj - 1 : 0][t.di];
-          const double sp = sm[(L - 1) & 1][t.dj][t.di > 0 ? t.di - 1 : 0];
-          double vq = t.dj > 0 ? sq : (edge_q ? cl.eq : 0.0);
-          double vp = t.di > 0 ? sp : (edge_p ? cl.ep : 0.0);
-          if (edge_q && is_sentinel(vq)) vq = sf_value(&out[r + t.step_j], &ctl[3], spin, &ok);
-          if (edge_p && is_sentinel(vp)) vp = sf_value(&out[r + t.step_i], &ctl[3], spin, &ok);
-          if (!ok) sf_fail(&ctl[3], S);
-          double acc;
-          if (!BWD) {  // lower entries in CSR order: k, j, i
-            acc = __dsub_rn(part, __dmul_rn(cl.c1, vq));
-            acc = __dsub_rn(acc, __dmul_rn(cl.c2, vp));
-          } else {  // upper entries in CSR order: i, j, k
-            acc = __dsub_rn(part, __dmul_rn(cl.c0, vp));
-            acc = __dsub_rn(acc, __dmul_rn(cl.c1, vq));
-            acc = __dsub_rn(acc, part2);
-          }
-          val = acc * cl.dd;
-          st_relaxed64(&out[r], val);
-          prev = val;
-        }
-        load(s + kRing, ring[u]);
-        sm[L & 1][t.dj][t.di] = val;
-        own(ring[(u + 1) % kRing], prev);
-        __syncthreads();
-      }
-    }
   }
 }
 
@@ -1170,14 +1040,8 @@ static int ensure_state(fcg_context *c, int nsw) {
     size_t total = 14 * n + (size_t)a_len(c) + (size_t)c->sell_len + 8 * (size_t)G + 64;
     FCG_CUDA_TRY(c, k->vec.ensure(total * sizeof(double)));
     FCG_CUDA_TRY(c, cudaMemset(k->vec.p, 0, total * sizeof(double)));
-    if (c->hex.ok) {
-      FCG_CUDA_TRY(c, k->wcoef.ensure(6 * n * sizeof(double)));
-      k->wlo = k->wcoef.as<double>();
-      k->wup = k->wlo + 3 * n;
-    } else {
-      k->wcoef.release();
-      k->wlo = k->wup = nullptr;
-    }
+    k->wbuf.release();
+    k->wv = wave::Arrays<double>{};
     double *p = k->vec.as<double>();
     double **vecs[] = {&k->x, &k->res, &k->su, &k->pk, &k->zk, &k->qk, &k->invd,
                        &k->d, &k->reso, &k->uk, &k->vk, &k->rtmp, &k->rdi};
@@ -1235,11 +1099,6 @@ static int ensure_state(fcg_context *c, int nsw) {
       const char *e = std::getenv("FCG_SWEEP");
       k->sf_on = !(e && std::string(e) == "levels");
       k->wave_on = !(e && (std::string(e) == "levels" || std::string(e) == "rows"));
-      // 16 x 8 tiles while 8 x 8 ones would number fewer than two per SM; FCG_WAVE_TILE
-      // (8x8 or 16x8) overrides
-      const char *wt = std::getenv("FCG_WAVE_TILE");
-      const long long t88 = (long long)((c->hex.nx + 7) / 8) * ((c->hex.ny + 7) / 8);
-      k->wave_wide = wt ? std::string(wt) == "16x8" : t88 < 2LL * c->num_sms;
       // two blocks per SM: more resident warps only poll further ahead (measured)
       k->sf_grid = std::min(k->sf_grid, c->num_sms * 2);
     }
@@ -1346,29 +1205,12 @@ const double *sliced64(const fcg_context *c) { return c->ks ? c->ks->sval : null
 // never publishes (only the row-claiming form has one).
 static bool wave_sweeps(const fcg_context *c) {
   const KrylovState *k = c->ks;
-  return k->sf_on && k->wave_on && c->hex.ok && k->wlo && k->sf_absent_row < 0;
+  return k->sf_on && k->wave_on && c->hex.ok && k->sf_absent_row < 0;
 }
 
-// Tiles of 16 x 8 or 8 x 8 columns (64 or 128 threads per block).  Measured on 20 ICCG
-// sweeps: at 128^3 (256 tiles of 8 x 8) 16 x 8 tiles are 4% faster, at 256^3 (1024 tiles of
-// 8 x 8) 8 x 8 tiles are 11% faster, where enough tiles are in flight to keep the SMs'
-// FP64 units busy.
 template <int TX, int TY>
 static int wave_tiles(const fcg_context *c) {
   return ((c->hex.nx + TX - 1) / TX) * ((c->hex.ny + TY - 1) / TY);
-}
-
-template <int TX, int TY>
-static void launch_wave_sweep(fcg_context *c, cudaStream_t st, bool forward, const double *b,
-                              double *z) {
-  KrylovState *k = c->ks;
-  const HexBlock &h = c->hex;
-  if (forward)
-    k_wave_sweep<TX, TY, false><<<wave_tiles<TX, TY>(c), TX * TY, 0, st>>>(
-        h.nx, h.ny, h.nz, k->wlo, b, k->d, k->rdi, k->sf_y, k->sf_ctl, k->S, k->sf_spin);
-  else
-    k_wave_sweep<TX, TY, true><<<wave_tiles<TX, TY>(c), TX * TY, 0, st>>>(
-        h.nx, h.ny, h.nz, k->wup, k->sf_y, k->d, k->rdi, z, k->sf_ctl, k->S, k->sf_spin);
 }
 
 template <int TX, int TY>
@@ -1385,32 +1227,33 @@ static void launch_wave_factor(fcg_context *c, bool dilu) {
         k->S, k->sf_spin);
 }
 
+// Factor, records and armed vectors of a solve with the wavefront-tiled sweeps.
+static int start_wave(fcg_context *c, bool dilu) {
+  KrylovState *k = c->ks;
+  int rc;
+  if (!k->wv.fwd && (rc = wave::allocate(c, 1, k->wbuf, k->wv))) return rc;
+  launch_wave_factor<16, 8>(c, dilu);
+  return wave::start(c, 1, c->nnz, k->a, k->d, k->rdi, 0.0, k->wv, k->sf_ctl);
+}
+
 static void launch_sweeps(fcg_context *c, cudaStream_t st, const Level &lv, bool forward,
                           const double *b, double *z) {
   KrylovState *k = c->ks;
   if (k->sf_on) {
-    const bool wave = wave_sweeps(c);
-    auto wave_launch = [&](bool fwd) {
-      if (k->wave_wide)
-        launch_wave_sweep<16, 8>(c, st, fwd, b, z);
-      else
-        launch_wave_sweep<8, 8>(c, st, fwd, b, z);
-    };
+    if (wave_sweeps(c)) {
+      wave::launch<double>(c, st, 1, forward, k->wv, b, z, k->sf_ctl, &k->S->wait_fail,
+                           &k->S->status, &k->S->done, k->sf_spin);
+      return;
+    }
     if (forward) {  // b -> sf_y, after the sentinel fill of sf_y and z
       k_sf_fill<<<grid_for(c->n, c->num_sms), kTPB, 0, st>>>(c->n, k->sf_y, z, k->sf_ctl);
-      if (wave)
-        wave_launch(true);
-      else
-        k_fwd_sf<<<k->sf_grid, kTPB, 0, st>>>(lv.pad, lv.pad_len, c->mv.ioffset, c->mv.ja,
-                                              c->mv.diag, k->a, k->d, b, k->sf_y, k->sf_ctl,
-                                              k->S, k->sf_spin, k->sf_absent_row);
+      k_fwd_sf<<<k->sf_grid, kTPB, 0, st>>>(lv.pad, lv.pad_len, c->mv.ioffset, c->mv.ja,
+                                            c->mv.diag, k->a, k->d, b, k->sf_y, k->sf_ctl, k->S,
+                                            k->sf_spin, k->sf_absent_row);
     } else {  // sf_y -> z
-      if (wave)
-        wave_launch(false);
-      else
-        k_bwd_sf<<<k->sf_grid, kTPB, 0, st>>>(lv.pad, lv.pad_len, c->mv.ioffset, c->mv.ja,
-                                              c->mv.diag, k->a, k->d, k->rdi, k->sf_y, z,
-                                              k->sf_ctl, k->S, k->sf_spin);
+      k_bwd_sf<<<k->sf_grid, kTPB, 0, st>>>(lv.pad, lv.pad_len, c->mv.ioffset, c->mv.ja,
+                                            c->mv.diag, k->a, k->d, k->rdi, k->sf_y, z,
+                                            k->sf_ctl, k->S, k->sf_spin);
     }
     return;
   }
@@ -1647,13 +1490,7 @@ static int run_solver(fcg_context *c, int kind, const double *a, const double *s
     k_sf_fill<<<grid_for(c->n, c->num_sms), kTPB, 0, c->stream>>>(c->n, k->d, nullptr,
                                                                     k->sf_ctl);
     if (wave_sweeps(c)) {
-      const HexBlock &h = c->hex;
-      k_wave_coef<<<grid_for(c->n, c->num_sms), kTPB, 0, c->stream>>>(
-          h.nx, h.ny, h.nz, c->mv.ioffset, c->mv.diag, k->a, k->wlo, k->wup);
-      if (k->wave_wide)
-        launch_wave_factor<16, 8>(c, kind == SK_BICG);
-      else
-        launch_wave_factor<8, 8>(c, kind == SK_BICG);
+      if ((rc = start_wave(c, kind == SK_BICG))) return rc;
     } else {
       k_factor_sf<<<k->sf_grid, kTPB, 0, c->stream>>>(
           c->lf.pad, c->lf.pad_len, c->mv.ioffset, c->mv.ja, c->mv.diag, c->tpos, k->a, k->d,
