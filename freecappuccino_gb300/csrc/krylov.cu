@@ -350,8 +350,8 @@ __global__ void __launch_bounds__(kTPB, 8) k_cg_dot(int n, const double *__restr
 
 // --- triangular sweeps, one launch per level -----------------------------------
 // The row arithmetic is explicit -- the sweeps' coefficient a_k d_i rounded, then a fused
-// multiply-add per entry; the factors' products and differences each rounded -- so that
-// every kernel form (per level, one launch, wavefront tiles) gives the same bits.
+// multiply-add per entry; the factors' product a_k^2 or a_k a_k^T likewise -- so that every
+// kernel form (per level, one launch, wavefront tiles) gives the same bits.
 // forward: z_i = b_i d_i - sum_{k<diag} (a_k d_i) z_{ja_k}        (iccg.f90:248-254)
 __global__ void k_fwd_level(const int *__restrict__ rows, int count,
                             const int *__restrict__ ioffset, const int *__restrict__ ja,
@@ -542,10 +542,7 @@ __global__ void k_factor_sf(const int *__restrict__ rows, int len, const int *__
     bool ok = true;
     for (int k = ioffset[i]; k < diag[i]; ++k) {
       const double dj = sf_value(&d[ja[k]], &ctl[3], spin, &ok);
-      if (dilu)
-        di = __dsub_rn(di, __dmul_rn(__dmul_rn(a[k], dj), a[tpos[k]]));
-      else
-        di = __dsub_rn(di, __dmul_rn(__dmul_rn(a[k], a[k]), dj));
+      di = __fma_rn(-(a[k] * (dilu ? a[tpos[k]] : a[k])), dj, di);
     }
     if (!ok) sf_fail(&ctl[3], S);
     const double inv = 1.0 / di;
@@ -568,101 +565,12 @@ __global__ void k_factor_level(const int *__restrict__ rows, int count,
   int i = rows[t];
   double di = a[diag[i]];
   for (int k = ioffset[i]; k < diag[i]; ++k) {
-    int j = ja[k];
-    if (dilu)
-      di = __dsub_rn(di, __dmul_rn(__dmul_rn(a[k], d[j]), a[tpos[k]]));
-    else
-      di = __dsub_rn(di, __dmul_rn(__dmul_rn(a[k], a[k]), d[j]));
+    di = __fma_rn(-(a[k] * (dilu ? a[tpos[k]] : a[k])), d[ja[k]], di);
   }
   double inv = 1.0 / di;
   d[i] = inv;
   rdi[i] = inv / (inv + S->small);
   if (!isfinite(inv) || di == 0.0) fail_status(S, FCG_ERR_PIVOT);
-}
-
-// --- wavefront-tiled factor on a lexicographic hex block --------------------------
-// The tiles and steps of wave_sweep.cuh, from the CSR and in the natural order (once per
-// solve): a tile's first row and column read the cells of other tiles from global memory
-// through the value-as-flag wait of the one-launch sweeps.  Tiles are claimed in an order
-// in which a tile's upstream tiles come first.  The level kernel's arithmetic: the same
-// bits.
-template <int TX, int TY>
-struct WaveTile {
-  int ntx, nty, di, dj, p, q;
-  bool col_ok;
-  long long col0, step_i, step_j;
-};
-
-// Claims a tile (thread 0, broadcast); false when every tile is taken.
-template <int TX, int TY>
-__device__ __forceinline__ bool wave_claim(int nx, int ny, int *counter, WaveTile<TX, TY> &t) {
-  __shared__ int tile_sh;
-  if (threadIdx.x == 0) tile_sh = atomicAdd(counter, 1);
-  __syncthreads();
-  t.ntx = (nx + TX - 1) / TX;
-  t.nty = (ny + TY - 1) / TY;
-  const int tile = tile_sh;
-  if (tile >= t.ntx * t.nty) return false;
-  t.di = threadIdx.x % TX;
-  t.dj = threadIdx.x / TX;
-  t.p = (tile % t.ntx) * TX + t.di;
-  t.q = (tile / t.ntx) * TY + t.dj;
-  t.col_ok = t.p < nx && t.q < ny;
-  t.col0 = t.p + (long long)nx * t.q;
-  t.step_i = -1;
-  t.step_j = -nx;
-  return true;
-}
-
-// DIC (DILU) factor d = 1/(a_ii - sum a_ik^2 d_k) (1/(a_ii - sum a_ik d_k a_ki)) in the
-// forward wavefront, reading the CSR directly (once per solve); also rdi = d/(d + small).
-template <int TX, int TY, bool DILU>
-__global__ void __launch_bounds__(TX * TY)
-    k_wave_factor(int nx, int ny, int nz, const int *__restrict__ ioffset,
-                  const int *__restrict__ diag, const int *__restrict__ tpos,
-                  const double *__restrict__ a, double *d, double *__restrict__ rdi, int *ctl,
-                  Scal *S, int spin) {
-  __shared__ double sm[2][TY][TX];
-  WaveTile<TX, TY> t;
-  if (!wave_claim<TX, TY>(nx, ny, &ctl[0], t)) return;
-  const long long nxy = (long long)nx * ny;
-  const int nlev = TX + TY - 2 + nz;
-  double prev = 0.0;
-  for (int L = 0; L < nlev; ++L) {
-    const int s = L - t.di - t.dj;
-    double val = 0.0;
-    if (t.col_ok && s >= 0 && s < nz) {
-      const long long r = t.col0 + nxy * s;
-      bool ok = true;
-      double vq = 0.0, vp = 0.0;
-      if (t.q > 0)
-        vq = t.dj > 0 ? sm[(L - 1) & 1][t.dj - 1][t.di]
-                      : sf_value(&d[r + t.step_j], &ctl[3], spin, &ok);
-      if (t.p > 0)
-        vp = t.di > 0 ? sm[(L - 1) & 1][t.dj][t.di - 1]
-                      : sf_value(&d[r + t.step_i], &ctl[3], spin, &ok);
-      if (!ok) sf_fail(&ctl[3], S);
-      int e = ioffset[r];
-      double dd = a[diag[r]];
-      auto term = [&](double v) {
-        if (DILU)
-          dd = __dsub_rn(dd, __dmul_rn(__dmul_rn(a[e], v), a[tpos[e]]));
-        else
-          dd = __dsub_rn(dd, __dmul_rn(__dmul_rn(a[e], a[e]), v));
-        ++e;
-      };
-      if (s > 0) term(prev);  // CSR order of the lower entries: k, j, i
-      if (t.q > 0) term(vq);
-      if (t.p > 0) term(vp);
-      val = 1.0 / dd;
-      st_relaxed64(&d[r], val);
-      rdi[r] = val / (val + S->small);
-      if (!isfinite(val) || dd == 0.0) fail_status(S, FCG_ERR_PIVOT);
-      prev = val;
-    }
-    sm[L & 1][t.dj][t.di] = val;
-    __syncthreads();
-  }
 }
 
 // --- BiCGStab sweep (bicgstab.f90:99-224) -------------------------------------
@@ -1208,23 +1116,8 @@ static bool wave_sweeps(const fcg_context *c) {
   return k->sf_on && k->wave_on && c->hex.ok && k->sf_absent_row < 0;
 }
 
-template <int TX, int TY>
-static int wave_tiles(const fcg_context *c) {
-  return ((c->hex.nx + TX - 1) / TX) * ((c->hex.ny + TY - 1) / TY);
-}
-
-template <int TX, int TY>
-static void launch_wave_factor(fcg_context *c, bool dilu) {
-  KrylovState *k = c->ks;
-  const HexBlock &h = c->hex;
-  if (dilu)
-    k_wave_factor<TX, TY, true><<<wave_tiles<TX, TY>(c), TX * TY, 0, c->stream>>>(
-        h.nx, h.ny, h.nz, c->mv.ioffset, c->mv.diag, c->tpos, k->a, k->d, k->rdi, k->sf_ctl,
-        k->S, k->sf_spin);
-  else
-    k_wave_factor<TX, TY, false><<<wave_tiles<TX, TY>(c), TX * TY, 0, c->stream>>>(
-        h.nx, h.ny, h.nz, c->mv.ioffset, c->mv.diag, c->tpos, k->a, k->d, k->rdi, k->sf_ctl,
-        k->S, k->sf_spin);
+static wave::Control wave_control(KrylovState *k) {
+  return wave::Control{k->sf_ctl, &k->S->wait_fail, &k->S->status, &k->S->done, k->sf_spin};
 }
 
 // Factor, records and armed vectors of a solve with the wavefront-tiled sweeps.
@@ -1232,8 +1125,7 @@ static int start_wave(fcg_context *c, bool dilu) {
   KrylovState *k = c->ks;
   int rc;
   if (!k->wv.fwd && (rc = wave::allocate(c, 1, k->wbuf, k->wv))) return rc;
-  launch_wave_factor<16, 8>(c, dilu);
-  return wave::start(c, 1, c->nnz, k->a, k->d, k->rdi, 0.0, k->wv, k->sf_ctl);
+  return wave::start(c, 1, c->nnz, k->a, dilu, k->small, k->wv, wave_control(k));
 }
 
 static void launch_sweeps(fcg_context *c, cudaStream_t st, const Level &lv, bool forward,
@@ -1241,8 +1133,8 @@ static void launch_sweeps(fcg_context *c, cudaStream_t st, const Level &lv, bool
   KrylovState *k = c->ks;
   if (k->sf_on) {
     if (wave_sweeps(c)) {
-      wave::launch<double>(c, st, 1, forward, k->wv, b, z, k->sf_ctl, &k->S->wait_fail,
-                           &k->S->status, &k->S->done, k->sf_spin);
+      wave::launch<double>(c, st, 1, forward ? wave::kForward : wave::kBackward, k->wv, b, z,
+                           wave_control(k));
       return;
     }
     if (forward) {  // b -> sf_y, after the sentinel fill of sf_y and z
@@ -1487,11 +1379,11 @@ static int run_solver(fcg_context *c, int kind, const double *a, const double *s
     FCG_CHECK_LAUNCH(c, "mixed set-up");
   }
   if (kind != SK_DPCG && k->sf_on) {  // factor diagonal in one sync-free launch
-    k_sf_fill<<<grid_for(c->n, c->num_sms), kTPB, 0, c->stream>>>(c->n, k->d, nullptr,
-                                                                    k->sf_ctl);
     if (wave_sweeps(c)) {
       if ((rc = start_wave(c, kind == SK_BICG))) return rc;
     } else {
+      k_sf_fill<<<grid_for(c->n, c->num_sms), kTPB, 0, c->stream>>>(c->n, k->d, nullptr,
+                                                                    k->sf_ctl);
       k_factor_sf<<<k->sf_grid, kTPB, 0, c->stream>>>(
           c->lf.pad, c->lf.pad_len, c->mv.ioffset, c->mv.ja, c->mv.diag, c->tpos, k->a, k->d,
           k->rdi, k->sf_ctl, k->S, k->sf_spin, kind == SK_BICG);

@@ -164,7 +164,11 @@ struct Arrays {
   T *ze;  // backward result on the tiles' first rows and columns (likewise)
 };
 
-// One sweep of ns systems over the planes [k0, k1): forward y = (b - L y) d from `in`
+constexpr int kForward = 0, kBackward = 1, kFactor = 2;
+
+// One sweep of ns systems over the planes [k0, k1): the factor y = 1/(a_ii - sum w y) from
+// the forward records {w of lower k, lower j, lower i, a_ii} (w = a_ij^2 for DIC, a_ij a_ji
+// for DILU), forward y = (b - L y) d from `in`
 // (natural order, system s at s n), or backward z = y rescale - (U z) d into `out`
 // (natural order), rescale = d / (d + small).
 // Measured (GB300, FP64, us forward / backward): 128^3 156 / 155 against 356 / 380 with the
@@ -173,13 +177,14 @@ struct Arrays {
 // 34.7 -> 18.0 ms, at 256^3 125 -> 68 ms.  One tile alone takes 0.28 us a step (FP32 0.16).
 // kD = 4 or 12 measured 189 and 170 us forward at 128^3 and 1217 and 475 us at 256^3
 // (kD = 8: 156 and 473); clusters of 1 x 8, 4 x 2 or 4 x 4 tiles are within 3% of 2 x 4.
-template <class T, bool BWD>
+template <class T, int MODE>
 __global__ void __launch_bounds__(kThreads) __cluster_dims__(CX *CY, 1, 1)
     k_wave_sweep(int nx, int ny, int nz, int k0, int k1, int ns, Arrays<T> A,
                  const T *__restrict__ in, T *out, int *ctl, int *fail, int *status,
                  const int *done, int spin) {
   using W = Word<T>;
   constexpr int P = kPlanes;
+  constexpr bool BWD = MODE == kBackward, FACTOR = MODE == kFactor;
   if (__ldcg(done) != 0) return;
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
@@ -278,7 +283,7 @@ __global__ void __launch_bounds__(kThreads) __cluster_dims__(CX *CY, 1, 1)
     T *yw = A.y + sys * vl + tile0 + (long long)L0 * NT + tid;
     T *zw = A.ze + sys * vl + tile0 + (long long)L0 * NT + tid;
     // natural position of the column's cell, from the slab's first plane on
-    const T *xin = BWD ? nullptr : in + i + (long long)nx * j + (long long)nxy * k0 + sys * n;
+    const T *xin = MODE != kForward ? nullptr : in + i + (long long)nx * j + (long long)nxy * k0 + sys * n;
     T *xout = BWD ? out + i + (long long)nx * j + (long long)nxy * k0 + sys * n : nullptr;
     // The neighbours' values of step u stand at p_at + u p_inc and q_at + u q_inc: for the
     // tile's first (last) row and column in the edge buffers, cell by cell; for the others
@@ -315,7 +320,7 @@ __global__ void __launch_bounds__(kThreads) __cluster_dims__(CX *CY, 1, 1)
       for (int p = 0; p < P; ++p) cl.c[p] = __ldg(rec + step * u * (P * NT) + p * NT);
       if (BWD) {
         cl.x = yw[step * u * NT];
-      } else {
+      } else if (!FACTOR) {
         const int kk = k + u;
         cl.x = T(0);
         if ((unsigned)kk < (unsigned)depth && col_ok) cl.x = __ldg(xin + (long long)nxy * kk);
@@ -330,7 +335,7 @@ __global__ void __launch_bounds__(kThreads) __cluster_dims__(CX *CY, 1, 1)
     T prev = T(0);
     if (col_ok && !BWD && k0 > 0) prev = A.y[sys * vl + lay.at(i, j, k0 - 1)];
     if (col_ok && BWD && k1 < nz) prev = xout[(long long)nxy * depth];
-    part = ring[0].x * ring[0].c[3];
+    part = FACTOR ? ring[0].c[3] : ring[0].x * ring[0].c[3];
     if (!BWD) part = W::sub(part, ring[0].c[0], prev);
     const int steps = depth + TX + TY - 2;
     for (int s0 = 0; s0 < steps; s0 += kD) {
@@ -363,6 +368,7 @@ __global__ void __launch_bounds__(kThreads) __cluster_dims__(CX *CY, 1, 1)
         if (!BWD) {  // lower entries in CSR order: k, j, i
           val = W::sub(part, c1, vq);
           val = W::sub(val, c2, vp);
+          if (FACTOR) val = T(1) / val;
         } else {  // upper entries in CSR order: i, j, k
           val = W::sub(part, c0, vp);
           val = W::sub(val, c1, vq);
@@ -370,7 +376,7 @@ __global__ void __launch_bounds__(kThreads) __cluster_dims__(CX *CY, 1, 1)
         }
         const Cell &next = ring[(u + 1) % kD];
         load(u + kD, ring[u]);
-        part = next.x * next.c[3];
+        part = FACTOR ? next.c[3] : next.x * next.c[3];
         sm[(u + 1) % kD][dj][di] = val;
         if (act) prev = val;
         if (!BWD) part = W::sub(part, next.c[0], prev);
@@ -399,27 +405,56 @@ __global__ void __launch_bounds__(kThreads) __cluster_dims__(CX *CY, 1, 1)
   cluster.sync();  // no block leaves while a neighbour may store into its buffers
 }
 
-// Records of ns systems from the CSR values a (system s at s nnz), the factor d and, in
-// FP64, the rescale d / (d + small) (both natural order, system s at s n; without resc it
-// is formed here); once per solve.
+// Records of the factor of ns systems from the CSR values a (system s at s nnz).
+template <class T>
+__global__ void k_wave_pack_factor(int nx, int ny, int nz, int ns, long long nnz,
+                                   const int *__restrict__ ioffset, const int *__restrict__ diag,
+                                   const int *__restrict__ tpos, const T *__restrict__ a, int dilu,
+                                   Arrays<T> A) {
+  const Layout lay(nx, ny, nz);
+  const int nxy = nx * ny;
+  const long long n = (long long)nxy * nz;
+  FCG_GRID_STRIDE(r, n) {
+    const int i = (int)(r % nx), j = (int)((r / nx) % ny), k = (int)(r / nxy);
+    const long long q = lay.at(i, j, k), at = q / NT * kPlanes * NT + q % NT;
+    const int lo = ioffset[r], dg = diag[r];
+    const bool has[3] = {k > 0, j > 0, i > 0};
+    for (int s = 0; s < ns; ++s) {
+      const T *as = a + s * nnz;
+      T *f = A.fwd + s * lay.rec_len() + at;
+      int e = lo;
+#pragma unroll
+      for (int p = 0; p < 3; ++p) {
+        f[p * NT] = has[p] ? as[e] * (dilu ? as[tpos[e]] : as[e]) : T(0);
+        e += has[p];
+      }
+      f[3 * NT] = as[dg];
+    }
+  }
+}
+
+// Records of the sweeps of ns systems from the CSR values a (system s at s nnz) and the
+// factor, which the factor sweep left in A.y; a pivot that is not finite is recorded.
 template <class T>
 __global__ void k_wave_pack(int nx, int ny, int nz, int ns, long long nnz,
                             const int *__restrict__ ioffset, const int *__restrict__ diag,
-                            const T *__restrict__ a, const T *__restrict__ d,
-                            const T *__restrict__ resc, T small, Arrays<T> A) {
+                            const T *__restrict__ a, T small, Arrays<T> A, int *status,
+                            const int *done) {
+  if (__ldcg(done) != 0) return;  // the factor sweep has not run
   const Layout lay(nx, ny, nz);
-  const long long nxy = (long long)nx * ny, n = nxy * nz;
+  const int nxy = nx * ny;
+  const long long n = (long long)nxy * nz;
   FCG_GRID_STRIDE(r, n) {
     const int i = (int)(r % nx), j = (int)((r / nx) % ny), k = (int)(r / nxy);
-    const long long q = lay.at(i, j, k), rec = q / NT, tid = q % NT;
+    const long long q = lay.at(i, j, k), at = q / NT * kPlanes * NT + q % NT;
     const int lo = ioffset[r], up = diag[r] + 1;
     const bool l0 = k > 0, l1 = j > 0, l2 = i > 0;
     const bool u0 = i < nx - 1, u1 = j < ny - 1, u2 = k < nz - 1;
     for (int s = 0; s < ns; ++s) {
       const T *as = a + s * nnz;
-      T *f = A.fwd + s * lay.rec_len() + rec * kPlanes * NT + tid;
-      T *b = A.bwd + s * lay.rec_len() + rec * kPlanes * NT + tid;
-      const T dd = d[s * n + r];
+      T *f = A.fwd + s * lay.rec_len() + at;
+      T *b = A.bwd + s * lay.rec_len() + at;
+      const T dd = A.y[s * lay.vec_len() + q];
       f[0] = l0 ? as[lo] * dd : T(0);
       f[NT] = l1 ? as[lo + l0] * dd : T(0);
       f[2 * NT] = l2 ? as[lo + l0 + l1] * dd : T(0);
@@ -427,7 +462,8 @@ __global__ void k_wave_pack(int nx, int ny, int nz, int ns, long long nnz,
       b[0] = u0 ? as[up] * dd : T(0);
       b[NT] = u1 ? as[up + u0] * dd : T(0);
       b[2 * NT] = u2 ? as[up + u0 + u1] * dd : T(0);
-      b[3 * NT] = resc ? resc[s * n + r] : dd / (dd + small);
+      b[3 * NT] = dd / (dd + small);
+      if (!isfinite(dd)) atomicCAS(status, 0, FCG_ERR_PIVOT);
     }
   }
 }
@@ -452,10 +488,10 @@ int allocate(fcg_context *c, int ns, DBuf &buf, Arrays<T> &A) {
   FCG_CUDA_TRY(c, buf.ensure(bytes));
   FCG_CUDA_TRY(c, cudaMemsetAsync(buf.p, 0, bytes, c->stream));
   const int smem = (TX + TY) * kSlab * (int)sizeof(T);
-  FCG_CUDA_TRY(c, cudaFuncSetAttribute(k_wave_sweep<T, false>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  FCG_CUDA_TRY(c, cudaFuncSetAttribute(k_wave_sweep<T, true>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  for (const void *f : {(const void *)k_wave_sweep<T, kForward>,
+                        (const void *)k_wave_sweep<T, kBackward>,
+                        (const void *)k_wave_sweep<T, kFactor>})
+    FCG_CUDA_TRY(c, cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   T *p = buf.as<T>();
   A.fwd = p + g;
   A.bwd = p + ns * rl + g;
@@ -464,39 +500,54 @@ int allocate(fcg_context *c, int ns, DBuf &buf, Arrays<T> &A) {
   return FCG_OK;
 }
 
-// Packs the records and arms the vectors of a solve.
-template <class T>
-int start(fcg_context *c, int ns, long long nnz, const T *a, const T *d, const T *resc, T small,
-          const Arrays<T> &A, int *ctl) {
-  const HexBlock &h = c->hex;
-  const Layout lay(h.nx, h.ny, h.nz);
-  k_wave_pack<T><<<grid_for(c->n, c->num_sms), kTPB, 0, c->stream>>>(
-      h.nx, h.ny, h.nz, ns, nnz, c->mv.ioffset, c->mv.diag, a, d, resc, small, A);
-  const long long vl = ns * lay.vec_len(), g = Layout::guard();
-  k_wave_arm<T><<<grid_for(vl, c->num_sms), kTPB, 0, c->stream>>>(vl, A.y - g, A.ze - g, ctl);
-  FCG_CHECK_LAUNCH(c, "wavefront records");
-  return FCG_OK;
-}
+// What a launch needs besides the arrays: the solver's control words {forward claims,
+// backward claims, -, error}, its status and stop flags (fail may be null) and the polls
+// after which a wait gives up.
+struct Control {
+  int *ctl, *fail, *status;
+  const int *done;
+  int spin;
+};
 
 // One sweep, in launches of at most kSlab planes (each a whole sweep over its planes).
 template <class T>
-void launch(fcg_context *c, cudaStream_t st, int ns, bool forward, const Arrays<T> &A, const T *in,
-            T *out, int *ctl, int *fail, int *status, const int *done, int spin) {
+void launch(fcg_context *c, cudaStream_t st, int ns, int mode, const Arrays<T> &A, const T *in,
+            T *out, const Control &w) {
   const HexBlock &h = c->hex;
   const int g = Layout(h.nx, h.ny, h.nz).clusters() * ns * CX * CY;
   const int slabs = (h.nz + kSlab - 1) / kSlab;
   for (int s = 0; s < slabs; ++s) {
-    const int b = forward ? s : slabs - 1 - s;
+    const int b = mode == kBackward ? slabs - 1 - s : s;
     const int k0 = (int)((long long)h.nz * b / slabs), k1 = (int)((long long)h.nz * (b + 1) / slabs);
     const size_t smem = (size_t)(TX + TY) * (k1 - k0) * sizeof(T);
-    if (s > 0) cudaMemsetAsync(ctl, 0, 2 * sizeof(int), st);
-    if (forward)
-      k_wave_sweep<T, false><<<g, kThreads, smem, st>>>(h.nx, h.ny, h.nz, k0, k1, ns, A, in, out,
-                                                        ctl, fail, status, done, spin);
-    else
-      k_wave_sweep<T, true><<<g, kThreads, smem, st>>>(h.nx, h.ny, h.nz, k0, k1, ns, A, in, out,
-                                                       ctl, fail, status, done, spin);
+    if (s > 0) cudaMemsetAsync(w.ctl, 0, 2 * sizeof(int), st);
+    auto kernel = mode == kForward    ? k_wave_sweep<T, kForward>
+                  : mode == kBackward ? k_wave_sweep<T, kBackward>
+                                      : k_wave_sweep<T, kFactor>;
+    kernel<<<g, kThreads, smem, st>>>(h.nx, h.ny, h.nz, k0, k1, ns, A, in, out, w.ctl, w.fail,
+                                      w.status, w.done, w.spin);
   }
+}
+
+// The factor and the records of ns systems, and armed vectors: before the first sweep of
+// a solve.  128^3, FP64: about 0.4 ms; a factor that read the CSR at every step, with every
+// hand-over through global memory, took 1.08 ms.
+template <class T>
+int start(fcg_context *c, int ns, long long nnz, const T *a, bool dilu, T small,
+          const Arrays<T> &A, const Control &w) {
+  const HexBlock &h = c->hex;
+  const Layout lay(h.nx, h.ny, h.nz);
+  const long long vl = ns * lay.vec_len(), g = Layout::guard();
+  const int gc = grid_for(c->n, c->num_sms), gv = grid_for(vl, c->num_sms);
+  k_wave_pack_factor<T><<<gc, kTPB, 0, c->stream>>>(h.nx, h.ny, h.nz, ns, nnz, c->mv.ioffset,
+                                                    c->mv.diag, c->tpos, a, dilu, A);
+  k_wave_arm<T><<<gv, kTPB, 0, c->stream>>>(vl, A.y - g, A.ze - g, w.ctl);
+  launch<T>(c, c->stream, ns, kFactor, A, nullptr, nullptr, w);
+  k_wave_pack<T><<<gc, kTPB, 0, c->stream>>>(h.nx, h.ny, h.nz, ns, nnz, c->mv.ioffset,
+                                             c->mv.diag, a, small, A, w.status, w.done);
+  k_wave_arm<T><<<gv, kTPB, 0, c->stream>>>(vl, A.y - g, A.ze - g, w.ctl);
+  FCG_CHECK_LAUNCH(c, "wavefront factor and records");
+  return FCG_OK;
 }
 
 }  // namespace wave

@@ -80,3 +80,29 @@ def test_tiled_sweeps_equal_row_sweeps(dims):
             assert np.array_equal(r.fi, o.fi) and r.resl == o.resl, (dims, solver)
     for c in ctxs:
         c.close()
+
+
+@pytest.mark.parametrize("dims,nsys", [((17, 9, 4), 1), ((35, 37, 6), 5), ((5, 9, 513), 3)])
+def test_tiled_multi_rhs_sweeps_equal_row_sweeps(dims, nsys):
+    """The FP32 form, several systems in one launch."""
+    from freecappuccino_gb300.systems import transport_systems
+
+    m = box_mesh(*dims)
+    out = []
+    for mode in (None, "rows"):
+        c = _context(m)
+        a, su, _ = transport_systems(m, c.create_csr(), nsys=nsys)
+        saved = os.environ.pop("FCG_SWEEP", None)
+        if mode:
+            os.environ["FCG_SWEEP"] = mode  # read when the multi-RHS state is made
+        try:
+            out.append([c.bicgstab_multi(a, su, np.zeros_like(su), 1e-10, 200)
+                        for _ in range(2)][1])
+        finally:
+            os.environ.pop("FCG_SWEEP", None)
+            if saved is not None:
+                os.environ["FCG_SWEEP"] = saved
+        c.close()
+    (x1, r1), (x2, r2) = out
+    assert np.array_equal(x1, x2) and [r.iters for r in r1] == [r.iters for r in r2]
+    assert all(r.converged for r in r1)
