@@ -273,6 +273,7 @@ extern "C" int fcg_bind_mesh(fcg_context *c, const fcg_mesh_desc *m) {
   c->bound_allocs.clear();
   c->bound = false;
   c->dmat_ready = false;
+  c->order = LevelOrder{};
   c->fgeo_ready = false;
   c->bgeo_ready = false;
 

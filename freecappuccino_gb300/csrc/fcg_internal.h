@@ -108,6 +108,20 @@ struct Level {
   int pad_len = 0;
 };
 
+// The level order of one triangle's sweeps (level_sweep.cuh): chunks of 32 positions, row[p]
+// the row at position p (-1: padding, the Level's pad list); the entries of chunk c are the
+// columns [ptr[c], ptr[c+1]) of 32: dep[32 t + lane] the position whose result the row at
+// lane reads (-1: none) and src its coefficient's CSR position; xpos[p] (upper triangle) the
+// position of the same row in the lower triangle's order.
+struct LevelSide {
+  int chunks = 0, entries = 0;  // entries = ptr[chunks]
+  const int *row = nullptr, *ptr = nullptr, *dep = nullptr, *src = nullptr, *xpos = nullptr;
+};
+struct LevelOrder {
+  LevelSide lo, up;
+  bool ready = false;
+};
+
 }  // namespace fcg
 
 namespace fcg {
@@ -141,6 +155,7 @@ struct fcg_context {
   int sell_maxw = 0;
   long long sell_len = 0, sell_nuniform = 0;
   fcg::Level lf, lb;  // forward (lower) and backward (upper) level schedules
+  fcg::LevelOrder order;  // of those schedules, built at the first solve that needs it
   fcg::HexBlock hex;  // the block structure of the cell numbering, when it has one
   const int *tpos = nullptr;  // CSR position of the transpose entry of every entry
   // every topology array bound to the device (pointer, bytes), for fcg_topology_digest
@@ -220,6 +235,8 @@ int build_rest(const fcg_mesh_desc &m, const int cnt[B_NTYPES], const int fst[B_
 int scan_ints(fcg_context *c, const int *in, int *out, int n, DBuf &tmp);
 // a[i] -= 1 on the device (1-based index arrays to 0-based), on c's stream.
 int to_zero_based(fcg_context *c, int *a, long long n);
+// Builds c->order (level_order.cu) when it is not there; synchronises c's stream.
+int level_order(fcg_context *c);
 // Fills c->hex from the bound CSR pattern (hexblock.cu); synchronises c's stream.
 int detect_hex_block(fcg_context *c);
 // The whole topology built on c's device (setup.cu), 0-based and owned by the bound

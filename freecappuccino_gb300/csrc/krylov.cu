@@ -34,6 +34,7 @@
 #include "fcg_internal.h"
 #include "krylov_common.cuh"
 #include "launch.h"
+#include "level_sweep.cuh"
 #include "wave_sweep.cuh"
 
 namespace fcg {
@@ -95,12 +96,12 @@ struct KrylovState {
   int last_kind = -1;
   double small = (double)1e-20f;  // parameters::small (modules_allocatable.f90:27)
   int early_exit = 1;
-  // sync-free triangular sweeps: the forward result and the control words
-  // {forward claim counter, backward claim counter, -, error}
-  DBuf sfb;
-  double *sf_y = nullptr;
+  // one-launch triangular sweeps: the control words {forward claim counter, backward claim
+  // counter, -, error} and, on meshes that are no block, the arrays in level order
+  // (level_sweep.cuh), made at the first solve that sweeps
+  DBuf sfb, lbuf;
   int *sf_ctl = nullptr;
-  int sf_grid = 0;
+  level::Arrays<double> lv{};
   bool sf_on = true;
   int sf_spin = 1 << 20;     // polls before a dependency wait gives up
   int sf_absent_row = -1;    // test hook: this row never publishes its flag
@@ -123,6 +124,7 @@ void destroy_krylov(KrylovState *k) {
   k->trace.release();
   k->mixed.release();
   k->sfb.release();
+  k->lbuf.release();
   delete k;
 }
 
@@ -383,173 +385,6 @@ __global__ void k_bwd_level(const int *__restrict__ rows, int count,
   double zi = z[i] * rdi[i];
   for (int k = diag[i] + 1; k < ioffset[i + 1]; ++k) zi = __fma_rn(-(a[k] * di), z[ja[k]], zi);
   z[i] = zi;
-}
-
-// --- sync-free triangular sweeps ---------------------------------------------------
-// The same row arithmetic as the level kernels, in one launch: warps claim 32 entries of
-// the level-ordered row list (levels padded to multiples of 32, so a warp's rows are
-// independent) through an atomic counter, and each row waits for the values it reads.
-// The output vector is filled with a sentinel before the sweep, a signalling-NaN bit
-// pattern that arithmetic never produces; a row polls the 64-bit word it needs until the
-// sentinel is gone and uses the value it read, so the value is its own ready flag (an
-// aligned 64-bit access is single-copy atomic) and no fence is needed.  Claims are
-// monotone and a row only reads rows of earlier levels, so every awaited row was claimed
-// earlier by a warp that is running: the waits end.  Each wait is bounded; one that gives
-// up records FCG_ERR_TIMEOUT, and every row still writes its result so no other wait is
-// held up by it.  The backward sweep writes a second vector, so a forward result is
-// never mistaken for a backward one.
-constexpr unsigned long long kSentinel = 0x7ff0dead0badf00dULL;
-
-__device__ __forceinline__ double ld_relaxed64(const double *p) {
-  unsigned long long v;
-  asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-  return __longlong_as_double((long long)v);
-}
-
-__device__ __forceinline__ void st_relaxed64(double *p, double x) {
-  asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p),
-               "l"((unsigned long long)__double_as_longlong(x))
-               : "memory");
-}
-
-__device__ __forceinline__ bool is_sentinel(double v) {
-  return (unsigned long long)__double_as_longlong(v) == kSentinel;
-}
-
-// The value at p once it is not the sentinel; gives up after `spin` polls (or when
-// another wait has given up) and returns what it last read.
-__device__ __forceinline__ double sf_value(const double *p, const int *err, int spin, bool *ok) {
-  double v = ld_relaxed64(p);
-  if (!is_sentinel(v)) return v;
-  for (int it = 0; it < spin; ++it) {
-    if (it >= 16) __nanosleep(32);
-    v = ld_relaxed64(p);
-    if (!is_sentinel(v)) return v;
-    if ((it & 63) == 63 && *(volatile const int *)err) break;
-  }
-  *ok = false;
-  return v;
-}
-
-__device__ __forceinline__ void sf_fail(int *err, Scal *S) {
-  if (atomicExch(err, 1) == 0) {
-    S->wait_fail = 1;
-    fail_status(S, FCG_ERR_TIMEOUT);
-  }
-}
-
-constexpr int kSfBatch = 8;  // dependencies of a row loaded and awaited together
-
-// Sentinel into the sweep outputs; ctl = {forward counter, backward counter, -, error}.
-__global__ void k_sf_fill(int n, double *__restrict__ o1, double *__restrict__ o2, int *ctl) {
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    ctl[0] = 0;
-    ctl[1] = 0;
-    ctl[3] = 0;
-  }
-  const double s = __longlong_as_double((long long)kSentinel);
-  FCG_GRID_STRIDE(i, n) {
-    o1[i] = s;
-    if (o2) o2[i] = s;
-  }
-}
-
-// One row: acc - sum (a_k di) v_{ja_k} over k in [k0, hi), the values awaited in batches.
-__device__ __forceinline__ double sf_row(double acc, double di, int k0, int hi, const int *__restrict__ ja,
-                                         const double *__restrict__ a, const double *v, int *ctl,
-                                         Scal *S, int spin) {
-  for (; k0 < hi; k0 += kSfBatch) {
-    int jj[kSfBatch];
-    double aa[kSfBatch], vv[kSfBatch];
-#pragma unroll
-    for (int t = 0; t < kSfBatch; ++t)
-      if (k0 + t < hi) {
-        jj[t] = ja[k0 + t];
-        aa[t] = a[k0 + t];
-      }
-    bool ok = true;
-#pragma unroll
-    for (int t = 0; t < kSfBatch; ++t)  // all first reads in flight together
-      if (k0 + t < hi) vv[t] = ld_relaxed64(&v[jj[t]]);
-#pragma unroll
-    for (int t = 0; t < kSfBatch; ++t)
-      if (k0 + t < hi && is_sentinel(vv[t])) vv[t] = sf_value(&v[jj[t]], &ctl[3], spin, &ok);
-    if (!ok) sf_fail(&ctl[3], S);
-#pragma unroll
-    for (int t = 0; t < kSfBatch; ++t)
-      if (k0 + t < hi) acc = __fma_rn(-(aa[t] * di), vv[t], acc);
-  }
-  return acc;
-}
-
-// forward: y_i = b_i d_i - sum_{k<diag} (a_k d_i) y_{ja_k}        (iccg.f90:248-254)
-__global__ void k_fwd_sf(const int *__restrict__ rows, int len, const int *__restrict__ ioffset,
-                         const int *__restrict__ ja, const int *__restrict__ diag,
-                         const double *__restrict__ a, const double *__restrict__ d,
-                         const double *__restrict__ b, double *y, int *ctl, Scal *S, int spin,
-                         int absent) {
-  if (solve_done(S)) return;
-  const int lane = threadIdx.x & 31;
-  for (;;) {
-    int base = 0;
-    if (lane == 0) base = atomicAdd(&ctl[0], 32);
-    base = __shfl_sync(0xffffffffu, base, 0);
-    if (base >= len) break;
-    const int i = rows[base + lane];
-    if (i < 0 || i == absent) continue;
-    const double di = d[i];
-    st_relaxed64(&y[i], sf_row(b[i] * di, di, ioffset[i], diag[i], ja, a, y, ctl, S, spin));
-  }
-}
-
-// backward from the forward result y with the reference's rescale zk/(d+small) folded
-// in (iccg.f90:256-265): z_i = y_i rdi_i - sum_{k>diag} (a_k d_i) z_{ja_k}, rdi = d/(d+small)
-__global__ void k_bwd_sf(const int *__restrict__ rows, int len, const int *__restrict__ ioffset,
-                         const int *__restrict__ ja, const int *__restrict__ diag,
-                         const double *__restrict__ a, const double *__restrict__ d,
-                         const double *__restrict__ rdi, const double *__restrict__ y, double *z,
-                         int *ctl, Scal *S, int spin) {
-  if (solve_done(S)) return;
-  const int lane = threadIdx.x & 31;
-  for (;;) {
-    int base = 0;
-    if (lane == 0) base = atomicAdd(&ctl[1], 32);
-    base = __shfl_sync(0xffffffffu, base, 0);
-    if (base >= len) break;
-    const int i = rows[base + lane];
-    if (i < 0) continue;
-    const double di = d[i];
-    st_relaxed64(&z[i], sf_row(y[i] * rdi[i], di, diag[i] + 1, ioffset[i + 1], ja, a, z, ctl, S,
-                               spin));
-  }
-}
-
-// DIC / DILU factor in one launch (iccg.f90:231-237, bicgstab.f90:68-79); d holds the
-// sentinel on entry.
-__global__ void k_factor_sf(const int *__restrict__ rows, int len, const int *__restrict__ ioffset,
-                            const int *__restrict__ ja, const int *__restrict__ diag,
-                            const int *__restrict__ tpos, const double *__restrict__ a, double *d,
-                            double *__restrict__ rdi, int *ctl, Scal *S, int spin, int dilu) {
-  const int lane = threadIdx.x & 31;
-  for (;;) {
-    int base = 0;
-    if (lane == 0) base = atomicAdd(&ctl[0], 32);
-    base = __shfl_sync(0xffffffffu, base, 0);
-    if (base >= len) break;
-    const int i = rows[base + lane];
-    if (i < 0) continue;
-    double di = a[diag[i]];
-    bool ok = true;
-    for (int k = ioffset[i]; k < diag[i]; ++k) {
-      const double dj = sf_value(&d[ja[k]], &ctl[3], spin, &ok);
-      di = __fma_rn(-(a[k] * (dilu ? a[tpos[k]] : a[k])), dj, di);
-    }
-    if (!ok) sf_fail(&ctl[3], S);
-    const double inv = 1.0 / di;
-    st_relaxed64(&d[i], inv);
-    rdi[i] = inv / (inv + S->small);
-    if (!isfinite(inv) || di == 0.0) fail_status(S, FCG_ERR_PIVOT);
-  }
 }
 
 // Factor diagonals, level by level: DIC d_i = 1/(a_ii - sum a_ik^2 d_k) (iccg.f90:
@@ -950,6 +785,8 @@ static int ensure_state(fcg_context *c, int nsw) {
     FCG_CUDA_TRY(c, cudaMemset(k->vec.p, 0, total * sizeof(double)));
     k->wbuf.release();
     k->wv = wave::Arrays<double>{};
+    k->lbuf.release();
+    k->lv = level::Arrays<double>{};
     double *p = k->vec.as<double>();
     double **vecs[] = {&k->x, &k->res, &k->su, &k->pk, &k->zk, &k->qk, &k->invd,
                        &k->d, &k->reso, &k->uk, &k->vk, &k->rtmp, &k->rdi};
@@ -995,20 +832,15 @@ static int ensure_state(fcg_context *c, int nsw) {
     g.mru1 = occ((const void *)k_mx_ru1);
     g.mru2 = occ((const void *)k_mx_ru2);
     g.mp = occ((const void *)k_mx_p);
-    // sync-free sweeps: the forward result vector and the control words
-    FCG_CUDA_TRY(c, k->sfb.ensure(sizeof(double) * (n + 4)));
-    FCG_CUDA_TRY(c, cudaMemset(k->sfb.p, 0, sizeof(double) * (n + 4)));
-    k->sf_y = k->sfb.as<double>();
-    k->sf_ctl = (int *)(k->sf_y + n);
-    k->sf_grid = std::min(occ((const void *)k_fwd_sf), occ((const void *)k_bwd_sf));
+    FCG_CUDA_TRY(c, k->sfb.ensure(4 * sizeof(int)));
+    FCG_CUDA_TRY(c, cudaMemset(k->sfb.p, 0, 4 * sizeof(int)));
+    k->sf_ctl = k->sfb.as<int>();
     {
-      // FCG_SWEEP=levels: one launch per level; =rows: the row-claiming one-launch form
-      // on every mesh; default: the wavefront-tiled form on hex blocks, rows elsewhere
+      // FCG_SWEEP=levels: one launch per level; =rows: one launch in level order on every
+      // mesh; default: wavefront tiles on hex blocks, level order elsewhere
       const char *e = std::getenv("FCG_SWEEP");
       k->sf_on = !(e && std::string(e) == "levels");
       k->wave_on = !(e && (std::string(e) == "levels" || std::string(e) == "rows"));
-      // two blocks per SM: more resident warps only poll further ahead (measured)
-      k->sf_grid = std::min(k->sf_grid, c->num_sms * 2);
     }
     k->bind_gen = c->bind_gen;
     k->matrix_loaded = false;
@@ -1120,10 +952,14 @@ static wave::Control wave_control(KrylovState *k) {
   return wave::Control{k->sf_ctl, &k->S->wait_fail, &k->S->status, &k->S->done, k->sf_spin};
 }
 
-// Factor, records and armed vectors of a solve with the wavefront-tiled sweeps.
-static int start_wave(fcg_context *c, bool dilu) {
+// Factor, coefficients and armed vectors of a solve with one-launch sweeps.
+static int start_sweeps(fcg_context *c, bool dilu) {
   KrylovState *k = c->ks;
   int rc;
+  if (!wave_sweeps(c)) {
+    if (!k->lv.y && (rc = level::allocate(c, 1, k->lbuf, k->lv))) return rc;
+    return level::start(c, 1, c->nnz, k->a, dilu, k->small, k->lv, wave_control(k));
+  }
   if (!k->wv.fwd && (rc = wave::allocate(c, 1, k->wbuf, k->wv))) return rc;
   return wave::start(c, 1, c->nnz, k->a, dilu, k->small, k->wv, wave_control(k));
 }
@@ -1137,16 +973,8 @@ static void launch_sweeps(fcg_context *c, cudaStream_t st, const Level &lv, bool
                            wave_control(k));
       return;
     }
-    if (forward) {  // b -> sf_y, after the sentinel fill of sf_y and z
-      k_sf_fill<<<grid_for(c->n, c->num_sms), kTPB, 0, st>>>(c->n, k->sf_y, z, k->sf_ctl);
-      k_fwd_sf<<<k->sf_grid, kTPB, 0, st>>>(lv.pad, lv.pad_len, c->mv.ioffset, c->mv.ja,
-                                            c->mv.diag, k->a, k->d, b, k->sf_y, k->sf_ctl, k->S,
-                                            k->sf_spin, k->sf_absent_row);
-    } else {  // sf_y -> z
-      k_bwd_sf<<<k->sf_grid, kTPB, 0, st>>>(lv.pad, lv.pad_len, c->mv.ioffset, c->mv.ja,
-                                            c->mv.diag, k->a, k->d, k->rdi, k->sf_y, z,
-                                            k->sf_ctl, k->S, k->sf_spin);
-    }
+    level::launch<double>(c, st, 1, forward ? wave::kForward : wave::kBackward, k->lv, b, z,
+                          wave_control(k), k->sf_absent_row);
     return;
   }
   for (int l = 0; l < lv.count; ++l) {
@@ -1378,17 +1206,8 @@ static int run_solver(fcg_context *c, int kind, const double *a, const double *s
                                                      k->p32, k->S, k->partials);
     FCG_CHECK_LAUNCH(c, "mixed set-up");
   }
-  if (kind != SK_DPCG && k->sf_on) {  // factor diagonal in one sync-free launch
-    if (wave_sweeps(c)) {
-      if ((rc = start_wave(c, kind == SK_BICG))) return rc;
-    } else {
-      k_sf_fill<<<grid_for(c->n, c->num_sms), kTPB, 0, c->stream>>>(c->n, k->d, nullptr,
-                                                                    k->sf_ctl);
-      k_factor_sf<<<k->sf_grid, kTPB, 0, c->stream>>>(
-          c->lf.pad, c->lf.pad_len, c->mv.ioffset, c->mv.ja, c->mv.diag, c->tpos, k->a, k->d,
-          k->rdi, k->sf_ctl, k->S, k->sf_spin, kind == SK_BICG);
-    }
-    FCG_CHECK_LAUNCH(c, "factor");
+  if (kind != SK_DPCG && k->sf_on) {  // the mixed solver too reports a pivot that breaks down
+    if ((rc = start_sweeps(c, kind == SK_BICG))) return rc;
   } else if (kind != SK_DPCG) {  // factor diagonal, level by level
     for (int l = 0; l < c->lf.count; ++l) {
       int start = c->lf.ptr[l], cnt = c->lf.ptr[l + 1] - c->lf.ptr[l];

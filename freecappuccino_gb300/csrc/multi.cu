@@ -22,6 +22,7 @@
 #include "fcg_internal.h"
 #include "krylov_common.cuh"
 #include "launch.h"
+#include "level_sweep.cuh"
 #include "wave_sweep.cuh"
 
 namespace fcg {
@@ -55,16 +56,16 @@ struct MultiState {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   int G = 0;
-  // one-launch DILU sweeps (as krylov.cu): forward results and the control words
-  // {forward claim counter, backward claim counter, -, error}
-  DBuf sfb;
-  float *y32 = nullptr;
+  // one-launch DILU sweeps (as krylov.cu): the control words {forward claim counter,
+  // backward claim counter, -, error}, and on meshes that are no block the arrays in level
+  // order (level_sweep.cuh)
+  DBuf sfb, lbuf;
   int *ctl = nullptr;
-  int sf_grid = 0;
+  level::Arrays<float> lv{};
   bool sf_on = true;
   // the wavefront-tiled sweeps on hex blocks (wave_sweep.cuh), every system's tiles in one
-  // launch: five transport systems at 128^3 to 1e-10 take 9.4 ms, 76.3 with the
-  // row-claiming sweeps below, whose rows poll the second-level cache at every level
+  // launch: five transport systems at 128^3 to 1e-10 take 9.4 ms, 76.3 with row-claiming
+  // sweeps in the natural order
   bool wave_on = false;
   DBuf wbuf;
   wave::Arrays<float> wv{};
@@ -80,6 +81,7 @@ void destroy_multi(MultiState *m) {
   m->buf.release();
   m->sfb.release();
   m->wbuf.release();
+  m->lbuf.release();
   delete m;
 }
 
@@ -314,170 +316,6 @@ __global__ void k_m_bwd(const int *__restrict__ rows, int count, long long nnz, 
   }
 }
 
-// --- DILU sweeps in one launch (the scheme of krylov.cu's k_fwd_sf): rows claimed in
-// level order by warps, each waiting on the FP32 values it reads, which are filled with
-// a signalling-NaN sentinel before the sweep.  The same row arithmetic as the level
-// kernels above.
-constexpr unsigned kSent32 = 0x7f80deadu;
-constexpr int kSfSpin = 1 << 20;
-
-__device__ __forceinline__ float ld_relaxed32(const float *p) {
-  unsigned v;
-  asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return __uint_as_float(v);
-}
-
-__device__ __forceinline__ void st_relaxed32(float *p, float x) {
-  asm volatile("st.relaxed.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(__float_as_uint(x)) : "memory");
-}
-
-__device__ __forceinline__ bool sent32(float v) { return __float_as_uint(v) == kSent32; }
-
-__device__ __forceinline__ float sf_value32(const float *p, const int *err, bool *ok) {
-  float v = ld_relaxed32(p);
-  if (!sent32(v)) return v;
-  for (int it = 0; it < kSfSpin; ++it) {
-    if (it >= 16) __nanosleep(32);
-    v = ld_relaxed32(p);
-    if (!sent32(v)) return v;
-    if ((it & 63) == 63 && *(volatile const int *)err) break;
-  }
-  *ok = false;
-  return v;
-}
-
-__device__ __forceinline__ void sf_fail32(int *err, MScal *S) {
-  if (atomicExch(err, 1) == 0) atomicCAS(&S->status, 0, FCG_ERR_TIMEOUT);
-}
-
-__global__ void k_m_sf_fill(long long count, float *__restrict__ o1, float *__restrict__ o2,
-                            int *ctl) {
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    ctl[0] = 0;
-    ctl[1] = 0;
-    ctl[3] = 0;
-  }
-  const float s = __uint_as_float(kSent32);
-  FCG_GRID_STRIDE(i, count) {
-    o1[i] = s;
-    if (o2) o2[i] = s;
-  }
-}
-
-// Claims the next 32 entries of the level list for the calling warp (-1: none left).
-__device__ __forceinline__ int sf_claim(int *ctr) {
-  int base = 0;
-  if ((threadIdx.x & 31) == 0) base = atomicAdd(ctr, 32);
-  return __shfl_sync(0xffffffffu, base, 0);
-}
-
-template <int NS>
-__global__ void k_m_fwd_sf(const int *__restrict__ rows, int len, long long nnz, int n,
-                           const int *__restrict__ io, const int *__restrict__ ja,
-                           const int *__restrict__ dg, const float *__restrict__ a32,
-                           const float *__restrict__ d32, const float *__restrict__ b, float *y,
-                           int *ctl, MScal *S) {
-  if (inner_done(S)) return;
-  for (;;) {
-    const int base = sf_claim(&ctl[0]);
-    if (base >= len) break;
-    const int i = rows[base + (threadIdx.x & 31)];
-    if (i < 0) continue;
-    float zi[NS], di[NS];
-#pragma unroll
-    for (int k = 0; k < NS; ++k) {
-      di[k] = d32[(long long)k * n + i];
-      zi[k] = b[(long long)k * n + i] * di[k];
-    }
-    bool ok = true;
-    for (int q = io[i]; q < dg[i]; ++q) {
-      const int j = ja[q];
-      float v[NS];
-#pragma unroll
-      for (int k = 0; k < NS; ++k) v[k] = ld_relaxed32(&y[(long long)k * n + j]);
-#pragma unroll
-      for (int k = 0; k < NS; ++k) {
-        if (sent32(v[k])) v[k] = sf_value32(&y[(long long)k * n + j], &ctl[3], &ok);
-        zi[k] = __fmaf_rn(-(a32[k * nnz + q] * di[k]), v[k], zi[k]);
-      }
-    }
-    if (!ok) sf_fail32(&ctl[3], S);
-#pragma unroll
-    for (int k = 0; k < NS; ++k)
-      st_relaxed32(&y[(long long)k * n + i], zi[k]);
-  }
-}
-
-template <int NS>
-__global__ void k_m_bwd_sf(const int *__restrict__ rows, int len, long long nnz, int n,
-                           const int *__restrict__ io, const int *__restrict__ ja,
-                           const int *__restrict__ dg, const float *__restrict__ a32,
-                           const float *__restrict__ d32, const float *__restrict__ y, float *z,
-                           int *ctl, MScal *S) {
-  if (inner_done(S)) return;
-  const float small = (float)S->small;
-  for (;;) {
-    const int base = sf_claim(&ctl[1]);
-    if (base >= len) break;
-    const int i = rows[base + (threadIdx.x & 31)];
-    if (i < 0) continue;
-    float zi[NS], di[NS];
-#pragma unroll
-    for (int k = 0; k < NS; ++k) {
-      di[k] = d32[(long long)k * n + i];
-      zi[k] = y[(long long)k * n + i] * (di[k] / (di[k] + small));
-    }
-    bool ok = true;
-    for (int q = dg[i] + 1; q < io[i + 1]; ++q) {
-      const int j = ja[q];
-      float v[NS];
-#pragma unroll
-      for (int k = 0; k < NS; ++k) v[k] = ld_relaxed32(&z[(long long)k * n + j]);
-#pragma unroll
-      for (int k = 0; k < NS; ++k) {
-        if (sent32(v[k])) v[k] = sf_value32(&z[(long long)k * n + j], &ctl[3], &ok);
-        zi[k] = __fmaf_rn(-(a32[k * nnz + q] * di[k]), v[k], zi[k]);
-      }
-    }
-    if (!ok) sf_fail32(&ctl[3], S);
-#pragma unroll
-    for (int k = 0; k < NS; ++k) st_relaxed32(&z[(long long)k * n + i], zi[k]);
-  }
-}
-
-template <int NS>
-__global__ void k_m_factor_sf(const int *__restrict__ rows, int len, long long nnz, int n,
-                              const int *__restrict__ io, const int *__restrict__ ja,
-                              const int *__restrict__ dg, const int *__restrict__ tpos,
-                              const float *__restrict__ a32, float *d32, int *ctl, MScal *S) {
-  for (;;) {
-    const int base = sf_claim(&ctl[0]);
-    if (base >= len) break;
-    const int i = rows[base + (threadIdx.x & 31)];
-    if (i < 0) continue;
-    float di[NS];
-#pragma unroll
-    for (int k = 0; k < NS; ++k) di[k] = a32[k * nnz + dg[i]];
-    bool ok = true;
-    for (int q = io[i]; q < dg[i]; ++q) {
-      const int j = ja[q];
-#pragma unroll
-      for (int k = 0; k < NS; ++k) {
-        const float *a = a32 + k * nnz;
-        const float dj = sf_value32(&d32[(long long)k * n + j], &ctl[3], &ok);
-        di[k] = __fmaf_rn(-(a[q] * a[tpos[q]]), dj, di[k]);
-      }
-    }
-    if (!ok) sf_fail32(&ctl[3], S);
-#pragma unroll
-    for (int k = 0; k < NS; ++k) {
-      const float inv = 1.0f / di[k];
-      st_relaxed32(&d32[(long long)k * n + i], inv);
-      if (!isfinite(inv)) atomicCAS(&S->status, 0, FCG_ERR_PIVOT);
-    }
-  }
-}
-
 // y = A z for every system; sums y.w (and y.y when TWO) per system.
 template <int NS, bool TWO>
 __global__ void __launch_bounds__(kTPB, 4)
@@ -614,7 +452,7 @@ __global__ void k_m_correct(int n, double *__restrict__ x, const float *__restri
 // host side
 // ---------------------------------------------------------------------------
 wave::Control wave_control(MultiState *m) {
-  return wave::Control{m->ctl, nullptr, &m->S->status, &m->S->idone, kSfSpin};
+  return wave::Control{m->ctl, nullptr, &m->S->status, &m->S->idone, 1 << 20};
 }
 
 template <int NS>
@@ -628,17 +466,8 @@ struct Launch {
       return;
     }
     if (m->sf_on) {
-      if (fwd) {  // b -> y32, after the sentinel fill of y32 and z
-        k_m_sf_fill<<<grid_for((long long)NS * m->n, c->num_sms), kTPB, 0, st>>>(
-            (long long)NS * m->n, m->y32, z, m->ctl);
-        k_m_fwd_sf<NS><<<m->sf_grid, kTPB, 0, st>>>(lv.pad, lv.pad_len, m->nnz, m->n,
-                                                    c->mv.ioffset, c->mv.ja, c->mv.diag, m->a32,
-                                                    m->d32, b, m->y32, m->ctl, m->S);
-      } else {  // y32 -> z
-        k_m_bwd_sf<NS><<<m->sf_grid, kTPB, 0, st>>>(lv.pad, lv.pad_len, m->nnz, m->n,
-                                                    c->mv.ioffset, c->mv.ja, c->mv.diag, m->a32,
-                                                    m->d32, m->y32, z, m->ctl, m->S);
-      }
+      level::launch<float>(c, st, NS, fwd ? wave::kForward : wave::kBackward, m->lv, b, z,
+                           wave_control(m));
       return;
     }
     for (int l = 0; l < lv.count; ++l) {
@@ -675,14 +504,9 @@ struct Launch {
     if (m->wave_on)
       return wave::start(c, NS, m->nnz, m->a32, true, (float)(double)1e-20f, m->wv,
                          wave_control(m));
-    if (m->sf_on) {
-      k_m_sf_fill<<<grid_for((long long)NS * m->n, c->num_sms), kTPB, 0, c->stream>>>(
-          (long long)NS * m->n, m->d32, nullptr, m->ctl);
-      k_m_factor_sf<NS><<<m->sf_grid, kTPB, 0, c->stream>>>(
-          c->lf.pad, c->lf.pad_len, m->nnz, m->n, c->mv.ioffset, c->mv.ja, c->mv.diag, c->tpos,
-          m->a32, m->d32, m->ctl, m->S);
-      return FCG_OK;
-    }
+    if (m->sf_on)
+      return level::start(c, NS, m->nnz, m->a32, true, (float)(double)1e-20f, m->lv,
+                          wave_control(m));
     for (int l = 0; l < c->lf.count; ++l) {
       const int start = c->lf.ptr[l], cnt = c->lf.ptr[l + 1] - c->lf.ptr[l];
       k_m_factor<NS><<<(cnt + kTPB - 1) / kTPB, kTPB, 0, c->stream>>>(
@@ -834,22 +658,23 @@ int ensure_multi(fcg_context *c, int ns) {
     *v = f;
     f += nn;
   }
-  FCG_CUDA_TRY(c, m->sfb.ensure(nn * sizeof(float) + 16 * sizeof(int)));
-  FCG_CUDA_TRY(c, cudaMemset(m->sfb.p, 0, nn * sizeof(float) + 16 * sizeof(int)));
-  m->y32 = m->sfb.as<float>();
-  m->ctl = (int *)(m->y32 + nn);
-  m->sf_grid = c->num_sms * 2;
+  FCG_CUDA_TRY(c, m->sfb.ensure(4 * sizeof(int)));
+  FCG_CUDA_TRY(c, cudaMemset(m->sfb.p, 0, 4 * sizeof(int)));
+  m->ctl = m->sfb.as<int>();
   {
     const char *e = std::getenv("FCG_SWEEP");
     m->sf_on = !(e && std::string(e) == "levels");
     m->wave_on = c->hex.ok && !(e && (std::string(e) == "levels" || std::string(e) == "rows"));
   }
   m->wbuf.release();
-  m->wv = wave::Arrays<float>{};
-  if (m->wave_on) {
-    int rc = wave::allocate(c, ns, m->wbuf, m->wv);
-    if (rc) return rc;
-  }
+  m->lbuf.release();
+  m->n = 0;  // until the arrays are there
+  int rc = FCG_OK;
+  if (m->wave_on)
+    rc = wave::allocate(c, ns, m->wbuf, m->wv);
+  else if (m->sf_on)
+    rc = level::allocate(c, ns, m->lbuf, m->lv);
+  if (rc) return rc;
   m->n = c->n;
   m->ns = ns;
   m->nnz = c->nnz;

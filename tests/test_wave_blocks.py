@@ -1,7 +1,8 @@
 """The wavefront-tiled DIC / DILU sweeps on blocks of unequal extents against the
-row-claiming form: tiles and clusters cut at the block's edge, blocks of fewer planes than
-a tile has steps, and more planes than one launch takes.  Both forms use the same row
-arithmetic in the same entry order, so the same bits."""
+level-ordered form: tiles and clusters cut at the block's edge, blocks of fewer planes than
+a tile has steps, and more planes than one launch takes.  And the level-ordered form on a
+mesh whose rows hold more entries of one triangle than it keeps in registers.  All forms
+use the same row arithmetic in the same entry order, so the same bits."""
 import os
 
 import numpy as np
@@ -106,3 +107,24 @@ def test_tiled_multi_rhs_sweeps_equal_row_sweeps(dims, nsys):
     (x1, r1), (x2, r2) = out
     assert np.array_equal(x1, x2) and [r.iters for r in r1] == [r.iters for r in r2]
     assert all(r.converged for r in r1)
+
+
+@pytest.mark.parametrize("N", [3, 11])
+def test_level_order_of_a_scattered_numbering(N):
+    """Cells numbered at random: up to six entries in a row's triangle, uneven levels."""
+    m = fcg.hex_mesh(N, 0.2, seed=3)
+    p = np.random.default_rng(N).permutation(m.numCells)
+    inv = np.argsort(p)
+    m.owner = (p[m.owner - 1] + 1).astype(np.int32)
+    m.neighbour = (p[m.neighbour - 1] + 1).astype(np.int32)
+    for k in ("xc", "yc", "zc", "vol"):
+        setattr(m, k, np.ascontiguousarray(getattr(m, k)[inv]))
+    ctxs = [_context(m), _context(m, "levels")]
+    mu, phi, su0 = poisson_system(m)
+    a, su = ctxs[0].laplacian(mu, phi, su0)
+    for solver in ("iccg", "bicgstab"):
+        for _ in range(2):
+            r, o = [getattr(c, solver)(a, su, np.zeros(m.numCells), 0.0, 5) for c in ctxs]
+            assert np.array_equal(r.fi, o.fi) and r.resl == o.resl, (N, solver)
+    for c in ctxs:
+        c.close()
