@@ -3,14 +3,22 @@
 // a CUDA graph.  No reference counterpart as a batch: every system follows dpcg.f90:3-154
 // exactly as fcg_dpcg does (same recurrence, constants and L1 stop test per system).
 //
-// Work is a list of items (system, run of 32-row slices).  The kernel walks all systems
-// in lockstep phases -- initial residual; then per CG iteration p-update | SpMV | update
-// -- separated by a grid-wide barrier; the items of a phase are spread over the CTAs, so
-// a large system uses the whole GPU and small ones share it.  Each system's global sums
-// are formed deterministically: every item stores its block partial, and the CTA that
-// commits the system's last item (ticket counter) adds the partials in item order with a
-// fixed block tree and updates that system's scalars.  A system that meets its stop test
-// drops out (its items are skipped); the kernel ends when none is left.
+// Work is a list of items, runs of 32-row slices, numbered over the systems still
+// iterating.  The kernel walks all systems in lockstep phases -- initial residual; then per
+// CG iteration p-update | SpMV | update -- separated by a grid-wide barrier.  In every
+// phase each CTA takes an equal, consecutive share of the items, so a large system uses the
+// whole GPU, small ones share it, and a CTA meets one system or two: it forms one partial
+// sum per system it meets.  The CTA that arrives last at the barrier adds every system's
+// partials in CTA order and updates the systems' scalars before it opens the barrier, so a
+// solve gives the same bits run after run.  A system that meets its stop test drops out and
+// the items are numbered anew; the kernel ends when none is left.
+//
+// What bounds it: memory latency in the phases, hidden by resident warps (the kernel is held
+// to 40 registers, six CTAs an SM), and three barriers of 2 to 5 us a sweep.  12 systems of
+// 5.9 M cells, a sweep: p 47, SpMV 147, update 101 us.  With one partial sum, block barrier
+// and ticket per item and two CTAs an SM a sweep took 811 us, and at its best setting
+// (five CTAs, items of 128 slices) 360; rows of eight loads issued together, which need 64
+// registers, 444.
 //
 // The grid barrier spins with a bounded number of polls; a CTA that gives up sets the
 // error flag, which ends every CTA at its next barrier, and the call returns
@@ -32,21 +40,17 @@ namespace fcg {
 namespace {
 
 constexpr int kMaxBatch = 64;
+constexpr int kResident = 6;  // CTAs an SM the kernel's registers are held to
 
 // One system of the batch (device-resident; the host writes the inputs before a solve).
 struct BSys {
   SellView sv;
-  int n, item0, nitems, nsw;
+  int n, nitems, nsw;
   const double *val, *invd, *su;
   double *x, *res, *p, *q;
   double sor, small, tol;
   double res0, resl, sk, s0, bet, alf, l2r, l2b;
-  int iter, active, converged, status, early, pad;
-  unsigned int ticket, pad2;
-};
-
-struct BItem {
-  int sys, s0, s1;  // slices [s0, s1) of system sys
+  int iter, active, converged, status, early;
 };
 
 struct BCtl {
@@ -55,46 +59,135 @@ struct BCtl {
   int nactive;              // systems still iterating
 };
 
-// Grid-wide barrier with a bounded wait.  Returns false when any CTA has given up.
-__device__ bool grid_sync(BCtl *ctl, long long limit) {
-  __shared__ int ok_sh;
+// The items of the systems still iterating, base[k] .. base[k+1] system k's, in equal shares:
+// q items for every CTA and one more for the first rem.
+struct Split {
+  int base[kMaxBatch + 1], n[kMaxBatch];
+  int q, rem;
+  __device__ __forceinline__ int begin(int b) const { return b * q + min(b, rem); }
+  // the CTA whose share holds `item`
+  __device__ __forceinline__ int cta_of(int item) const {
+    return item < rem * (q + 1) ? item / (q + 1) : rem + (item - rem * (q + 1)) / q;
+  }
+};
+
+__device__ void make_split(Split &sp, const BSys *sys, int nsys, bool all) {
+  __syncthreads();
+  for (int k = threadIdx.x; k < nsys; k += blockDim.x)
+    sp.n[k] = all || __ldcg(&sys[k].active) ? sys[k].nitems : 0;
+  __syncthreads();
+  for (int k = threadIdx.x; k <= nsys; k += blockDim.x) {
+    int t = 0;
+    for (int j = 0; j < k; ++j) t += sp.n[j];
+    sp.base[k] = t;
+    if (k == nsys) {
+      sp.q = t / (int)gridDim.x;
+      sp.rem = t % (int)gridDim.x;
+    }
+  }
+  __syncthreads();
+}
+
+// Runs f(k, s0, s1) on this CTA's share: slices [s0, s1) of system k.
+template <class F>
+__device__ __forceinline__ void for_share(const Split &sp, const BSys *sys, int nsys, int spi,
+                                          F &&f) {
+  int i = sp.begin(blockIdx.x);
+  const int end = sp.begin(blockIdx.x + 1);
+  for (int k = 0; i < end; ++k) {
+    if (sp.base[k + 1] <= i) continue;
+    const int e = min(end, sp.base[k + 1]);
+    f(k, (i - sp.base[k]) * spi,
+      (int)min((long long)(e - sp.base[k]) * spi, (long long)sys[k].sv.nslices));
+    i = e;
+  }
+}
+
+// This CTA's block sums of system k: part[(k gridDim + CTA) 2 ..].
+template <int NV>
+__device__ __forceinline__ void put_partial(double (&v)[NV], double *part, int k,
+                                            double (*sh)[kWarps]) {
+  block_sum<NV>(v, sh);
+  if (threadIdx.x == 0)
+#pragma unroll
+    for (int q = 0; q < NV; ++q) part[((long long)k * gridDim.x + blockIdx.x) * 2 + q] = v[q];
+}
+
+// Grid-wide barrier with a bounded wait.  The CTA that arrives last runs `last` (all its
+// threads) before the others go on: everything they wrote is visible to it.  Returns false
+// when any CTA has given up.
+template <class F>
+__device__ __forceinline__ bool grid_sync(BCtl *ctl, long long limit, F &&last) {
+  __shared__ int state_sh;  // 0: gave up, 1: passed, 2: last to arrive
+  __shared__ unsigned int gen_sh;
   __syncthreads();
   if (threadIdx.x == 0) {
-    int ok = 1;
-    volatile unsigned int *vgen = &ctl->gen;
-    volatile int *verr = &ctl->err;
-    if (*verr) {
-      ok = 0;
-    } else {
-      const unsigned int g = *vgen;
+    state_sh = 0;
+    if (!*(volatile int *)&ctl->err) {
+      const unsigned int g = *(volatile unsigned int *)&ctl->gen;
+      gen_sh = g;
       __threadfence();
-      const unsigned int arrived = atomicAdd(&ctl->count, 1u);
-      if (arrived == gridDim.x - 1) {
-        ctl->count = 0u;
-        __threadfence();
-        atomicAdd(&ctl->gen, 1u);
-      } else {
-        long long polls = 0;
-        while (*vgen == g) {
-          if (*verr) {
-            ok = 0;
-            break;
-          }
-          if (++polls > limit) {
-            atomicExch(&ctl->err, 1);
-            ok = 0;
-            break;
-          }
-          __nanosleep(64);
-        }
-      }
+      state_sh = atomicAdd(&ctl->count, 1u) == gridDim.x - 1 ? 2 : 1;
     }
+  }
+  __syncthreads();
+  if (state_sh == 2) {
     __threadfence();
-    ok_sh = ok;
+    last();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      ctl->count = 0u;
+      __threadfence();
+      atomicAdd(&ctl->gen, 1u);
+    }
+  } else if (state_sh == 1 && threadIdx.x == 0) {
+    long long polls = 0;
+    while (*(volatile unsigned int *)&ctl->gen == gen_sh) {
+      const bool over = ++polls > limit;
+      if (over) atomicCAS(&ctl->err, 0, 1);
+      if (over || *(volatile int *)&ctl->err) {
+        state_sh = 0;
+        break;
+      }
+      __nanosleep(20);
+    }
   }
   __syncthreads();
   __threadfence();
-  return ok_sh != 0;
+  return state_sh != 0;
+}
+__device__ __forceinline__ bool grid_sync(BCtl *ctl, long long limit) {
+  return grid_sync(ctl, limit, [] {});
+}
+
+// In the last CTA of a barrier: every system's partials added in CTA order (one warp a
+// system), then fin(k, sums) by one lane.
+template <class F>
+__device__ __forceinline__ void sum_systems(const Split &sp, int nsys, const double *part, F &&fin) {
+  const int lane = threadIdx.x & 31;
+  for (int k = threadIdx.x >> 5; k < nsys; k += kWarps) {
+    if (sp.n[k] == 0) continue;
+    const int b0 = sp.cta_of(sp.base[k]), b1 = sp.cta_of(sp.base[k + 1] - 1);
+    const double *pk = part + (long long)k * gridDim.x * 2;
+    double v[2] = {0.0, 0.0};
+    for (int b = b0 + lane; b <= b1; b += 8 * 32) {
+      double2 t[8];  // the loads of eight partials in flight together
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        t[u] = b + 32 * u <= b1 ? __ldcg(reinterpret_cast<const double2 *>(pk + 2 * (b + 32 * u)))
+                                : make_double2(0.0, 0.0);
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        v[0] += t[u].x;
+        v[1] += t[u].y;
+      }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int q = 0; q < 2; ++q) v[q] += __shfl_down_sync(0xffffffffu, v[q], o);
+    if (lane == 0) fin(k, v);
+  }
 }
 
 // Row sum of A x for lane `lane` of slice `slice` (FP64, slot order = CSR column order).
@@ -116,38 +209,6 @@ __device__ __forceinline__ double brow(const SellView &s, int n, const double *_
       acc += __ldg(&val[base + (long long)j * 32]) * x[__ldg(&s.off[op + 32 * j + lane])];
   }
   return acc;
-}
-
-// Stores this item's block sums; in the CTA that commits the system's last item, returns
-// true with the system's totals in v (all threads), summed over the items in order.
-template <int NV>
-__device__ bool item_commit(double (&v)[NV], double *part, int it, BSys &S,
-                            double (*sh)[kWarps]) {
-  __shared__ int last_sh;
-  block_sum<NV>(v, sh);
-  if (threadIdx.x == 0) {
-#pragma unroll
-    for (int k = 0; k < NV; ++k) part[(long long)it * 2 + k] = v[k];
-    __threadfence();
-    const unsigned int t = atomicAdd(&S.ticket, 1u);
-    last_sh = (t == (unsigned int)S.nitems - 1u);
-  }
-  __syncthreads();
-  if (!last_sh) return false;
-  __threadfence();
-  double s[NV];
-#pragma unroll
-  for (int k = 0; k < NV; ++k) s[k] = 0.0;
-  for (int j = threadIdx.x; j < S.nitems; j += blockDim.x)
-#pragma unroll
-    for (int k = 0; k < NV; ++k) s[k] += __ldcg(&part[(long long)(S.item0 + j) * 2 + k]);
-  block_sum<NV>(s, sh);
-  if (threadIdx.x == 0) {
-    S.ticket = 0u;
-#pragma unroll
-    for (int k = 0; k < NV; ++k) v[k] = s[k];
-  }
-  return true;
 }
 
 __device__ __noinline__ void fin_init(BSys &S, BCtl *ctl, double l1, double sk) {
@@ -186,107 +247,137 @@ __device__ __noinline__ void fin_update(BSys &S, BCtl *ctl, double resl, double 
   }
 }
 
-__global__ void __launch_bounds__(kTPB)
-    k_batch_dpcg(BSys *sys, const BItem *__restrict__ items, int nitems, double *part,
-                 BCtl *ctl, int max_loops, long long spin_limit, int absent_block) {
+// The phases' row loops and the barriers' sums are functions of their own, so that each is
+// allocated registers for itself: inlined into the kernel they spilled.
+
+// res = su - A x of slices [s0, s1), or only its squares (FINAL) with those of su.
+template <bool FINAL>
+__device__ __noinline__ double2 residual_rows(const BSys &S, int s0, int s1) {
+  const int lane = threadIdx.x & 31;
+  double2 v = {0.0, 0.0};
+  for (int slice = s0 + (threadIdx.x >> 5); slice < s1; slice += kWarps) {
+    const int r = slice * 32 + lane;
+    const double ax = brow(S.sv, S.n, S.val, S.x, slice, lane);
+    if (r < S.n) {
+      const double rr = S.su[r] - ax;
+      if (FINAL) {
+        v.x += rr * rr;
+        v.y += S.su[r] * S.su[r];
+      } else {
+        S.res[r] = rr;
+        v.x += fabs(rr);
+        v.y += rr * (rr * __ldg(&S.invd[r]));
+      }
+    }
+  }
+  return v;
+}
+
+// q = A p of slices [s0, s1), returns p.q
+__device__ __noinline__ double spmv_rows(const BSys &S, int s0, int s1) {
+  const int lane = threadIdx.x & 31;
+  const SellView sv = S.sv;
+  const int n = S.n;
+  const double *val = S.val, *p = S.p;
+  double *q = S.q, v = 0.0;
+  for (int slice = s0 + (threadIdx.x >> 5); slice < s1; slice += kWarps) {
+    const int r = slice * 32 + lane;
+    const double t = brow(sv, n, val, p, slice, lane);
+    if (r < n) {
+      q[r] = t;
+      v += p[r] * t;
+    }
+  }
+  return v;
+}
+
+enum Phase { kInit, kSpmv, kUpdate, kFinal };
+
+__device__ __noinline__ void close_phase(int phase, BSys *sys, BCtl *ctl, const Split &sp, int nsys,
+                                         const double *part) {
+  sum_systems(sp, nsys, part, [&](int k, double *v) {
+    if (phase == kInit) fin_init(sys[k], ctl, v[0], v[1]);
+    if (phase == kSpmv) fin_spmv(sys[k], v[0]);
+    if (phase == kUpdate) fin_update(sys[k], ctl, v[0], v[1]);
+    if (phase == kFinal) {
+      sys[k].l2r = v[0];
+      sys[k].l2b = v[1];
+    }
+  });
+}
+
+__global__ void __launch_bounds__(kTPB, kResident)
+    k_batch_dpcg(BSys *sys, int nsys, int spi, double *part, BCtl *ctl, int max_loops,
+                 long long spin_limit, int absent_block) {
   __shared__ double sh[2][kWarps];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  __shared__ Split sp;
   // diagnostics only (fcg_batch_set_wait_test): one CTA never reaches a barrier, so the
   // others' bounded waits run out and the solve ends with FCG_ERR_TIMEOUT
   if ((int)blockIdx.x == absent_block) return;
+  make_split(sp, sys, nsys, true);
   // initial residual res = su - A x, res0 = sum|res|, sk = sum res^2 / a_PP (dpcg.f90:51-90)
-  for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
-    const BItem I = items[it];
-    BSys &S = sys[I.sys];
-    double v[2] = {0.0, 0.0};
-    for (int slice = I.s0 + warp; slice < I.s1; slice += kWarps) {
-      const int r = slice * 32 + lane;
-      const double ax = brow(S.sv, S.n, S.val, S.x, slice, lane);
-      if (r < S.n) {
-        const double rr = S.su[r] - ax;
-        S.res[r] = rr;
-        v[0] += fabs(rr);
-        v[1] += rr * (rr * __ldg(&S.invd[r]));
-      }
-    }
-    if (item_commit<2>(v, part, it, S, sh) && threadIdx.x == 0) fin_init(S, ctl, v[0], v[1]);
-  }
-  if (!grid_sync(ctl, spin_limit)) return;
+  for_share(sp, sys, nsys, spi, [&](int k, int s0, int s1) {
+    const double2 t = residual_rows<false>(sys[k], s0, s1);
+    double v[2] = {t.x, t.y};
+    put_partial<2>(v, part, k, sh);
+  });
+  if (!grid_sync(ctl, spin_limit, [&] { close_phase(kInit, sys, ctl, sp, nsys, part); })) return;
+  int active = nsys;
   for (int loop = 0;; ++loop) {
-    if (__ldcg(&ctl->nactive) <= 0) break;
+    const int now = __ldcg(&ctl->nactive);
+    if (now <= 0) break;
     if (loop > max_loops) {
       if (blockIdx.x == 0 && threadIdx.x == 0) atomicExch(&ctl->err, 2);
       return;
     }
+    if (now != active) make_split(sp, sys, nsys, false);
+    active = now;
     // p = a_PP^-1 res + bet p (dpcg.f90:85-100)
-    for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
-      const BItem I = items[it];
-      BSys &S = sys[I.sys];
-      if (!__ldcg(&S.active)) continue;
+    for_share(sp, sys, nsys, spi, [&](int k, int s0, int s1) {
+      const BSys &S = sys[k];
       const double bet = __ldcg(&S.bet);
-      const int r0 = I.s0 * 32, r1 = min(S.n, I.s1 * 32);
-      for (int r = r0 + threadIdx.x; r < r1; r += blockDim.x)
-        S.p[r] = S.res[r] * __ldg(&S.invd[r]) + bet * S.p[r];
-    }
+      double *p = S.p;
+      const double *res = S.res, *invd = S.invd;
+      const int r1 = min(S.n, s1 * 32);
+#pragma unroll 4
+      for (int r = s0 * 32 + threadIdx.x; r < r1; r += kTPB)
+        p[r] = res[r] * __ldg(&invd[r]) + bet * p[r];
+    });
     if (!grid_sync(ctl, spin_limit)) return;
     // q = A p, alf = sk / p.q (dpcg.f90:105-121)
-    for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
-      const BItem I = items[it];
-      BSys &S = sys[I.sys];
-      if (!__ldcg(&S.active)) continue;
-      double v[2] = {0.0, 0.0};
-      for (int slice = I.s0 + warp; slice < I.s1; slice += kWarps) {
-        const int r = slice * 32 + lane;
-        const double q = brow(S.sv, S.n, S.val, S.p, slice, lane);
-        if (r < S.n) {
-          S.q[r] = q;
-          v[0] += S.p[r] * q;
-        }
-      }
-      if (item_commit<2>(v, part, it, S, sh) && threadIdx.x == 0) fin_spmv(S, v[0]);
-    }
-    if (!grid_sync(ctl, spin_limit)) return;
+    for_share(sp, sys, nsys, spi, [&](int k, int s0, int s1) {
+      double v[1] = {spmv_rows(sys[k], s0, s1)};
+      put_partial<1>(v, part, k, sh);
+    });
+    if (!grid_sync(ctl, spin_limit, [&] { close_phase(kSpmv, sys, ctl, sp, nsys, part); })) return;
     // x += alf p, res -= alf q, resl = sum|res|, next sk (dpcg.f90:124-142)
-    for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
-      const BItem I = items[it];
-      BSys &S = sys[I.sys];
-      if (!__ldcg(&S.active)) continue;
+    for_share(sp, sys, nsys, spi, [&](int k, int s0, int s1) {
+      const BSys &S = sys[k];
       const double alf = __ldcg(&S.alf);
+      double *x = S.x, *res = S.res;
+      const double *p = S.p, *q = S.q, *invd = S.invd;
+      const int r1 = min(S.n, s1 * 32);
       double v[2] = {0.0, 0.0};
-      for (int slice = I.s0 + warp; slice < I.s1; slice += kWarps) {
-        const int r = slice * 32 + lane;
-        if (r < S.n) {
-          S.x[r] = S.x[r] + alf * S.p[r];
-          const double rr = S.res[r] - alf * S.q[r];
-          S.res[r] = rr;
-          v[0] += fabs(rr);
-          v[1] += rr * (rr * __ldg(&S.invd[r]));
-        }
+#pragma unroll 4
+      for (int r = s0 * 32 + threadIdx.x; r < r1; r += kTPB) {
+        x[r] = x[r] + alf * p[r];
+        const double rr = res[r] - alf * q[r];
+        res[r] = rr;
+        v[0] += fabs(rr);
+        v[1] += rr * (rr * __ldg(&invd[r]));
       }
-      if (item_commit<2>(v, part, it, S, sh) && threadIdx.x == 0)
-        fin_update(S, ctl, v[0], v[1]);
-    }
-    if (!grid_sync(ctl, spin_limit)) return;
+      put_partial<2>(v, part, k, sh);
+    });
+    if (!grid_sync(ctl, spin_limit, [&] { close_phase(kUpdate, sys, ctl, sp, nsys, part); })) return;
   }
   // final FP64 check of every system: ||su - A x||^2, ||su||^2
-  for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
-    const BItem I = items[it];
-    BSys &S = sys[I.sys];
-    double v[2] = {0.0, 0.0};
-    for (int slice = I.s0 + warp; slice < I.s1; slice += kWarps) {
-      const int r = slice * 32 + lane;
-      const double ax = brow(S.sv, S.n, S.val, S.x, slice, lane);
-      if (r < S.n) {
-        const double rr = S.su[r] - ax;
-        v[0] += rr * rr;
-        v[1] += S.su[r] * S.su[r];
-      }
-    }
-    if (item_commit<2>(v, part, it, S, sh) && threadIdx.x == 0) {
-      S.l2r = v[0];
-      S.l2b = v[1];
-    }
-  }
+  make_split(sp, sys, nsys, true);
+  for_share(sp, sys, nsys, spi, [&](int k, int s0, int s1) {
+    const double2 t = residual_rows<true>(sys[k], s0, s1);
+    double v[2] = {t.x, t.y};
+    put_partial<2>(v, part, k, sh);
+  });
+  grid_sync(ctl, spin_limit, [&] { close_phase(kFinal, sys, ctl, sp, nsys, part); });
 }
 
 }  // namespace
@@ -299,17 +390,17 @@ struct fcg_batch {
   int device = 0, num_sms = 0, occ = 1;
   cudaStream_t stream = nullptr;
   std::string err;
-  int slices_per_item = 32, blocks_per_sm = 2;
-  DBuf dsys, ditems, dpart, dctl;
+  int slices_per_item = 8, blocks_per_sm = 1;
+  DBuf dsys, dpart, dctl;
   BSys *hsys = nullptr;  // pinned: the graph copies it to the device at every launch
   BCtl *hctl = nullptr;
-  int nitems = 0, items_for = -1;
+  int items_for = -1;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   int graph_grid = 0, graph_loops = 0;
-  long long spin_limit = 1LL << 22;  // polls of 64 ns sleeps per barrier wait: over 0.25 s
+  long long spin_limit = 1LL << 22;  // polls per barrier wait: over a second
   int absent_block = -1;              // diagnostics: a CTA that skips the barriers
-  cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+  cudaEvent_t ev0 = nullptr, ev1 = nullptr, loaded = nullptr;
 };
 
 namespace {
@@ -333,22 +424,12 @@ void drop_graph(fcg_batch *b) {
   b->graph = nullptr;
 }
 
-// Items of `slices_per_item` slices for every system, system after system.
+// Item counts of `slices_per_item` slices for every system, and room for the partials.
 int build_items(fcg_batch *b) {
   if (b->items_for == b->slices_per_item) return FCG_OK;
-  std::vector<BItem> items;
-  for (size_t k = 0; k < b->ctx.size(); ++k) {
-    const int ns = b->ctx[k]->sv.nslices;
-    b->hsys[k].item0 = (int)items.size();
-    for (int s0 = 0; s0 < ns; s0 += b->slices_per_item)
-      items.push_back({(int)k, s0, std::min(ns, s0 + b->slices_per_item)});
-    b->hsys[k].nitems = (int)items.size() - b->hsys[k].item0;
-  }
-  b->nitems = (int)items.size();
-  B_TRY(b, b->ditems.ensure(sizeof(BItem) * items.size()));
-  B_TRY(b, b->dpart.ensure(sizeof(double) * 2 * items.size()));
-  B_TRY(b, cudaMemcpy(b->ditems.p, items.data(), sizeof(BItem) * items.size(),
-                      cudaMemcpyHostToDevice));
+  for (size_t k = 0; k < b->ctx.size(); ++k)
+    b->hsys[k].nitems = (b->ctx[k]->sv.nslices + b->slices_per_item - 1) / b->slices_per_item;
+  B_TRY(b, b->dpart.ensure(sizeof(double) * 2 * b->ctx.size() * (size_t)b->num_sms * b->occ));
   b->items_for = b->slices_per_item;
   drop_graph(b);
   return FCG_OK;
@@ -371,9 +452,8 @@ int enqueue(fcg_batch *b, cudaStream_t st, int grid, int max_loops) {
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   B_TRY(b, cudaLaunchKernelEx(&cfg, k_batch_dpcg, b->dsys.as<BSys>(),
-                              (const BItem *)b->ditems.as<BItem>(), b->nitems,
-                              b->dpart.as<double>(), b->dctl.as<BCtl>(), max_loops,
-                              b->spin_limit, b->absent_block));
+                              (int)ns, b->slices_per_item, b->dpart.as<double>(),
+                              b->dctl.as<BCtl>(), max_loops, b->spin_limit, b->absent_block));
   return FCG_OK;
 }
 
@@ -450,11 +530,13 @@ int load_system(fcg_batch *b, int k, const double *a, const double *su, const do
   BatchVecs v;
   if ((rc = batch_load(c, (const double *)da, (const double *)dsu, (const double *)dfi, &v)))
     return bfail(b, rc, fcg_last_error(c));
-  B_TRY(b, cudaStreamSynchronize(c->stream));
+  if (c->stream != b->stream) {  // the batch runs after this system's copies
+    B_TRY(b, cudaEventRecord(b->loaded, c->stream));
+    B_TRY(b, cudaStreamWaitEvent(b->stream, b->loaded, 0));
+  }
   BSys &S = b->hsys[k];
-  const int item0 = S.item0, nitems = S.nitems;
+  const int nitems = S.nitems;
   std::memset(&S, 0, sizeof S);
-  S.item0 = item0;
   S.nitems = nitems;
   S.sv = c->sv;
   S.n = c->n;
@@ -500,13 +582,19 @@ extern "C" int fcg_batch_create(fcg_context *const *ctxs, int nsys, fcg_batch **
       cudaMallocHost(&b->hctl, sizeof(BCtl)) != cudaSuccess ||
       b->dsys.ensure(sizeof(BSys) * nsys) != cudaSuccess ||
       b->dctl.ensure(sizeof(BCtl)) != cudaSuccess || cudaEventCreate(&b->ev0) != cudaSuccess ||
-      cudaEventCreate(&b->ev1) != cudaSuccess) {
+      cudaEventCreate(&b->ev1) != cudaSuccess ||
+      cudaEventCreateWithFlags(&b->loaded, cudaEventDisableTiming) != cudaSuccess) {
     cudaGetLastError();
     fcg_batch_destroy(b);
     return FCG_ERR_CUDA;
   }
   b->occ = occ;
-  b->blocks_per_sm = std::min(2, occ);
+  // two slices a warp before another CTA an SM: two systems of 16^3 take 18 us a sweep with
+  // four CTAs an SM and 26 with six, 12 systems of 5.9 M cells 330 and 295
+  long long slices = 0;
+  for (int k = 0; k < nsys; ++k) slices += ctxs[k]->sv.nslices;
+  const long long warps = (long long)b->num_sms * kWarps;
+  b->blocks_per_sm = (int)std::min<long long>(occ, 1 + slices / (2 * warps));
   std::memset(b->hsys, 0, sizeof(BSys) * nsys);
   if (build_items(b)) {
     fcg_batch_destroy(b);
@@ -523,10 +611,10 @@ extern "C" int fcg_batch_destroy(fcg_batch *b) {
   drop_graph(b);
   if (b->ev0) cudaEventDestroy(b->ev0);
   if (b->ev1) cudaEventDestroy(b->ev1);
+  if (b->loaded) cudaEventDestroy(b->loaded);
   if (b->hsys) cudaFreeHost(b->hsys);
   if (b->hctl) cudaFreeHost(b->hctl);
   b->dsys.release();
-  b->ditems.release();
   b->dpart.release();
   b->dctl.release();
   delete b;
@@ -596,7 +684,6 @@ extern "C" int fcg_batch_dpcg(fcg_batch *b, const double *const *a, const double
     B_TRY(b, cudaMemcpyAsync(dfi[k], S.x, n1, cudaMemcpyDeviceToDevice, c->stream));
     int r2 = stage_out(c, fi[k], dfi[k], n1, hfi[k] != 0);
     if (r2) return bfail(b, r2, fcg_last_error(c));
-    B_TRY(b, cudaStreamSynchronize(c->stream));
     if (resor && S.iter > 0) resor[k] = S.res0;  // dpcg.f90:139
     if (rep) {
       rep[k].res0 = S.res0;
@@ -607,6 +694,9 @@ extern "C" int fcg_batch_dpcg(fcg_batch *b, const double *const *a, const double
       rep[k].seconds = ms * 1e-3;
     }
   }
+  for (int k = 0; k < ns; ++k)
+    if (k == 0 || b->ctx[k]->stream != b->ctx[k - 1]->stream)
+      B_TRY(b, cudaStreamSynchronize(b->ctx[k]->stream));
   if (timeout) return timeout;
   for (int k = 0; k < ns; ++k)
     if (b->hsys[k].status)
