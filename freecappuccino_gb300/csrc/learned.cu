@@ -154,11 +154,14 @@ __global__ void __launch_bounds__(kTPB, 8)
   if (reduce_commit<1>(v, partials, ticket) && threadIdx.x == 0) out[0] = v[0];
 }
 
-__global__ void k_lp_features(MeshView m, const double *__restrict__ s64,
-                              const double *__restrict__ vsum, float *__restrict__ feat) {
+// Features 2..5 depend on the mesh alone: once per mesh the handle serves in a row.  Their
+// 100 FP64 operations a cell, six divisions among them, took most of the 77 us that all
+// features took at 745 k cells on every new matrix.
+__global__ void k_lp_features_mesh(MeshView m, const double *__restrict__ vsum,
+                                   float *__restrict__ feat) {
   const double vmean = vsum[0] / m.n;
   FCG_GRID_STRIDE(i, m.n) {
-    const double v = m.vol[i], d = 1.0 / (s64[i] * s64[i]);
+    const double v = m.vol[i];
     const double h = (double)cbrtf((float)v);  // the features are FP32
     double ax = 0.0, ay = 0.0, az = 0.0;
     for (int e = m.cf_ptr[i]; e < m.cf_ptr[i + 1]; ++e) {
@@ -175,12 +178,21 @@ __global__ void k_lp_features(MeshView m, const double *__restrict__ s64,
     }
     const double a2 = 2.0 * h * h;
     const long long nn = m.n;  // feature-major: feature k of cell i at k * n + i
-    feat[i] = 0.f;
-    feat[nn + i] = logf((float)(d / h)) - 1.7917595f;  // log 6
     feat[2 * nn + i] = logf((float)(v / vmean));
     feat[3 * nn + i] = (float)(ax / a2 - 1.0);
     feat[4 * nn + i] = (float)(ay / a2 - 1.0);
     feat[5 * nn + i] = (float)(az / a2 - 1.0);
+  }
+}
+
+// Feature 1 of the matrix and a zero residual feature.
+__global__ void k_lp_features_matrix(int n, const double *__restrict__ vol,
+                                     const double *__restrict__ s64, float *__restrict__ feat) {
+  FCG_GRID_STRIDE(i, n) {
+    const double d = 1.0 / (s64[i] * s64[i]);
+    const double h = (double)cbrtf((float)vol[i]);
+    feat[i] = 0.f;
+    feat[(long long)n + i] = logf((float)(d / h)) - 1.7917595f;  // log 6
   }
 }
 
@@ -572,12 +584,22 @@ __global__ void __launch_bounds__(kTPB)
   const float k2 = 2.0f / fmaxf(sums[1], 1e-30f);
   const float wl = prm[lp::oWout + lane];
   float gw = 0.f, gb = 0.f;
-  for (long long i = (long long)blockIdx.x * (kTPB / 32) + warp; i < n;
-       i += (long long)gridDim.x * (kTPB / 32)) {
-    const float dy = k2 * ad[i];
-    dh[i * C + lane] = dy * wl;
-    gw += dy * bf(h[i * C + lane]);
-    gb += dy;
+  const long long nw = (long long)gridDim.x * (kTPB / 32);
+  for (long long i0 = (long long)blockIdx.x * (kTPB / 32) + warp; i0 < n; i0 += 4 * nw) {
+    float dy[4], hv[4];  // four cells' loads in flight
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const long long i = i0 + u * nw;
+      dy[u] = i < n ? k2 * ad[i] : 0.f;
+      hv[u] = i < n ? bf(h[i * C + lane]) : 0.f;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const long long i = i0 + u * nw;
+      if (i < n) dh[i * C + lane] = dy[u] * wl;
+      gw += dy[u] * hv[u];
+      gb += dy[u];
+    }
   }
   acc[warp][lane] = gw;
   if (lane == 0) acc[warp][C] = gb;
@@ -593,81 +615,183 @@ __global__ void __launch_bounds__(kTPB)
 // dh_prev = dh + dh_x (skip connection), dm kept for the aggregation.  Per-block sums of
 // dz [h; m]^T and dz give the gradient of W_l and b_l.  Block b owns a contiguous run of
 // cells, staged 64 at a time in shared memory.
-__global__ void __launch_bounds__(kTPB, 2)
+//
+// Two FP32 products of 2,048 multiply-adds a cell.  What bounded the first form (274 us at
+// 64^3, one output and two shared-memory loads for every one or two multiply-adds) was the
+// shared-memory pipe; here a thread holds a 4 x 4 block of the first product and a 4 x 8
+// block of the second (a quarter of the tile's cells; the quarters are added at the end),
+// 16-byte loads, 8 to 11 multiply-adds a load: about 88 us.
+__global__ void __launch_bounds__(kTPB, 3)
     k_lp_layer_bwd(int n, const float *__restrict__ dh, const float *__restrict__ z,
                    const __nv_bfloat16 *__restrict__ hin, const float *__restrict__ m,
                    const float *__restrict__ prm_l, float *__restrict__ dh_prev,
                    float *__restrict__ dm, float *__restrict__ part /* [G][kLayerParams] */) {
-  __shared__ float W[C * 2 * C];
-  __shared__ float dzs[lp::kBwdTile][C + 1];
-  __shared__ float xs[lp::kBwdTile][2 * C];
-  for (int t = threadIdx.x; t < C * 2 * C; t += blockDim.x) W[t] = prm_l[t];
-  float gw[8], gbias = 0.f;  // thread t: weights t + 256 q, bias t (t < 32)
+  constexpr int B = lp::kBwdTile, ZS = C + 4, XS = 2 * C + 4;  // padded rows
+  __shared__ __align__(16) float W[C * 2 * C];
+  __shared__ __align__(16) float dzs[B][ZS];
+  __shared__ __align__(16) float xs[B][XS];
+  static_assert(B * XS >= 2 * C * C + C, "the closing sums reuse the tile");
+  const int t = threadIdx.x;
+  for (int i = t; i < C * 2 * C; i += kTPB) W[i] = prm_l[i];
+  float gw[4][8], gb[4];
 #pragma unroll
-  for (int q = 0; q < 8; ++q) gw[q] = 0.f;
-  __syncthreads();
+  for (int o = 0; o < 4; ++o) {
+    gb[o] = 0.f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) gw[o][k] = 0.f;
+  }
+  const int cg = t & 15, rg = t >> 4;                        // columns 4 cg.., cells 4 rg..
+  const int kg = t >> 6, og = (t >> 3) & 7, xg = t & 7;      // cells 16 kg.., outputs 4 og..
   const long long per = ((long long)n + gridDim.x - 1) / gridDim.x;
   const long long c0 = (long long)blockIdx.x * per, c1 = min((long long)n, c0 + per);
-  for (long long base = c0; base < c1; base += lp::kBwdTile) {
-    const int cnt = (int)min((long long)lp::kBwdTile, c1 - base);
-    for (int t = threadIdx.x; t < cnt * C; t += blockDim.x) {
-      const int cl = t / C, ch = t % C;
-      const long long o = (base + cl) * C + ch;
-      dzs[cl][ch] = z[o] > 0.f ? dh[o] : 0.f;
-      xs[cl][ch] = bf(hin[o]);
-      xs[cl][C + ch] = m[o];
-    }
+  for (long long base = c0; base < c1; base += B) {
+    const int cnt = (int)min((long long)B, c1 - base);
     __syncthreads();
-    for (int t = threadIdx.x; t < cnt * C; t += blockDim.x) {
-      const int cl = t / C, k = t % C;
-      float gh = 0.f, gm = 0.f;
-#pragma unroll 8
-      for (int o = 0; o < C; ++o) {
-        const float dz = dzs[cl][o];
-        gh += W[o * 2 * C + k] * dz;
-        gm += W[o * 2 * C + C + k] * dz;
+#pragma unroll
+    for (int q = 0; q < B * C / 4 / kTPB; ++q) {
+      const int i = t + q * kTPB, cl = i >> 3, c4 = 4 * (i & 7);
+      float4 dz = make_float4(0.f, 0.f, 0.f, 0.f), mv = dz, hv = dz;
+      if (cl < cnt) {
+        const long long o = (base + cl) * C + c4;
+        const float4 zv = *reinterpret_cast<const float4 *>(z + o);
+        const float4 dv = *reinterpret_cast<const float4 *>(dh + o);
+        mv = *reinterpret_cast<const float4 *>(m + o);
+        const uint2 hq = *reinterpret_cast<const uint2 *>(hin + o);
+        const __nv_bfloat16 *he = reinterpret_cast<const __nv_bfloat16 *>(&hq);
+        hv = make_float4(bf(he[0]), bf(he[1]), bf(he[2]), bf(he[3]));
+        dz = make_float4(zv.x > 0.f ? dv.x : 0.f, zv.y > 0.f ? dv.y : 0.f,
+                         zv.z > 0.f ? dv.z : 0.f, zv.w > 0.f ? dv.w : 0.f);
       }
-      const long long oo = (base + cl) * C + k;
-      dh_prev[oo] = dh[oo] + gh;
-      dm[oo] = gm;
+      *reinterpret_cast<float4 *>(&dzs[cl][c4]) = dz;
+      *reinterpret_cast<float4 *>(&xs[cl][c4]) = hv;
+      *reinterpret_cast<float4 *>(&xs[cl][C + c4]) = mv;
     }
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const int idx = threadIdx.x + q * kTPB;
-      const int o = idx / (2 * C), k = idx % (2 * C);
-      float sacc = 0.f;
-      for (int cl = 0; cl < cnt; ++cl) sacc += dzs[cl][o] * xs[cl][k];
-      gw[q] += sacc;
-    }
-    if (threadIdx.x < C)
-      for (int cl = 0; cl < cnt; ++cl) gbias += dzs[cl][threadIdx.x];
     __syncthreads();
-  }
-  float *pb = part + (long long)blockIdx.x * lp::kLayerParams;
+    float acc[4][4];
 #pragma unroll
-  for (int q = 0; q < 8; ++q) pb[threadIdx.x + q * kTPB] = gw[q];
-  if (threadIdx.x < C) pb[2 * C * C + threadIdx.x] = gbias;
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) acc[r][k] = 0.f;
+#pragma unroll 2
+    for (int o = 0; o < C; o += 4) {
+      float4 d[4], w[4];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) d[r] = *reinterpret_cast<const float4 *>(&dzs[4 * rg + r][o]);
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        w[j] = *reinterpret_cast<const float4 *>(&W[(o + j) * 2 * C + 4 * cg]);
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          const float dv = j == 0 ? d[r].x : j == 1 ? d[r].y : j == 2 ? d[r].z : d[r].w;
+          acc[r][0] += w[j].x * dv;
+          acc[r][1] += w[j].y * dv;
+          acc[r][2] += w[j].z * dv;
+          acc[r][3] += w[j].w * dv;
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int cl = 4 * rg + r;
+      if (cl >= cnt) break;
+      float4 v = make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
+      if (cg < C / 4) {
+        const long long o = (base + cl) * C + 4 * cg;
+        const float4 dv = *reinterpret_cast<const float4 *>(dh + o);
+        v = make_float4(dv.x + v.x, dv.y + v.y, dv.z + v.z, dv.w + v.w);
+        *reinterpret_cast<float4 *>(dh_prev + o) = v;
+      } else {
+        *reinterpret_cast<float4 *>(dm + (base + cl) * C + 4 * cg - C) = v;
+      }
+    }
+#pragma unroll 4
+    for (int cl = 16 * kg; cl < 16 * kg + 16; ++cl) {
+      const float4 d = *reinterpret_cast<const float4 *>(&dzs[cl][4 * og]);
+      const float4 xa = *reinterpret_cast<const float4 *>(&xs[cl][8 * xg]);
+      const float4 xb = *reinterpret_cast<const float4 *>(&xs[cl][8 * xg + 4]);
+      const float dv[4] = {d.x, d.y, d.z, d.w};
+#pragma unroll
+      for (int o = 0; o < 4; ++o) {
+        gw[o][0] += dv[o] * xa.x;
+        gw[o][1] += dv[o] * xa.y;
+        gw[o][2] += dv[o] * xa.z;
+        gw[o][3] += dv[o] * xa.w;
+        gw[o][4] += dv[o] * xb.x;
+        gw[o][5] += dv[o] * xb.y;
+        gw[o][6] += dv[o] * xb.z;
+        gw[o][7] += dv[o] * xb.w;
+        gb[o] += dv[o];
+      }
+    }
+  }
+  // the four quarters' sums, added in order
+  float *red = &xs[0][0];
+  for (int g = 0; g < 4; ++g) {
+    __syncthreads();
+    if (kg != g) continue;
+#pragma unroll
+    for (int o = 0; o < 4; ++o) {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        float *p = &red[(4 * og + o) * 2 * C + 8 * xg + k];
+        *p = g == 0 ? gw[o][k] : *p + gw[o][k];
+      }
+      if (xg == 0) {
+        float *p = &red[2 * C * C + 4 * og + o];
+        *p = g == 0 ? gb[o] : *p + gb[o];
+      }
+    }
+  }
+  __syncthreads();
+  float *pb = part + (long long)blockIdx.x * lp::kLayerParams;
+  for (int i = t; i < lp::kLayerParams; i += kTPB) pb[i] = red[i];
 }
 
-// dh_prev += Ahat dm (Ahat of the pressure system is symmetric); a warp per cell, a
-// lane per channel.
-__global__ void __launch_bounds__(kTPB)
+// dh_prev += Ahat dm (Ahat of the pressure system is symmetric); eight lanes a cell, four
+// channels a lane, the loads of a row of at most eight slots in flight together, four blocks
+// an SM: about 71 us at 64^3 (96 with the 68 registers of three blocks, 83 with the spills
+// of five); a lane a channel and a slot at a time took 128.
+__global__ void __launch_bounds__(kTPB, 4)
     k_lp_agg_bwd(SellView s, int n, const float *__restrict__ aval,
                  const float *__restrict__ dm, float *__restrict__ dh_prev) {
-  const int lane = threadIdx.x & 31;
-  for (long long r = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < n;
-       r += ((long long)gridDim.x * blockDim.x) >> 5) {
-    const int slice = (int)(r >> 5), ln = (int)(r & 31);
+  FCG_GRID_STRIDE(g, 8LL * n) {
+    const long long r = g >> 3;
+    const int q = 4 * (int)(g & 7), slice = (int)(r >> 5), ln = (int)(r & 31);
     const long long base = __ldg(&s.ptr[slice]) + ln;
     const int w = __ldg(&s.width[slice]), op = __ldg(&s.offp[slice]);
     const bool uni = __ldg(&s.kind[slice]) == 0;
-    float acc = 0.f;
-    for (int j = 0; j < w; ++j) {
-      long long col = uni ? r + __ldg(&s.off[op + j]) : __ldg(&s.off[op + 32 * j + ln]);
-      col = col < 0 ? 0 : (col >= n ? n - 1 : col);
-      acc += __ldg(&aval[base + (long long)j * 32]) * dm[col * C + lane];
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int j0 = 0; j0 < w; j0 += 8) {
+      float a[8];
+      float4 x[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        a[j] = 0.f;
+        if (j0 + j < w) {
+          long long col = uni ? r + __ldg(&s.off[op + j0 + j])
+                              : __ldg(&s.off[op + 32 * (j0 + j) + ln]);
+          col = col < 0 ? 0 : (col >= n ? n - 1 : col);
+          a[j] = __ldg(&aval[base + (long long)(j0 + j) * 32]);
+          x[j] = __ldg(reinterpret_cast<const float4 *>(dm + col * C + q));
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (j0 + j < w) {
+          acc.x += a[j] * x[j].x;
+          acc.y += a[j] * x[j].y;
+          acc.z += a[j] * x[j].z;
+          acc.w += a[j] * x[j].w;
+        }
     }
-    dh_prev[r * C + lane] += acc;
+    float4 *o = reinterpret_cast<float4 *>(dh_prev + r * C + q);
+    float4 v = *o;
+    v.x += acc.x;
+    v.y += acc.y;
+    v.z += acc.z;
+    v.w += acc.w;
+    *o = v;
   }
 }
 
@@ -680,13 +804,22 @@ __global__ void __launch_bounds__(kTPB)
   float g[F + 1];
 #pragma unroll
   for (int k = 0; k <= F; ++k) g[k] = 0.f;
-  for (long long i = (long long)blockIdx.x * (kTPB / 32) + warp; i < n;
-       i += (long long)gridDim.x * (kTPB / 32)) {
-    const long long o = i * C + lane;
-    const float dz = z0[o] > 0.f ? dh[o] : 0.f;
+  const long long nw = (long long)gridDim.x * (kTPB / 32);
+  for (long long i0 = (long long)blockIdx.x * (kTPB / 32) + warp; i0 < n; i0 += 2 * nw) {
+    float dz[2], f[2][F];  // two cells' loads in flight
 #pragma unroll
-    for (int k = 0; k < F; ++k) g[k] += dz * feat[k * (long long)n + i];
-    g[F] += dz;
+    for (int u = 0; u < 2; ++u) {
+      const long long i = i0 + u * nw, o = i * C + lane;
+      dz[u] = i < n && z0[o] > 0.f ? dh[o] : 0.f;
+#pragma unroll
+      for (int k = 0; k < F; ++k) f[u][k] = i < n ? feat[k * (long long)n + i] : 0.f;
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+#pragma unroll
+      for (int k = 0; k < F; ++k) g[k] += dz[u] * f[u][k];
+      g[F] += dz[u];
+    }
   }
 #pragma unroll
   for (int k = 0; k < F; ++k) acc[warp][lane * F + k] = g[k];
@@ -699,12 +832,22 @@ __global__ void __launch_bounds__(kTPB)
   }
 }
 
-// grad[t] = sum over blocks, in block order, of part[b][t]
-__global__ void k_lp_sum_parts(const float *__restrict__ part, int nblocks, int width,
-                               float *__restrict__ grad) {
-  FCG_GRID_STRIDE(t, width) {
-    double sacc = 0.0;
-    for (int b = 0; b < nblocks; ++b) sacc += part[(long long)b * width + t];
+// grad[t] = sum over blocks of part[b][t] in FP64: a block takes 32 values, its warps every
+// eighth partial each, and their sums are added in warp order.  One thread adding all of a
+// value's partials, one dependent FP64 sum each, took 62 us for 304.
+__global__ void __launch_bounds__(kTPB)
+    k_lp_sum_parts(const float *__restrict__ part, int nblocks, int width,
+                   float *__restrict__ grad) {
+  __shared__ double sums[kTPB / 32][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, t = blockIdx.x * 32 + lane;
+  double sacc = 0.0;
+  if (t < width)
+#pragma unroll 8
+    for (int b = warp; b < nblocks; b += kTPB / 32) sacc += part[(long long)b * width + t];
+  sums[warp][lane] = sacc;
+  __syncthreads();
+  if (warp == 0 && t < width) {
+    for (int w = 1; w < kTPB / 32; ++w) sacc += sums[w][lane];
     grad[t] = (float)sacc;
   }
 }
@@ -1193,12 +1336,16 @@ int hex_status(fcg_learned *Lp, fcg_context *c) {
 int compute_features(fcg_learned *Lp, fcg_context *c) {
   int rc = ensure_workspace(Lp, c, false);
   if (rc) return rc;
-  const int G = reduction_grid(c);
-  double *red = Lp->red.as<double>();
-  k_lp_volsum<<<G, kTPB, 0, c->stream>>>(c->n, c->mv.vol, red, Lp->scal.as<unsigned>() + 16,
-                                         red + lp::kMaxDir * kMaxBlocks);
-  k_lp_features<<<grid_for(c->n, c->num_sms), kTPB, 0, c->stream>>>(
-      c->mv, scale64(c), red + lp::kMaxDir * kMaxBlocks, Lp->feat.as<float>());
+  if (Lp->fuid != c->uid || Lp->fgen != c->bind_gen) {
+    double *red = Lp->red.as<double>();
+    k_lp_volsum<<<reduction_grid(c), kTPB, 0, c->stream>>>(
+        c->n, c->mv.vol, red, Lp->scal.as<unsigned>() + 16, red + lp::kMaxDir * kMaxBlocks);
+    k_lp_features_mesh<<<grid_for(c->n, c->num_sms), kTPB, 0, c->stream>>>(
+        c->mv, red + lp::kMaxDir * kMaxBlocks, Lp->feat.as<float>());
+    LP_TRY(Lp, cudaGetLastError());
+  }
+  k_lp_features_matrix<<<grid_for(c->n, c->num_sms), kTPB, 0, c->stream>>>(
+      c->n, c->mv.vol, scale64(c), Lp->feat.as<float>());
   LP_TRY(Lp, cudaGetLastError());
   if ((rc = hex_prepare(Lp, c))) return rc;
   Lp->fuid = c->uid;
@@ -1354,27 +1501,31 @@ int loss_grad(fcg_learned *Lp, fcg_context *c, const float *r, const float *e) {
       gy = aadvec;
     }
   }
-  const int GB = c->num_sms * 2;  // blocks of the weight-gradient kernels
+  const int GB = c->num_sms * 3;  // blocks of the layers' backward
+  const int GS = c->num_sms * 8;  // and of the narrower ones (their partials fit the same room)
+  static_assert(8 * (lp::C * lp::F + lp::C) <= 3 * lp::kLayerParams, "partials");
   float *part = Lp->part.as<float>();
   float *grad = Lp->grad.as<float>();
   const size_t hs = (size_t)n * lp::C;
   const __nv_bfloat16 *H = Lp->hbuf.as<__nv_bfloat16>();
   float *dh = Lp->dh.as<float>(), *dh2 = Lp->dh2.as<float>();
-  k_lp_out_bwd<<<GB, kTPB, 0, st>>>(n, gy, sums, H + (size_t)lp::L * hs, prm, dh, part);
-  k_lp_sum_parts<<<1, kTPB, 0, st>>>(part, GB, lp::C + 1, grad + lp::oWout);
+  k_lp_out_bwd<<<GS, kTPB, 0, st>>>(n, gy, sums, H + (size_t)lp::L * hs, prm, dh, part);
+  auto sum_parts = [&](int blocks, int width, float *out) {
+    k_lp_sum_parts<<<(width + 31) / 32, kTPB, 0, st>>>(part, blocks, width, out);
+  };
+  sum_parts(GS, lp::C + 1, grad + lp::oWout);
   for (int l = lp::L - 1; l >= 0; --l) {
     k_lp_layer_bwd<<<GB, kTPB, 0, st>>>(n, dh, Lp->zbuf.as<float>() + (l + 1) * hs, H + l * hs,
                                         Lp->mbuf.as<float>() + l * hs,
                                         prm + lp::oLayer0 + l * lp::kLayerParams, dh2,
                                         Lp->dm.as<float>(), part);
-    k_lp_sum_parts<<<grid_for(lp::kLayerParams, c->num_sms), kTPB, 0, st>>>(
-        part, GB, lp::kLayerParams, grad + lp::oLayer0 + l * lp::kLayerParams);
-    k_lp_agg_bwd<<<grid_for((long long)n * 32, c->num_sms), kTPB, 0, st>>>(
+    sum_parts(GB, lp::kLayerParams, grad + lp::oLayer0 + l * lp::kLayerParams);
+    k_lp_agg_bwd<<<grid_for((long long)n * 8, c->num_sms), kTPB, 0, st>>>(
         c->sv, n, scaled32(c), Lp->dm.as<float>(), dh2);
     std::swap(dh, dh2);
   }
-  k_lp_embed_bwd<<<GB, kTPB, 0, st>>>(n, dh, Lp->zbuf.as<float>(), Lp->feat.as<float>(), part);
-  k_lp_sum_parts<<<1, kTPB, 0, st>>>(part, GB, lp::C * lp::F + lp::C, grad + lp::oWin);
+  k_lp_embed_bwd<<<GS, kTPB, 0, st>>>(n, dh, Lp->zbuf.as<float>(), Lp->feat.as<float>(), part);
+  sum_parts(GS, lp::C * lp::F + lp::C, grad + lp::oWin);
   LP_TRY(Lp, cudaGetLastError());
   return FCG_OK;
 }
@@ -1432,7 +1583,7 @@ extern "C" int fcg_lp_create(int device, unsigned long long seed, fcg_learned **
   const size_t pb = sizeof(float) * lp::P;
   if (Lp->params.ensure(pb) || Lp->adam_m.ensure(pb) || Lp->adam_v.ensure(pb) ||
       Lp->grad.ensure(pb) || Lp->wbf.ensure(sizeof(__nv_bfloat16) * lp::L * 2 * lp::C * lp::C) ||
-      Lp->part.ensure(sizeof(float) * (size_t)Lp->num_sms * 2 * lp::kLayerParams) ||
+      Lp->part.ensure(sizeof(float) * (size_t)Lp->num_sms * 3 * lp::kLayerParams) ||
       Lp->red.ensure(sizeof(double) * (lp::kMaxDir * kMaxBlocks + 8)) ||
       Lp->scal.ensure(sizeof(float) * 64) || cudaMalloc(&Lp->S, sizeof(lp::LScal)) ||
       cudaMallocHost(&Lp->hS, sizeof(lp::LScal)) ||
