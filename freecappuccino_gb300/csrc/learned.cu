@@ -65,7 +65,7 @@ constexpr int P = oBout + 1;
 static_assert(P == FCG_LP_PARAMS, "parameter count must match the header");
 static_assert(oBin == oWin + C * F && oLayer0 == oBin + C, "parameter layout");
 constexpr int kBwdTile = 64;            // cells per shared-memory tile of the layer backward
-static_assert(kTileC == C && kTileStride == 2 * C + 8, "tile layout of lp_tile.cuh");
+static_assert(kTileC == C, "row layout of lp_tile.cuh");
 constexpr int kRed = 8;                 // reduction tickets
 constexpr int kMaxDir = 8;              // most previous directions the FCG keeps
 
@@ -253,7 +253,7 @@ __global__ void __launch_bounds__(kTPB, 4)
         __align__(16) __nv_bfloat16 hv[8];
 #pragma unroll
         for (int o = 0; o < 4; ++o) {  // channels 2p, 2p+1: z = fma(w, f, z) for k in order
-          const int pr = g * 4 + o;
+          const int pr = o * 4 + g;  // the stored order of lp::hpos
           float2 z = w2[C / 2 * F + pr];
 #pragma unroll
           for (int k = 0; k < F; ++k) z = __ffma2_rn(w2[pr * F + k], make_float2(f[k], f[k]), z);
@@ -290,35 +290,28 @@ using lp::fma8;
 // measured 14% slower at 256^3.  A warp owns 16 cells (one tile) at a time and takes them
 // in two rounds of 8: four lanes per cell, eight channels per lane, sum
 // m = Ahat h over the cell's sliced row -- for uniform slices the column offsets,
-// values and neighbour activations of four slots are loaded before any is used -- and
-// write the [h; m] row (64 BF16) into the warp's shared tile.  4 k-steps x 4 n-blocks of
-// mma.sync give the 16 x 32 pre-activation; the epilogue adds the bias, applies the ReLU
-// and the skip connection, puts h' back into the tile, and the tile leaves in 16-byte
-// stores (16 consecutive cells = 1 KB contiguous).  Rows of the tile and of W_l are
-// padded to 72 elements so that the fragment loads of the 8 row groups fall in distinct
-// banks.
+// values and neighbour activations of four slots are loaded before any is used.  The lane
+// then holds its fragments of the [h; m] rows (lp::hpos), the product and epilogue run in
+// registers, and h' leaves in 16-byte stores (16 consecutive cells = 1 KB contiguous).
 __global__ void __launch_bounds__(kTPB, 4)
     k_lp_layer(SellView s, int n, const float *__restrict__ aval,
                const __nv_bfloat16 *__restrict__ hin, __nv_bfloat16 *__restrict__ hout,
                const __nv_bfloat16 *__restrict__ wl, const float *__restrict__ bl,
                float *__restrict__ mout, float *__restrict__ zout, const int *done) {
   if (stopped(done)) return;
-  constexpr int TS = lp::kTileStride;
-  __shared__ __align__(16) __nv_bfloat16 wsm[C * TS];
-  __shared__ float bsm[C];
-  __shared__ __align__(16) __nv_bfloat16 tile[kTPB / 32][16 * TS];
-  for (int t = threadIdx.x; t < C * 2 * C; t += blockDim.x)
-    wsm[(t / (2 * C)) * TS + t % (2 * C)] = wl[t];
-  if (threadIdx.x < C) bsm[threadIdx.x] = bl[threadIdx.x];
+  __shared__ uint4 wf[lp::kFragWords];
+  lp::load_frags(wf, wl);
   __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31;
   const int qc = 8 * (lane & 3);
-  __nv_bfloat16 *tw = tile[warp];
+  float bias[8];
+  lp::load_bias(bias, bl, lane);
   const int ntiles = (n + 15) / 16;
   const int nwarps = (int)(((long long)gridDim.x * blockDim.x) >> 5);
   for (int tt = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5); tt < ntiles;
        tt += nwarps) {
-#pragma unroll 1
+    uint4 ownq[2], mq[2], o[2];
+#pragma unroll
     for (int rd = 0; rd < 2; ++rd) {
       const int rloc = rd * 8 + (lane >> 2);
       const int r = tt * 16 + rloc;
@@ -360,37 +353,34 @@ __global__ void __launch_bounds__(kTPB, 4)
         }
         own = __ldg(reinterpret_cast<const uint4 *>(hq + (long long)r * C));
       }
-      __align__(16) __nv_bfloat16 mb[8];
-      lp::tile_put_row(tw, rloc, qc, own, acc, mb);
-      if (mout && r < n) {
-        float4 *mo = reinterpret_cast<float4 *>(mout + (long long)r * C + qc);
-        mo[0] = make_float4(bf(mb[0]), bf(mb[1]), bf(mb[2]), bf(mb[3]));
-        mo[1] = make_float4(bf(mb[4]), bf(mb[5]), bf(mb[6]), bf(mb[7]));
+      ownq[rd] = own;
+      mq[rd] = lp::round8(acc);
+      if (mout && r < n) {  // channels 8 i + 2 tg, + 1
+        const __nv_bfloat162 *e = reinterpret_cast<const __nv_bfloat162 *>(&mq[rd]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          *reinterpret_cast<float2 *>(mout + (long long)r * C + 8 * i + qc / 4) =
+              __bfloat1622float2(e[i]);
       }
     }
-    __syncwarp();
-    lp::tile_dense(tw, wsm, bsm, lane, [&](int rr, int col, float z0, float z1) {
+    lp::dense(ownq, mq, wf, bias, lane, o, [&](int rr, int col, float z0, float z1) {
       const int cell = tt * 16 + rr;
       if (zout && cell < n)
         *reinterpret_cast<float2 *>(zout + (long long)cell * C + col) = make_float2(z0, z1);
     });
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const int idx = lane + 32 * k, rr = idx >> 2, part = idx & 3;
-      const int cell = tt * 16 + rr;
-      if (cell < n)
-        *reinterpret_cast<uint4 *>(hout + (long long)cell * C + 8 * part) =
-            *reinterpret_cast<const uint4 *>(tw + rr * TS + 8 * part);
+    for (int rd = 0; rd < 2; ++rd) {
+      const int cell = tt * 16 + rd * 8 + (lane >> 2);
+      if (cell < n) *reinterpret_cast<uint4 *>(hout + (long long)cell * C + qc) = o[rd];
     }
-    __syncwarp();
   }
 }
 
 // The same layer as two streaming kernels (k_lp_agg, k_lp_dense), bit-identical to
 // k_lp_layer: the aggregation writes m = Ahat h rounded to BF16, four threads per cell
 // and eight channels per thread with all neighbour loads of a row in flight at full
-// occupancy; the dense kernel streams the [h; m] rows of a 16-cell tile into the warp's
-// shared tile and runs the same mma.sync product and epilogue.
+// occupancy; the dense kernel streams the [h; m] rows of 16 cells into a warp's registers
+// and runs the same mma.sync product and epilogue.
 __global__ void __launch_bounds__(kTPB)
     k_lp_agg(SellView s, int n, const float *__restrict__ aval,
              const __nv_bfloat16 *__restrict__ hin, __nv_bfloat16 *__restrict__ mout,
@@ -429,10 +419,7 @@ __global__ void __launch_bounds__(kTPB)
              __ldg(reinterpret_cast<const uint4 *>(hq + (long long)col * C)));
       }
     }
-    __align__(16) __nv_bfloat16 mb[8];
-#pragma unroll
-    for (int c = 0; c < 8; ++c) mb[c] = __float2bfloat16(acc[c]);
-    *reinterpret_cast<uint4 *>(mout + (long long)r * C + qc) = *reinterpret_cast<const uint4 *>(mb);
+    *reinterpret_cast<uint4 *>(mout + (long long)r * C + qc) = lp::round8(acc);
   }
 }
 
@@ -442,44 +429,32 @@ __global__ void __launch_bounds__(kTPB, 4)
                const __nv_bfloat16 *__restrict__ wl, const float *__restrict__ bl,
                const int *done) {
   if (stopped(done)) return;
-  constexpr int TS = lp::kTileStride;
-  __shared__ __align__(16) __nv_bfloat16 wsm[C * TS];
-  __shared__ float bsm[C];
-  __shared__ __align__(16) __nv_bfloat16 tile[kTPB / 32][16 * TS];
-  for (int t = threadIdx.x; t < C * 2 * C; t += blockDim.x)
-    wsm[(t / (2 * C)) * TS + t % (2 * C)] = wl[t];
-  if (threadIdx.x < C) bsm[threadIdx.x] = bl[threadIdx.x];
+  __shared__ uint4 wf[lp::kFragWords];
+  lp::load_frags(wf, wl);
   __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  __nv_bfloat16 *tw = tile[warp];
+  const int lane = threadIdx.x & 31, qc = 8 * (lane & 3);
+  float bias[8];
+  lp::load_bias(bias, bl, lane);
   const int ntiles = (n + 15) / 16;
   const int nwarps = (int)(((long long)gridDim.x * blockDim.x) >> 5);
   for (int tt = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5); tt < ntiles;
        tt += nwarps) {
-    // 16 rows x (4 uint4 of h + 4 uint4 of m): 128 copies, 4 per lane
+    uint4 own[2], m[2], o[2];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int idx = lane + 32 * k, rr = idx >> 3, part = idx & 7;
-      const int cell = tt * 16 + rr;
-      uint4 v = make_uint4(0, 0, 0, 0);
+    for (int rd = 0; rd < 2; ++rd) {
+      const int cell = tt * 16 + rd * 8 + (lane >> 2);
+      own[rd] = m[rd] = make_uint4(0, 0, 0, 0);
       if (cell < n) {
-        const __nv_bfloat16 *src = part < 4 ? hin + (long long)cell * C + 8 * part
-                                            : min_ + (long long)cell * C + 8 * (part - 4);
-        v = __ldg(reinterpret_cast<const uint4 *>(src));
+        own[rd] = __ldg(reinterpret_cast<const uint4 *>(hin + (long long)cell * C + qc));
+        m[rd] = __ldg(reinterpret_cast<const uint4 *>(min_ + (long long)cell * C + qc));
       }
-      *reinterpret_cast<uint4 *>(tw + rr * TS + 8 * part) = v;
     }
-    __syncwarp();
-    lp::tile_dense(tw, wsm, bsm, lane, lp::NoZ());
+    lp::dense(own, m, wf, bias, lane, o, lp::NoZ());
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const int idx = lane + 32 * k, rr = idx >> 2, part = idx & 3;
-      const int cell = tt * 16 + rr;
-      if (cell < n)
-        *reinterpret_cast<uint4 *>(hout + (long long)cell * C + 8 * part) =
-            *reinterpret_cast<const uint4 *>(tw + rr * TS + 8 * part);
+    for (int rd = 0; rd < 2; ++rd) {
+      const int cell = tt * 16 + rd * 8 + (lane >> 2);
+      if (cell < n) *reinterpret_cast<uint4 *>(hout + (long long)cell * C + qc) = o[rd];
     }
-    __syncwarp();
   }
 }
 
@@ -591,7 +566,7 @@ __global__ void __launch_bounds__(kTPB)
     for (int u = 0; u < 4; ++u) {
       const long long i = i0 + u * nw;
       dy[u] = i < n ? k2 * ad[i] : 0.f;
-      hv[u] = i < n ? bf(h[i * C + lane]) : 0.f;
+      hv[u] = i < n ? bf(h[i * C + lp::hpos(lane)]) : 0.f;
     }
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
@@ -658,12 +633,14 @@ __global__ void __launch_bounds__(kTPB, 3)
         mv = *reinterpret_cast<const float4 *>(m + o);
         const uint2 hq = *reinterpret_cast<const uint2 *>(hin + o);
         const __nv_bfloat16 *he = reinterpret_cast<const __nv_bfloat16 *>(&hq);
-        hv = make_float4(bf(he[0]), bf(he[1]), bf(he[2]), bf(he[3]));
+        hv = make_float4(bf(he[0]), bf(he[1]), bf(he[2]), bf(he[3]));  // see lp::hpos
         dz = make_float4(zv.x > 0.f ? dv.x : 0.f, zv.y > 0.f ? dv.y : 0.f,
                          zv.z > 0.f ? dv.z : 0.f, zv.w > 0.f ? dv.w : 0.f);
       }
       *reinterpret_cast<float4 *>(&dzs[cl][c4]) = dz;
-      *reinterpret_cast<float4 *>(&xs[cl][c4]) = hv;
+      const int ch = 8 * ((c4 & 7) >> 1) + 2 * (c4 >> 3);  // the first pair's channel
+      *reinterpret_cast<float2 *>(&xs[cl][ch]) = make_float2(hv.x, hv.y);
+      *reinterpret_cast<float2 *>(&xs[cl][ch + 8]) = make_float2(hv.z, hv.w);
       *reinterpret_cast<float4 *>(&xs[cl][C + c4]) = mv;
     }
     __syncthreads();

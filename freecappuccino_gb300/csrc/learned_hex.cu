@@ -10,18 +10,29 @@
 // neighbour), which keeps it latency bound.  Here a block owns a 16 x 16 tile of (i, j)
 // and marches along k over a chunk of planes:
 //
-//   - one producer warp streams the planes k-1 .. k_end of its tile, each with a
+//   - one thread streams the planes k-1 .. k_end of the tile, each with a
 //     one-cell halo in i and j (18 x 18 cells x 32 BF16 channels = 20.7 KB), plus the
 //     seven stencil value planes of the tile (7 x 16 x 16 FP32 = 7 KB), into a ring of
 //     five shared-memory stages with TMA tensor copies (cp.async.bulk.tensor, 4-D
 //     tensor maps over this GPU's memory, zero fill outside the block), each stage
 //     signalled by an mbarrier with a transaction count;
-//   - sixteen consumer warps compute plane k from stages k-1, k and k+1: per cell
-//     m = sum over the seven directions of val[d] * h[neighbour], summed in the CSR column
-//     order with the same fused multiply-adds as the gather form; then the per-warp
-//     16-cell tile [h; m] goes through the shared mma.sync product and epilogue
-//     (lp_tile.cuh) and h' leaves in 16-byte stores (16 consecutive cells = 1 KB);
-//   - after plane k the consumers release the stage of plane k-1 to the producer.
+//   - sixteen warps compute plane k: per cell m = sum over the seven directions of
+//     val[d] * h[neighbour], summed in the CSR column order with the same fused
+//     multiply-adds as the gather form; then the warp's 16 rows [h; m] go through the
+//     shared mma.sync product and epilogue (lp_tile.cuh), from and to registers, and h'
+//     leaves in 16-byte stores (8 consecutive cells = 512 B);
+//   - each warp releases plane k's stage, and the issuing thread refills what all have.
+//
+// What bounds it: the warps' instruction issue and shared-memory wavefronts (one block an
+// SM, 57% issue activity).  A lane therefore keeps its own column's planes k-1, k and k+1 in
+// FP32 registers (each converted once, not three times) and takes two cells that follow
+// one another in j, each the other's neighbour: four shared-memory loads and conversions a
+// cell instead of seven.  The rows' stored channel order is that of the product's
+// fragments, so no tile passes through shared memory.  The issuing thread is one of the
+// sixteen warps': a seventeenth held all to 96 registers.  One layer at 256^3, us: 896 with
+// seven loads a cell and the tile in shared memory; 786 with four loads; 724 with the
+// product in registers; 657 with sixteen warps (160^3: 261, 195, 182, 164; 64^3: 68, 22, 20,
+// 18, with the chunks below from the second on).
 //
 // So each activation row and each stencil value is read from HBM once per layer (the
 // halo rows of neighbouring tiles are L2 hits), and the loads are deep in flight without
@@ -45,13 +56,12 @@ namespace lphex {
 namespace {
 
 constexpr int C = lp::kTileC;
-constexpr int TS = lp::kTileStride;
+constexpr int OS = C + 8;                // padded row of the tile of a fused output
 constexpr int BX = 16, BY = 16;          // cells of a tile in i and j
 constexpr int HX = BX + 2, HY = BY + 2;  // with the one-cell halo
 constexpr int S = 5;                     // ring stages (planes)
-constexpr int KC = 32;                   // planes computed by one block
-constexpr int kCons = 16;                // consumer warps, one j row of the tile each
-constexpr int kThreads = (kCons + 1) * 32;
+constexpr int kCons = 16;                // consumer warps, 16 cells of every plane each
+constexpr int kThreads = (kCons + 1) * 32;  // of the tensor-memory form, with its producer
 constexpr unsigned kHBytes = HY * HX * C * 2;
 constexpr unsigned kVBytes = 7 * BY * BX * 4;
 constexpr unsigned long long kWaitNs = 1000000000ull;  // a wait gives up after 1 s
@@ -62,12 +72,11 @@ static_assert(kHBytes % 128 == 0 && kVBytes % 128 == 0, "TMA destinations stay 1
 struct __align__(128) Smem {
   __nv_bfloat16 h[S][HY][HX][C];
   float v[S][7][BY][BX];
-  __nv_bfloat16 w[C * TS];
-  float b[C];
+  uint4 w[lp::kFragWords];  // W_l as B fragments
   float wo[C + 4];  // w_out, b_out of a fused output (padded to 16 bytes)
-  __nv_bfloat16 tile[kCons][16 * TS];
+  __nv_bfloat16 tile[kCons][16 * OS];  // rows of a fused output
   unsigned long long full[S], empty[S];
-  int abort, issued;
+  int abort;
 };
 constexpr size_t kSmemBytes = sizeof(Smem) + 128;  // + alignment of the dynamic base
 static_assert(offsetof(Smem, tile) % 16 == 0, "the tile rows take 16-byte accesses");
@@ -127,9 +136,10 @@ __device__ __forceinline__ void tma_load_4d(void *dst, const CUtensorMap *map, i
       : "memory");
 }
 
-__global__ void __launch_bounds__(kThreads, 1)
+template <bool OUT>
+__global__ void __launch_bounds__(kCons * 32, 1)
     k_lp_layer_hex(const __grid_constant__ CUtensorMap tm_h, const __grid_constant__ CUtensorMap tm_v,
-                   int nx, int ny, int nz, __nv_bfloat16 *__restrict__ hout,
+                   int nx, int ny, int nz, int kc, __nv_bfloat16 *__restrict__ hout,
                    const __nv_bfloat16 *__restrict__ wl, const float *__restrict__ bl,
                    const int *done, int *status, OutFuse of) {
   if (done && __ldcg(done) != 0) return;
@@ -138,126 +148,152 @@ __global__ void __launch_bounds__(kThreads, 1)
                                        ~static_cast<uintptr_t>(127));
   const int ntx = (nx + BX - 1) / BX;
   const int i0 = (int)(blockIdx.x % ntx) * BX, j0 = (int)(blockIdx.x / ntx) * BY;
-  const int k0 = (int)blockIdx.y * KC;
-  const int k1 = min(k0 + KC, nz);
+  const int k0 = (int)blockIdx.y * kc;
+  const int k1 = min(k0 + kc, nz);
   const int np = k1 - k0 + 2;  // planes k0-1 .. k1
-  for (int t = threadIdx.x; t < C * 2 * C; t += blockDim.x)
-    sm.w[(t / (2 * C)) * TS + t % (2 * C)] = wl[t];
-  if (threadIdx.x < C) sm.b[threadIdx.x] = bl[threadIdx.x];
-  if (of.z && threadIdx.x <= C) sm.wo[threadIdx.x] = of.wout[threadIdx.x];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int s = 0; s < S; ++s) {
       mbar_init(&sm.full[s], 1);
       mbar_init(&sm.empty[s], kCons);
     }
     sm.abort = 0;
-    sm.issued = 0;
     fence_mbar_init();
   }
+  // The copies of ring index idx (plane k0 - 1 + idx), issued by one thread.
+  int issued = 0;
+  auto issue = [&]() {
+    const int s = issued % S, p = k0 - 1 + issued;
+    const bool want_v = p >= k0 && p < k1;
+    mbar_expect_tx(&sm.full[s], kHBytes + (want_v ? kVBytes : 0u));
+    tma_load_4d(&sm.h[s][0][0][0], &tm_h, 0, i0 - 1, j0 - 1, p, &sm.full[s]);
+    if (want_v) tma_load_4d(&sm.v[s][0][0][0], &tm_v, i0, j0, p, 0, &sm.full[s]);
+    ++issued;
+  };
+  if (threadIdx.x == 0)
+    while (issued < S && issued < np) issue();
+  lp::load_frags(sm.w, wl);
+  if (OUT && threadIdx.x <= C) sm.wo[threadIdx.x] = of.wout[threadIdx.x];
   __syncthreads();
   volatile int *abort = &sm.abort;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (warp == kCons) {
-    // producer: one thread issues every copy of the block
-    if (lane == 0) {
-      for (int idx = 0; idx < np; ++idx) {
-        const int s = idx % S;
-        if (idx >= S && !mbar_wait(&sm.empty[s], ((idx / S) - 1) & 1, abort)) break;
-        if (*abort) break;
-        const int p = k0 - 1 + idx;
-        const bool want_v = p >= k0 && p < k1;
-        mbar_expect_tx(&sm.full[s], kHBytes + (want_v ? kVBytes : 0u));
-        tma_load_4d(&sm.h[s][0][0][0], &tm_h, 0, i0 - 1, j0 - 1, p, &sm.full[s]);
-        if (want_v) tma_load_4d(&sm.v[s][0][0][0], &tm_v, i0, j0, p, 0, &sm.full[s]);
-        *(volatile int *)&sm.issued = idx + 1;
-      }
+  // A warp owns eight i by two j of the tile: the lane quad g takes cells (il, jr) and
+  // (il, jr + 1), eight channels a lane.
+  const int g = lane >> 2, qc = 8 * (lane & 3);
+  const int jr = 2 * (warp >> 1), il = 8 * (warp & 1) + g;
+  float bias[8];
+  lp::load_bias(bias, bl, lane);
+  // this lane's corner of stage 0: rows (jr - 1 .., il - 1 ..) of the halo plane, (jr, il)
+  // of the values
+  const __nv_bfloat16 *hs0 = &sm.h[0][jr][il][qc];
+  const float *vs0 = &sm.v[0][0][jr][il];
+  constexpr int kRow = HX * C, kHStage = HY * HX * C, kVStage = 7 * BY * BX;
+  auto quad = [](const __nv_bfloat16 *q) { return *reinterpret_cast<const uint4 *>(q); };
+  const long long row = (long long)nx * C, plane_len = row * ny;
+  __nv_bfloat16 *op = hout + plane_len * k0 + row * (j0 + jr) + (long long)(i0 + il) * C + qc;
+  const bool in0 = i0 + il < nx && j0 + jr < ny, in1 = i0 + il < nx && j0 + jr + 1 < ny;
+  // the lane's own channels of planes k-1, k and k+1, in FP32, turn by turn
+  float h0[2][8], h1[2][8], h2[2][8];
+  // every decision to stop is taken by the whole warp (__all_sync / __any_sync), so
+  // the warp never splits around its __syncwarp calls
+  bool ok = __all_sync(0xffffffffu, mbar_wait(&sm.full[0], 0, abort) &&
+                                        mbar_wait(&sm.full[1], 0, abort));
+  if (ok) {
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      lp::widen8(h0[r], quad(hs0 + (1 + r) * kRow + C));
+      lp::widen8(h1[r], quad(hs0 + kHStage + (1 + r) * kRow + C));
     }
     __syncwarp();
-  } else {
-    const int g = lane >> 2, qc = 8 * (lane & 3);
-    __nv_bfloat16 *tw = sm.tile[warp];
-    const float osc = of.z ? *of.rms : 0.f;
-    // every decision to stop is taken by the whole warp (__all_sync / __any_sync), so
-    // the warp never splits around its __syncwarp calls
-    bool ok = __all_sync(0xffffffffu, mbar_wait(&sm.full[0], 0, abort) &&
-                                          mbar_wait(&sm.full[1], 0, abort));
-    for (int k = k0; ok && k < k1; ++k) {
-      const int idx = k - k0 + 1;  // ring index of plane k
-      if (!__all_sync(0xffffffffu, mbar_wait(&sm.full[(idx + 1) % S], ((idx + 1) / S) & 1, abort))) {
-        ok = false;
-        break;
-      }
-      const int sP = (idx - 1) % S, sC = idx % S, sN = (idx + 1) % S;
-#pragma unroll 1
-      for (int rr = 0; rr < BY / kCons; ++rr) {
-        const int jr = warp + kCons * rr;
-#pragma unroll 1
-        for (int rd = 0; rd < 2; ++rd) {
-          const int il = rd * 8 + g;
-          const float *vv = &sm.v[sC][0][jr][il];
-          float acc[8];
-#pragma unroll
-          for (int c = 0; c < 8; ++c) acc[c] = 0.f;
-          // the seven terms in CSR column order: -nx ny, -nx, -1, 0, +1, +nx, +nx ny
-          const uint4 hm2 = *reinterpret_cast<const uint4 *>(&sm.h[sP][jr + 1][il + 1][qc]);
-          const uint4 hm1 = *reinterpret_cast<const uint4 *>(&sm.h[sC][jr][il + 1][qc]);
-          const uint4 hm0 = *reinterpret_cast<const uint4 *>(&sm.h[sC][jr + 1][il][qc]);
-          const uint4 own = *reinterpret_cast<const uint4 *>(&sm.h[sC][jr + 1][il + 1][qc]);
-          const uint4 hp0 = *reinterpret_cast<const uint4 *>(&sm.h[sC][jr + 1][il + 2][qc]);
-          const uint4 hp1 = *reinterpret_cast<const uint4 *>(&sm.h[sC][jr + 2][il + 1][qc]);
-          const uint4 hp2 = *reinterpret_cast<const uint4 *>(&sm.h[sN][jr + 1][il + 1][qc]);
-          lp::fma8(acc, vv[0 * BY * BX], hm2);
-          lp::fma8(acc, vv[1 * BY * BX], hm1);
-          lp::fma8(acc, vv[2 * BY * BX], hm0);
-          lp::fma8(acc, vv[3 * BY * BX], own);
-          lp::fma8(acc, vv[4 * BY * BX], hp0);
-          lp::fma8(acc, vv[5 * BY * BX], hp1);
-          lp::fma8(acc, vv[6 * BY * BX], hp2);
-          __align__(16) __nv_bfloat16 mb[8];
-          lp::tile_put_row(tw, il, qc, own, acc, mb);
-        }
-        __syncwarp();
-        lp::tile_dense(tw, sm.w, sm.b, lane, lp::NoZ());
-        const int jg = j0 + jr;
-        if (of.z) {
-          // the output instead of h': lane ri < 16 takes cell ri of the row, with the
-          // operations of the output kernel on the stored h'
-          const int ig = i0 + lane;
-          if (lane < 16 && ig < nx && jg < ny) {
-            const long long cell = ((long long)k * ny + jg) * nx + ig;
-            const float acc = lp::out_dot_row(tw + lane * TS, sm.wo);
-            of.z[cell] = of.r[cell] + osc * acc;
-          }
-        } else {
-#pragma unroll
-          for (int q = 0; q < 2; ++q) {
-            const int e = lane + 32 * q, ri = e >> 2, part = e & 3;
-            const int ig = i0 + ri;
-            if (ig < nx && jg < ny)
-              *reinterpret_cast<uint4 *>(
-                  hout + (((long long)k * ny + jg) * nx + ig) * C + 8 * part) =
-                  *reinterpret_cast<const uint4 *>(tw + ri * TS + 8 * part);
-          }
-        }
-        __syncwarp();
+    if (lane == 0) mbar_arrive(&sm.empty[0]);  // plane k0-1 is no longer read
+  }
+  int sC = 1, next_full = 2, phase = 0;  // stage of plane k; ring index and phase of plane k+1
+  // Plane k from its own stage (the in-plane neighbours) and the registers (own column):
+  // pv, ow, nx_ are the column's planes k-1, k and k+1, the last read here.
+  auto plane = [&](int k, const float(&pv)[2][8], const float(&ow)[2][8],
+                   float(&nx_)[2][8]) -> bool {
+    const int sN = sC + 1 == S ? 0 : sC + 1;
+    if (warp == 0) {
+      if (lane == 0 && issued <= next_full) {  // the plane this step needs, at the latest
+        if (mbar_wait(&sm.empty[sN], ((issued / S) - 1) & 1, abort)) issue();
       }
       __syncwarp();
-      if (lane == 0) mbar_arrive(&sm.empty[sP]);  // plane k-1 is no longer read
-      if (__any_sync(0xffffffffu, *abort != 0)) break;
     }
-    if (!ok && lane == 0) {
-      *abort = 1;
-      if (status) atomicExch(status, FCG_ERR_TIMEOUT);
+    if (!__all_sync(0xffffffffu, mbar_wait(&sm.full[sN], phase, abort))) {
+      ok = false;
+      return false;
     }
+    const __nv_bfloat16 *hc = hs0 + sC * kHStage, *hn = hs0 + sN * kHStage;
+    const float *vc = vs0 + sC * kVStage;
+    uint4 own[2], mq[2], o[2];
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      lp::widen8(nx_[r], quad(hn + (1 + r) * kRow + C));
+      const float *vv = vc + r * BX;
+      float acc[8];
+#pragma unroll
+      for (int c = 0; c < 8; ++c) acc[c] = 0.f;
+      // the seven terms in CSR column order: -nx ny, -nx, -1, 0, +1, +nx, +nx ny
+      lp::fma8(acc, vv[0 * BY * BX], pv[r]);
+      if (r == 0)
+        lp::fma8(acc, vv[1 * BY * BX], quad(hc + C));
+      else
+        lp::fma8(acc, vv[1 * BY * BX], ow[0]);
+      lp::fma8(acc, vv[2 * BY * BX], quad(hc + (1 + r) * kRow));
+      lp::fma8(acc, vv[3 * BY * BX], ow[r]);
+      lp::fma8(acc, vv[4 * BY * BX], quad(hc + (1 + r) * kRow + 2 * C));
+      if (r == 1)
+        lp::fma8(acc, vv[5 * BY * BX], quad(hc + 3 * kRow + C));
+      else
+        lp::fma8(acc, vv[5 * BY * BX], ow[1]);
+      lp::fma8(acc, vv[6 * BY * BX], nx_[r]);
+      mq[r] = lp::round8(acc);
+    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&sm.empty[sC]);  // plane k is no longer read
+#pragma unroll
+    for (int r = 0; r < 2; ++r) own[r] = lp::narrow8(ow[r]);
+    lp::dense(own, mq, sm.w, bias, lane, o, lp::NoZ());
+    if (OUT) {
+      // the output instead of h': lane ri < 16 takes cell ri of the warp's, with the
+      // operations of the output kernel on the stored h'
+      __nv_bfloat16 *tw = sm.tile[warp];
+#pragma unroll
+      for (int r = 0; r < 2; ++r) *reinterpret_cast<uint4 *>(tw + (8 * r + g) * OS + qc) = o[r];
+      __syncwarp();
+      const int i = i0 + 8 * (warp & 1) + (lane & 7), j = j0 + jr + (lane >> 3);
+      if (lane < 16 && i < nx && j < ny) {
+        const long long cell = ((long long)k * ny + j) * nx + i;
+        const float acc = lp::out_dot_row(tw + lane * OS, sm.wo);
+        of.z[cell] = of.r[cell] + *of.rms * acc;
+      }
+      __syncwarp();
+    } else {
+      if (in0) *reinterpret_cast<uint4 *>(op) = o[0];
+      if (in1) *reinterpret_cast<uint4 *>(op + row) = o[1];
+      op += plane_len;
+    }
+    // refill what every warp has released meanwhile
+    if (threadIdx.x == 0)
+      while (issued < np && mbar_try_wait(&sm.empty[issued % S], ((issued / S) - 1) & 1)) issue();
+    sC = sN;
+    if (++next_full % S == 0) phase ^= 1;
+    return !__any_sync(0xffffffffu, *abort != 0);
+  };
+  for (int k = k0; ok && k < k1; k += 3) {
+    if (!plane(k, h0, h1, h2)) break;
+    if (k + 1 >= k1 || !plane(k + 1, h1, h2, h0)) break;
+    if (k + 2 >= k1 || !plane(k + 2, h2, h0, h1)) break;
+  }
+  if (!ok && lane == 0) {
+    *abort = 1;
+    if (status) atomicExch(status, FCG_ERR_TIMEOUT);
   }
   __syncthreads();
   // After a wait that gave up, the copies still in flight must land before the block
   // leaves (their destination is this block's shared memory).
-  if (threadIdx.x == 0 && *abort) {
-    const int issued = *(volatile int *)&sm.issued;
+  if (threadIdx.x == 0 && *abort)
     for (int idx = issued - S > 0 ? issued - S : 0; idx < issued; ++idx)
       mbar_wait(&sm.full[idx % S], (idx / S) & 1, nullptr);
-  }
 }
 
 // ---------------------------------------------------------------------------
@@ -320,7 +356,7 @@ __device__ __forceinline__ bool cons_sync_or(bool v, int nthreads) {
 
 __global__ void __launch_bounds__(kThreads, 1)
     k_lp_layer_hex_tc(const __grid_constant__ CUtensorMap tm_h,
-                      const __grid_constant__ CUtensorMap tm_v, int nx, int ny, int nz,
+                      const __grid_constant__ CUtensorMap tm_v, int nx, int ny, int nz, int kc,
                       __nv_bfloat16 *__restrict__ hout, const __nv_bfloat16 *__restrict__ wl,
                       const float *__restrict__ bl, const int *done, int *status) {
   static_assert(kCons == 16 && BY == kCons, "one j row of the tile per consumer warp");
@@ -330,8 +366,8 @@ __global__ void __launch_bounds__(kThreads, 1)
                                            ~static_cast<uintptr_t>(1023));
   const int ntx = (nx + BX - 1) / BX;
   const int i0 = (int)(blockIdx.x % ntx) * BX, j0 = (int)(blockIdx.x / ntx) * BY;
-  const int k0 = (int)blockIdx.y * KC;
-  const int k1 = min(k0 + KC, nz);
+  const int k0 = (int)blockIdx.y * kc;
+  const int k1 = min(k0 + kc, nz);
   const int np = k1 - k0 + 2;  // planes k0-1 .. k1
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // W_l [out n][in k] is already K-major: chunk (n, kc) -> canonical position
@@ -406,25 +442,19 @@ __global__ void __launch_bounds__(kThreads, 1)
           : "memory");
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
       const int il = erow & 15, jrow = erow >> 4;
-      __align__(16) __nv_bfloat16 o[16];
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const uint4 hq =
-            *reinterpret_cast<const uint4 *>(&sm.h[st][jrow + 1][il + 1][16 * ech + 8 * u]);
-        const __nv_bfloat16 *hold = reinterpret_cast<const __nv_bfloat16 *>(&hq);
-#pragma unroll
-        for (int c = 0; c < 8; ++c) {
-          const int col = 16 * ech + 8 * u + c;
-          const float z = __uint_as_float(v[8 * u + c]) + sm.b[col];
-          o[8 * u + c] = __float2bfloat16(lp::bf(hold[c]) + fmaxf(z, 0.f));
-        }
-      }
       const int ig = i0 + il, jg = j0 + jrow;
-      if (ok && ig < nx && jg < ny) {
-        uint4 *dst = reinterpret_cast<uint4 *>(
-            hout + (((long long)k * ny + jg) * nx + ig) * C + 16 * ech);
-        dst[0] = *reinterpret_cast<const uint4 *>(&o[0]);
-        dst[1] = *reinterpret_cast<const uint4 *>(&o[8]);
+#pragma unroll
+      for (int c = 0; c < 16; c += 2) {
+        const int col = 16 * ech + c, at = lp::hpos(col);
+        const __nv_bfloat162 hold =
+            *reinterpret_cast<const __nv_bfloat162 *>(&sm.h[st][jrow + 1][il + 1][at]);
+        const float z0 = __uint_as_float(v[c]) + sm.b[col];
+        const float z1 = __uint_as_float(v[c + 1]) + sm.b[col + 1];
+        const __nv_bfloat162 o = __floats2bfloat162_rn(lp::bf(hold.x) + fmaxf(z0, 0.f),
+                                                       lp::bf(hold.y) + fmaxf(z1, 0.f));
+        if (ok && ig < nx && jg < ny)
+          *reinterpret_cast<__nv_bfloat162 *>(
+              hout + (((long long)k * ny + jg) * nx + ig) * C + at) = o;
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       return ok;
@@ -459,13 +489,15 @@ __global__ void __launch_bounds__(kThreads, 1)
           lp::fma8(acc, vv[4 * BY * BX], hp0);
           lp::fma8(acc, vv[5 * BY * BX], hp1);
           lp::fma8(acc, vv[6 * BY * BX], hp2);
-          __align__(16) __nv_bfloat16 mb[8];
-#pragma unroll
-          for (int c = 0; c < 8; ++c) mb[c] = __float2bfloat16(acc[c]);
+          const uint4 mq = lp::round8(acc);
           const int row = jr * 16 + il;
-          *reinterpret_cast<uint4 *>(ab + tc_off(row, qc >> 3)) = own;
-          *reinterpret_cast<uint4 *>(ab + tc_off(row, 4 + (qc >> 3))) =
-              *reinterpret_cast<const uint4 *>(mb);
+          // the operand is in channel order: pair i of quarter tg is channels 8 i + 2 tg, + 1
+          const unsigned hw[4] = {own.x, own.y, own.z, own.w}, mw[4] = {mq.x, mq.y, mq.z, mq.w};
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            *reinterpret_cast<unsigned *>(ab + tc_off(row, i) + qc / 2) = hw[i];
+            *reinterpret_cast<unsigned *>(ab + tc_off(row, 4 + i) + qc / 2) = mw[i];
+          }
         }
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -609,13 +641,36 @@ cudaError_t set_attributes(int dev) {
   if (dev < 0 || dev >= kMaxDevices) return cudaErrorInvalidDevice;
   std::lock_guard<std::mutex> lock(g_attr_mutex);
   if (g_attr_set[dev]) return cudaSuccess;
-  cudaError_t e = cudaFuncSetAttribute(k_lp_layer_hex, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)kSmemBytes);
+  cudaError_t e = cudaFuncSetAttribute(k_lp_layer_hex<false>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_lp_layer_hex<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)kSmemBytes);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_lp_layer_hex_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)kSmemTcBytes);
   if (e == cudaSuccess) g_attr_set[dev] = true;
   return e;
+}
+
+// Planes of a block's chunk: one block is resident an SM, and a chunk costs its planes and
+// about five more (the ring's start, two halo planes).  The number of chunks that makes
+// (waves of blocks) x (planes + 5) least.  With 32 planes whatever the mesh, 160^3 ran 500
+// blocks on 152 SMs, four waves for 3.3, and 64^3 ran 32.
+int chunk_planes(int tiles, int nz, int num_sms) {
+  int best = nz;
+  long long cost = -1;
+  for (int c = 1; c <= nz; ++c) {
+    const int kc = (nz + c - 1) / c;
+    const long long blocks = (long long)tiles * ((nz + kc - 1) / kc);
+    const long long t = (blocks + num_sms - 1) / num_sms * (kc + 5);
+    if (cost < 0 || t < cost) {
+      cost = t;
+      best = kc;
+    }
+    if (kc <= 4) break;
+  }
+  return best;
 }
 
 }  // namespace
@@ -647,22 +702,25 @@ cudaError_t values(const fcg_context *c, const HexGrid &g, const float *aval, fl
 cudaError_t layer(const HexGrid &g, int num_sms, const __nv_bfloat16 *hin, __nv_bfloat16 *hout,
                   const float *val, const __nv_bfloat16 *wl, const float *bl, const int *done,
                   int *status, cudaStream_t st, const OutFuse *out, bool *fused) {
-  (void)num_sms;
   if (fused) *fused = false;
   CUtensorMap th, tv;
   if (!encode_maps(g, hin, val, &th, &tv)) return cudaErrorInvalidValue;
   const int ntx = (g.nx + BX - 1) / BX, nty = (g.ny + BY - 1) / BY;
-  const dim3 grid((unsigned)(ntx * nty), (unsigned)((g.nz + KC - 1) / KC));
+  const int kc = chunk_planes(ntx * nty, g.nz, num_sms);
+  const dim3 grid((unsigned)(ntx * nty), (unsigned)((g.nz + kc - 1) / kc));
   // the tile product on mma.sync (default) or on tcgen05 (FCG_LP_HEX_MMA=tc: the same bits,
   // measured 1.17 against 0.94 ms per layer at 256^3)
   const char *mm = std::getenv("FCG_LP_HEX_MMA");
   if (mm && std::strcmp(mm, "tc") == 0)
-    k_lp_layer_hex_tc<<<grid, kThreads, kSmemTcBytes, st>>>(th, tv, g.nx, g.ny, g.nz, hout, wl,
+    k_lp_layer_hex_tc<<<grid, kThreads, kSmemTcBytes, st>>>(th, tv, g.nx, g.ny, g.nz, kc, hout, wl,
                                                             bl, done, status);
-  else {
-    k_lp_layer_hex<<<grid, kThreads, kSmemBytes, st>>>(th, tv, g.nx, g.ny, g.nz, hout, wl, bl,
-                                                       done, status, out ? *out : OutFuse{});
-    if (out && fused) *fused = true;
+  else if (out) {
+    k_lp_layer_hex<true><<<grid, kCons * 32, kSmemBytes, st>>>(th, tv, g.nx, g.ny, g.nz, kc, hout,
+                                                               wl, bl, done, status, *out);
+    if (fused) *fused = true;
+  } else {
+    k_lp_layer_hex<false><<<grid, kCons * 32, kSmemBytes, st>>>(th, tv, g.nx, g.ny, g.nz, kc, hout,
+                                                                wl, bl, done, status, OutFuse{});
   }
   return cudaPeekAtLastError();  // left set for the caller's launch check
 }
