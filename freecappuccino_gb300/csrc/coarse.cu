@@ -239,7 +239,7 @@ __device__ __forceinline__ float row_lanes(const int *ptr, const int *col, const
   return acc;
 }
 
-// y = x + omega dinv (b - A x); x == NULL stands for x = 0
+// y = x + omega dinv (b - A x)
 template <int LPR>
 __global__ void __launch_bounds__(kTPB)
     k_ml_jacobi(int n, const int *__restrict__ ptr, const int *__restrict__ col,
@@ -253,10 +253,6 @@ __global__ void __launch_bounds__(kTPB)
   const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
   for (long long base = w0 * RPW; base < n; base += nw * RPW) {
     const int row = (int)base + lane / LPR;
-    if (!x) {
-      if (q == 0 && row < n) y[row] = omega * dinv[row] * b[row];
-      continue;
-    }
     const float ax = row_lanes<LPR>(ptr, col, a, x, row, n, q);
     if (q == 0 && row < n) y[row] = x[row] + omega * dinv[row] * (b[row] - ax);
   }
@@ -280,15 +276,28 @@ __global__ void __launch_bounds__(kTPB)
   }
 }
 
+// The first damped Jacobi sweep of a level, from x = 0: omega dinv b.  The kernel that
+// forms b writes it too (x1 null: a level without sweeps), so it is no launch of its own.
+struct FirstSweep {
+  const float *dinv;
+  float *x1;
+  float omega;
+  __device__ __forceinline__ void operator()(long long I, float b) const {
+    if (x1) x1[I] = omega * dinv[I] * b;
+  }
+};
+
 // bc[I] = sum over the member rows i of I of t_i
 __global__ void __launch_bounds__(kTPB)
     k_ml_restrict(int nc, const int *__restrict__ mptr, const int *__restrict__ mem,
-                  const float *__restrict__ t, float *__restrict__ bc, const int *done) {
+                  const float *__restrict__ t, float *__restrict__ bc, FirstSweep first,
+                  const int *done) {
   if (stopped(done)) return;
   FCG_GRID_STRIDE(I, nc) {
     float acc = 0.f;
     for (int m = mptr[I]; m < mptr[I + 1]; ++m) acc += t[mem[m]];
     bc[I] = acc;
+    first(I, acc);
   }
 }
 
@@ -312,27 +321,23 @@ __global__ void __launch_bounds__(kTPB, 6)
   }
 }
 
-// fine level Jacobi sweep: zout = zin + omega (r - Ahat zin); zin == NULL: zout = omega r
+// fine level Jacobi sweep: zout = zin + omega (r - Ahat zin); zin == NULL: zout = omega r;
+// zin == r: the sweep after that one, omega (A r) for A (omega r)
 __global__ void __launch_bounds__(kTPB, 6)
     k_ml_jac0(SellView s, int n, const float *__restrict__ val, const float *__restrict__ r,
               const float *__restrict__ zin, float *__restrict__ zout, float omega,
               const int *done) {
   if (stopped(done)) return;
+  if (!zin) {
+    FCG_GRID_STRIDE(row, n) zout[row] = omega * r[row];
+    return;
+  }
+  const float f = zin == r ? omega : 1.f;
   FCG_SLICE_LOOP(slice, lane, s) {
     const int row = slice * 32 + lane;
-    if (!zin) {
-      if (row < n) zout[row] = omega * r[row];
-      continue;
-    }
-    const float az = sell_row(s, n, val, zin, slice, lane);
-    if (row < n) zout[row] = zin[row] + omega * (r[row] - az);
+    const float az = f * sell_row(s, n, val, zin, slice, lane);
+    if (row < n) zout[row] = f * zin[row] + omega * (r[row] - az);
   }
-}
-
-__global__ void __launch_bounds__(kTPB)
-    k_ml_copy(int n, const float *__restrict__ a, float *__restrict__ b, const int *done) {
-  if (stopped(done)) return;
-  FCG_GRID_STRIDE(i, n) b[i] = a[i];
 }
 
 // ---- smoothed first level: P = (I - omega D^-1 Ahat) P_tent, A P, P^T A P -----------
@@ -530,16 +535,24 @@ __global__ void __launch_bounds__(kTPB)
   FCG_GRID_STRIDE(m, nnz) pt_val[m] = p_val[t_pos[m]];
 }
 
-// b1 = P^T t
+// b1 = P^T t, eight lanes a row (about 36 entries a row, read in whole sectors; a thread a
+// row took 67 us at 511 k rows, this 39)
 __global__ void __launch_bounds__(kTPB)
     k_sa_restrict(int nc, const int *__restrict__ t_ptr, const int *__restrict__ t_row,
                   const float *__restrict__ pt_val, const float *__restrict__ t,
-                  float *__restrict__ bc, const int *done) {
+                  float *__restrict__ bc, FirstSweep first, const int *done) {
   if (stopped(done)) return;
-  FCG_GRID_STRIDE(I, nc) {
-    float acc = 0.f;
-    for (int m = t_ptr[I]; m < t_ptr[I + 1]; ++m) acc += pt_val[m] * t[t_row[m]];
-    bc[I] = acc;
+  constexpr int LPR = 8, RPW = 32 / LPR;
+  const int lane = threadIdx.x & 31, q = lane & (LPR - 1);
+  const long long w0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
+  for (long long base = w0 * RPW; base < nc; base += nw * RPW) {
+    const int row = (int)base + lane / LPR;
+    const float acc = row_lanes<LPR>(t_ptr, t_row, pt_val, t, row, nc, q);
+    if (q == 0 && row < nc) {
+      bc[row] = acc;
+      first(row, acc);
+    }
   }
 }
 
@@ -556,8 +569,16 @@ __global__ void __launch_bounds__(kTPB)
   }
 }
 
-// One V-cycle on level k of H.lv for right-hand side lv[k].b; returns the vector holding
-// the result (lv[k].x or lv[k].y).
+bool dense_level(const Hierarchy &H, int k) { return k + 1 == (int)H.lv.size() && H.has_dense; }
+
+// What the restriction to level k writes besides lv[k].b: the level's first sweep.
+FirstSweep first_sweep(const Hierarchy &H, const Options &o, int k) {
+  const DevLevel &L = H.lv[k];
+  return FirstSweep{L.dinv, dense_level(H, k) ? nullptr : L.x, (float)o.omega};
+}
+
+// One V-cycle on level k of H.lv for right-hand side lv[k].b, with the first sweep's result
+// in lv[k].x; returns the vector holding the result (lv[k].x or lv[k].y).
 float *enqueue_vcycle(Hierarchy &H, int num_sms, const Options &o, cudaStream_t st, int k,
                       const int *done) {
   DevLevel &L = H.lv[k];
@@ -569,13 +590,12 @@ float *enqueue_vcycle(Hierarchy &H, int num_sms, const Options &o, cudaStream_t 
   auto jacobi = wide ? k_ml_jacobi<8> : k_ml_jacobi<4>;
   auto resid = wide ? k_ml_resid<8> : k_ml_resid<4>;
   const bool last = k + 1 == (int)H.lv.size();
-  if (last && H.has_dense) {
+  if (dense_level(H, k)) {
     const int blocks = (L.n * 32 + kTPB - 1) / kTPB;
     k_ml_dense_apply<<<blocks, kTPB, 0, st>>>(L.n, H.dense.as<float>(), L.b, L.x, done);
     return L.x;
   }
   float *cur = L.x, *oth = L.y;
-  jacobi<<<g4, kTPB, 0, st>>>(L.n, L.ptr, L.col, L.a32, L.dinv, L.b, nullptr, cur, om, done);
   const int pre = last ? 2 * o.sweeps + 2 : o.sweeps;  // coarsest without a dense inverse
   for (int s = 1; s < pre; ++s) {
     jacobi<<<g4, kTPB, 0, st>>>(L.n, L.ptr, L.col, L.a32, L.dinv, L.b, cur, oth, om, done);
@@ -585,7 +605,7 @@ float *enqueue_vcycle(Hierarchy &H, int num_sms, const Options &o, cudaStream_t 
   DevLevel &Lc = H.lv[k + 1];
   resid<<<g4, kTPB, 0, st>>>(L.n, L.ptr, L.col, L.a32, L.b, cur, oth, done);
   k_ml_restrict<<<grid_for(Lc.n, num_sms, 8), kTPB, 0, st>>>(Lc.n, Lc.mptr, Lc.mem, oth, Lc.b,
-                                                            done);
+                                                            first_sweep(H, o, k + 1), done);
   const float *e = enqueue_vcycle(H, num_sms, o, st, k + 1, done);
   k_ml_prolong<<<g, kTPB, 0, st>>>(L.n, Lc.agg, e, cur, al, done);
   for (int s = 0; s < o.sweeps; ++s) {
@@ -597,14 +617,15 @@ float *enqueue_vcycle(Hierarchy &H, int num_sms, const Options &o, cudaStream_t 
 
 // Restriction of the fine residual t to level 1 and prolongation of its correction e:
 // the smoothed P (correction not scaled) or the aggregation (scaled by alpha).
-void fine_restrict(Hierarchy &H, int num_sms, cudaStream_t st, const float *t, const int *done) {
+void fine_restrict(Hierarchy &H, int num_sms, const Options &o, cudaStream_t st, const float *t,
+                   const int *done) {
   DevLevel &L1 = H.lv[0];
   if (H.smoothed)
-    k_sa_restrict<<<grid_for(L1.n, num_sms, 8), kTPB, 0, st>>>(L1.n, H.t_ptr, H.t_row,
-                                                              H.pt_val, t, L1.b, done);
+    k_sa_restrict<<<grid_for(8LL * L1.n, num_sms, 8), kTPB, 0, st>>>(
+        L1.n, H.t_ptr, H.t_row, H.pt_val, t, L1.b, first_sweep(H, o, 0), done);
   else
     k_ml_restrict<<<grid_for(L1.n, num_sms, 8), kTPB, 0, st>>>(L1.n, L1.mptr, L1.mem, t, L1.b,
-                                                              done);
+                                                              first_sweep(H, o, 0), done);
 }
 
 void fine_prolong(Hierarchy &H, int n, int num_sms, const Options &o, cudaStream_t st,
@@ -939,7 +960,7 @@ void enqueue_correction(Hierarchy &H, fcg_context *c, const Options &o, cudaStre
   const int n = c->n, ns = c->num_sms;
   float *t = H.fine_tmp.as<float>();
   k_ml_resid0<<<grid_for(n, ns, 6), kTPB, 0, st>>>(c->sv, n, scaled32(c), r, z, t, done);
-  fine_restrict(H, ns, st, t, done);
+  fine_restrict(H, ns, o, st, t, done);
   const float *e = enqueue_vcycle(H, ns, o, st, 0, done);
   fine_prolong(H, n, ns, o, st, e, z, done);
 }
@@ -951,15 +972,16 @@ void enqueue_jacobi_cycle(Hierarchy &H, fcg_context *c, const Options &o, cudaSt
   float *t = H.fine_tmp.as<float>();
   float *u = t + pad256(sizeof(float) * n) / sizeof(float);
   const int gs = grid_for(n, ns, 6);
-  float *cur = z, *oth = u;
-  k_ml_jac0<<<gs, kTPB, 0, st>>>(c->sv, n, scaled32(c), r, nullptr, cur, om, done);
+  float *cur = u, *oth = z;  // 2 sweeps - 1 swaps: the result ends in z
+  if (o.sweeps == 1)
+    k_ml_jac0<<<gs, kTPB, 0, st>>>(c->sv, n, scaled32(c), r, nullptr, cur, om, done);
   for (int s = 1; s < o.sweeps; ++s) {
-    k_ml_jac0<<<gs, kTPB, 0, st>>>(c->sv, n, scaled32(c), r, cur, oth, om, done);
+    k_ml_jac0<<<gs, kTPB, 0, st>>>(c->sv, n, scaled32(c), r, s == 1 ? r : cur, oth, om, done);
     std::swap(cur, oth);
   }
   if (!H.lv.empty()) {
     k_ml_resid0<<<gs, kTPB, 0, st>>>(c->sv, n, scaled32(c), r, cur, t, done);
-    fine_restrict(H, ns, st, t, done);
+    fine_restrict(H, ns, o, st, t, done);
     const float *e = enqueue_vcycle(H, ns, o, st, 0, done);
     fine_prolong(H, n, ns, o, st, e, cur, done);
   }
@@ -967,7 +989,6 @@ void enqueue_jacobi_cycle(Hierarchy &H, fcg_context *c, const Options &o, cudaSt
     k_ml_jac0<<<gs, kTPB, 0, st>>>(c->sv, n, scaled32(c), r, cur, oth, om, done);
     std::swap(cur, oth);
   }
-  if (cur != z) k_ml_copy<<<grid_for(n, ns, 8), kTPB, 0, st>>>(n, cur, z, done);
 }
 
 }  // namespace ml
