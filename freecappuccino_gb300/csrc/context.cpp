@@ -11,6 +11,7 @@ fcg_context::~fcg_context() {
   for (auto &b : bound_allocs) b.release();
   for (auto &b : stage) b.release();
   dmat.release();
+  gconst.release();
   fgeo.release();
   bgeo.release();
   scratch.release();
@@ -273,6 +274,7 @@ extern "C" int fcg_bind_mesh(fcg_context *c, const fcg_mesh_desc *m) {
   c->bound_allocs.clear();
   c->bound = false;
   c->dmat_ready = false;
+  c->gconst_ready = false;
   c->order = LevelOrder{};
   c->fgeo_ready = false;
   c->bgeo_ready = false;

@@ -164,6 +164,9 @@ struct fcg_context {
   // lazily built lsq matrices dmat(9,n)
   fcg::DBuf dmat;
   bool dmat_ready = false;
+  // lazily built constants of the Gauss gradient (gradients.cu): 1/vol, then a flag
+  fcg::DBuf gconst;
+  bool gconst_ready = false;
   // lazily built mesh-constant factors of the inner faces (assembly.cu: laplacian,
   // facefluxmass, fluxmc), planar [FG_COUNT][nin]
   fcg::DBuf fgeo;

@@ -5,7 +5,8 @@
 // Gauss: one thread per inner face computes the interpolated face value times the
 // area vector (gradco :128-190) into a face array; one thread per cell then adds its
 // inner faces in face order (+ as owner, - as neighbour), its boundary faces in the
-// reference's boundary-loop order (gradbc :194-211) and scales by 1/vol.  LSQ: one
+// reference's boundary-loop order (gradbc :194-211) and scales by 1/vol, straight into the
+// caller's array.  LSQ: one
 // thread per cell gathers the same per-face terms the reference scatters.  Compiled
 // with --fmad=false, so results are bit-identical to the Fortran loops.
 #include "fcg_internal.h"
@@ -15,21 +16,70 @@ using namespace fcg;
 
 namespace {
 
-// gradco: face value with the old gradient interpolated to the point on PN.
-__global__ void k_gauss_faces(MeshView m, const double *__restrict__ fi,
-                              const double *__restrict__ gold, double *__restrict__ dfe) {
+// The bound mesh's constants of the Gauss gradient: 1/vol per cell, and `odd`, set where a
+// face's interpolation factors or offset are not finite.
+struct GaussConst {
+  const double *volr;
+  const int *odd;
+};
+
+struct FaceOffset {
+  double fxn, fxp, dx, dy, dz;
+};
+
+// Face f between cells p and q with factor fxn: the offset of the face centre from the
+// interpolation point on PN.
+__device__ __forceinline__ FaceOffset face_offset(const MeshView &m, long long f, int p, int q,
+                                                  double fxn) {
+  const double fxp = 1.0 - fxn;
+  const double xi = m.xc[p] * fxp + m.xc[q] * fxn;
+  const double yi = m.yc[p] * fxp + m.yc[q] * fxn;
+  const double zi = m.zc[p] * fxp + m.zc[q] * fxn;
+  return {fxn, fxp, m.xf[f] - xi, m.yf[f] - yi, m.zf[f] - zi};
+}
+
+__global__ void k_gauss_const(MeshView m, double *__restrict__ volr, int *__restrict__ odd) {
+  FCG_GRID_STRIDE(c, m.n) volr[c] = 1.0 / m.vol[c];
   FCG_GRID_STRIDE(f, m.nin) {
-    int p = m.owner[f], q = m.neighbour[f];
-    double fxn = m.facint[f];
-    double fxp = 1.0 - fxn;
-    double xi = m.xc[p] * fxp + m.xc[q] * fxn;
-    double yi = m.yc[p] * fxp + m.yc[q] * fxn;
-    double zi = m.zc[p] * fxp + m.zc[q] * fxn;
-    double dfxi = gold[3 * p] * fxp + gold[3 * q] * fxn;
-    double dfyi = gold[3 * p + 1] * fxp + gold[3 * q + 1] * fxn;
-    double dfzi = gold[3 * p + 2] * fxp + gold[3 * q + 2] * fxn;
-    double fie = fi[p] * fxp + fi[q] * fxn + dfxi * (m.xf[f] - xi) + dfyi * (m.yf[f] - yi) +
-                 dfzi * (m.zf[f] - zi);
+    const FaceOffset o = face_offset(m, f, m.owner[f], m.neighbour[f], m.facint[f]);
+    if (!(isfinite(o.fxn) && isfinite(o.fxp) && isfinite(o.dx) && isfinite(o.dy) &&
+          isfinite(o.dz)))
+      *odd = 1;
+  }
+}
+
+// gradco: face value with the old gradient (zero without gold) interpolated to the point
+// on PN.
+__device__ __forceinline__ double face_value(const FaceOffset &o, int p, int q,
+                                             const double *__restrict__ fi,
+                                             const double *__restrict__ gold) {
+  auto old = [&](int c, int k) { return gold ? gold[3LL * c + k] : 0.0; };
+  const double dfxi = old(p, 0) * o.fxp + old(q, 0) * o.fxn;
+  const double dfyi = old(p, 1) * o.fxp + old(q, 1) * o.fxn;
+  const double dfzi = old(p, 2) * o.fxp + old(q, 2) * o.fxn;
+  return fi[p] * o.fxp + fi[q] * o.fxn + dfxi * o.dx + dfyi * o.dy + dfzi * o.dz;
+}
+
+// Bound by the FP64 pipe (629 G instructions/s): 34 of them a face with an old gradient,
+// 7 without (FIRST, the first pass).  With a zero gradient and finite factors the
+// correction terms are products with zero: adding them changes no bit of the face's
+// contribution (a zero's sign is lost in the cell's sum, which starts from +0), so the
+// first pass leaves them out and reads neither the cell centres nor the face centres.
+// Factors that are not finite would make those products NaN; such a mesh (odd) takes
+// the whole expression.  6.2 M faces (128^3): 94 us, with the zero terms 432.
+template <bool FIRST>
+__global__ void __launch_bounds__(kTPB)
+    k_gauss_faces(MeshView m, GaussConst k, const double *__restrict__ fi,
+                  const double *__restrict__ gold, double *__restrict__ dfe) {
+  const bool plain = FIRST && __ldg(k.odd) == 0;
+  FCG_GRID_STRIDE(f, m.nin) {
+    const int p = m.owner[f], q = m.neighbour[f];
+    const double fxn = m.facint[f];
+    double fie;
+    if (plain)
+      fie = fi[p] * (1.0 - fxn) + fi[q] * fxn;
+    else
+      fie = face_value(face_offset(m, f, p, q, fxn), p, q, fi, FIRST ? nullptr : gold);
     dfe[f] = fie * m.arx[f];
     dfe[m.nin + f] = fie * m.ary[f];
     dfe[2LL * m.nin + f] = fie * m.arz[f];
@@ -41,39 +91,52 @@ __global__ void k_gauss_oc(MeshView m, const double *__restrict__ fi,
                            const double *__restrict__ gold, double *__restrict__ dfo) {
   FCG_GRID_STRIDE(i, m.noc) {
     const int p = m.oc_l[i], q = m.oc_r[i], f = m.oc_fl[i];
-    double fxn = m.oc_foc[i];
-    double fxp = 1.0 - fxn;
-    double xi = m.xc[p] * fxp + m.xc[q] * fxn;
-    double yi = m.yc[p] * fxp + m.yc[q] * fxn;
-    double zi = m.zc[p] * fxp + m.zc[q] * fxn;
-    double dfxi = gold[3 * p] * fxp + gold[3 * q] * fxn;
-    double dfyi = gold[3 * p + 1] * fxp + gold[3 * q + 1] * fxn;
-    double dfzi = gold[3 * p + 2] * fxp + gold[3 * q + 2] * fxn;
-    double fie = fi[p] * fxp + fi[q] * fxn + dfxi * (m.xf[f] - xi) + dfyi * (m.yf[f] - yi) +
-                 dfzi * (m.zf[f] - zi);
+    const double fie = face_value(face_offset(m, f, p, q, m.oc_foc[i]), p, q, fi, gold);
     dfo[i] = fie * m.arx[f];
     dfo[m.noc + i] = fie * m.ary[f];
     dfo[2LL * m.noc + i] = fie * m.arz[f];
   }
 }
 
-__global__ void k_gauss_cells(MeshView m, const double *__restrict__ fi,
-                              const double *__restrict__ dfe, const double *__restrict__ dfo,
-                              double *__restrict__ g) {
+constexpr int kBatch = 3;
+
+// own ? x : -x on the integer pipe: the compiler's own choice adds an FP64 instruction, of
+// which a cell kernel has none to spare.
+__device__ __forceinline__ double signed_term(bool own, double x) {
+  const unsigned long long flip = own ? 0ULL : 0x8000000000000000ULL;
+  return __longlong_as_double(__double_as_longlong(x) ^ flip);
+}
+
+// Bound by the FP64 pipe: 21 instructions a cell (1/vol is the mesh's, and the sign of a
+// neighbour's term an integer flip).  128^3: 106 us; with a quotient and two signed sums a
+// face 208, with negations in FP64 189.  Batches of 2, 3 and 6 faces differ by 2 %.
+__global__ void __launch_bounds__(kTPB)
+    k_gauss_cells(MeshView m, GaussConst k, const double *__restrict__ fi,
+                  const double *__restrict__ dfe, const double *__restrict__ dfo,
+                  double *__restrict__ g) {
   FCG_GRID_STRIDE(c, m.n) {
     double gx = 0.0, gy = 0.0, gz = 0.0;
-    for (int e = m.cf_ptr[c]; e < m.cf_ptr[c + 1]; ++e) {
-      int ent = m.cf_ent[e];
-      long long f = (ent > 0 ? ent : -ent) - 1;
-      double ex = dfe[f], ey = dfe[m.nin + f], ez = dfe[2LL * m.nin + f];
-      if (ent > 0) {
-        gx = gx + ex;
-        gy = gy + ey;
-        gz = gz + ez;
-      } else {
-        gx = gx - ex;
-        gy = gy - ey;
-        gz = gz - ez;
+    // the loads of kBatch faces are issued together; added in face order, + as owner, - as
+    // neighbour (x - e is x + (-e) to the bit)
+    const int e1 = m.cf_ptr[c + 1];
+    for (int e = m.cf_ptr[c]; e < e1; e += kBatch) {
+      int ent[kBatch];
+#pragma unroll
+      for (int u = 0; u < kBatch; ++u) ent[u] = e + u < e1 ? m.cf_ent[e + u] : 0;
+      double t[kBatch][3];
+#pragma unroll
+      for (int u = 0; u < kBatch; ++u) {
+        const long long f = (ent[u] > 0 ? ent[u] : -ent[u]) - 1;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) t[u][k] = ent[u] ? dfe[(long long)k * m.nin + f] : 0.0;
+      }
+#pragma unroll
+      for (int u = 0; u < kBatch; ++u) {
+        if (!ent[u]) break;
+        const bool own = ent[u] > 0;
+        gx = gx + signed_term(own, t[u][0]);
+        gy = gy + signed_term(own, t[u][1]);
+        gz = gz + signed_term(own, t[u][2]);
       }
     }
     if (m.noc)  // the O-C pairs after the inner faces, + on the left cell, - on the right
@@ -98,7 +161,7 @@ __global__ void k_gauss_cells(MeshView m, const double *__restrict__ fi,
       gy = gy + fb * m.ary[f];
       gz = gz + fb * m.arz[f];
     }
-    double volr = 1.0 / m.vol[c];
+    const double volr = k.volr[c];
     g[3 * c] = gx * volr;
     g[3 * c + 1] = gy * volr;
     g[3 * c + 2] = gz * volr;
@@ -227,6 +290,27 @@ __global__ void k_bpres_oc(MeshView m, long long s0, double *__restrict__ p,
   }
 }
 
+int ensure_gauss_const(fcg_context *c, GaussConst *k) {
+  const size_t nv = sizeof(double) * (size_t)c->n;
+  if (!c->gconst_ready) {
+    FCG_CUDA_TRY(c, c->gconst.ensure(nv + sizeof(int)));
+    double *volr = c->gconst.as<double>();
+    FCG_CUDA_TRY(c, cudaMemsetAsync(volr + c->n, 0, sizeof(int), c->stream));
+    const int g = grid_for(std::max(c->mv.n, c->mv.nin), c->num_sms);
+    k_gauss_const<<<g, kTPB, 0, c->stream>>>(c->mv, volr, (int *)(volr + c->n));
+    FCG_CHECK_LAUNCH(c, "k_gauss_const");
+    c->gconst_ready = true;
+  }
+  *k = {c->gconst.as<double>(), (const int *)(c->gconst.as<double>() + c->n)};
+  return FCG_OK;
+}
+
+// Do the byte ranges [a, a + na) and [b, b + nb) share a byte?
+bool overlap(const void *a, size_t na, const void *b, size_t nb) {
+  const uintptr_t x = (uintptr_t)a, y = (uintptr_t)b;
+  return x < y + nb && y < x + na;
+}
+
 int ensure_lsq_matrix(fcg_context *c) {
   if (c->dmat_ready) return FCG_OK;
   FCG_CUDA_TRY(c, c->dmat.ensure(sizeof(double) * 9 * (size_t)c->n));
@@ -269,30 +353,32 @@ extern "C" int fcg_grad(fcg_context *c, const double *phi, double *dPhidxi, int 
   if ((rc = stage_in(c, phi, sizeof(double) * c->ntot, 0, true, &dphi, &hphi))) return rc;
   if ((rc = stage_in(c, dPhidxi, n3, 1, method == FCG_GRAD_GAUSS_CORRECTED, &dg, &hg))) return rc;
   const MeshView &m = c->mv;
-  const int gf = grid_for(m.nin, c->num_sms), gc = grid_for(m.n, c->num_sms);
+  // several waves of blocks: a block's start hides another's last loads (8 an SM: 256 us a
+  // pass at 128^3, 32: 232)
+  const int gf = grid_for(m.nin, c->num_sms, 32), gc = grid_for(m.n, c->num_sms, 32);
   if (method == FCG_GRAD_LSQ) {
     if ((rc = ensure_lsq_matrix(c))) return rc;
     k_lsq_cells<<<gc, kTPB, 0, c->stream>>>(m, (const double *)dphi, c->dmat.as<double>(),
                                             (double *)dg);
     FCG_CHECK_LAUNCH(c, "k_lsq_cells");
   } else {
-    // scratch: dfe[3*nin] | old gradient [3n] | new gradient [3n] | O-C terms [3*noc]
-    size_t nin3 = 3 * (size_t)(m.nin > 0 ? m.nin : 1), noc3 = 3 * (size_t)m.noc;
-    FCG_CUDA_TRY(c, c->scratch.ensure(sizeof(double) * (nin3 + noc3) + 2 * n3));
-    double *dfe = c->scratch.as<double>();
-    double *gA = dfe + nin3, *gB = gA + 3 * (size_t)m.n;
-    double *dfo = gB + 3 * (size_t)m.n;
-    int passes = method == FCG_GRAD_GAUSS_CORRECTED ? 1 : nigrad;
-    const double *gold = gA;
-    if (method == FCG_GRAD_GAUSS_CORRECTED) {
-      gold = (const double *)dg;  // old gradient = incoming (grad_gauss_corrected.f90:38-40)
-    } else {
-      FCG_CUDA_TRY(c, cudaMemsetAsync(gA, 0, n3, c->stream));  // grad_gauss.f90:38-40
-    }
+    // scratch: dfe[3*nin] | O-C terms [3*noc] | gradient [3n], if the result's array
+    // shares memory with phi.  A pass reads the old gradient in its face kernels only, so
+    // its cell kernel writes the new one over it (:116-120).
+    const bool apart = !overlap(dphi, sizeof(double) * c->ntot, dg, n3);
+    const size_t nin3 = 3 * (size_t)(m.nin > 0 ? m.nin : 1), noc3 = 3 * (size_t)m.noc;
+    FCG_CUDA_TRY(c, c->scratch.ensure(sizeof(double) * (nin3 + noc3) + (apart ? 0 : n3)));
+    GaussConst k;
+    if ((rc = ensure_gauss_const(c, &k))) return rc;
+    double *dfe = c->scratch.as<double>(), *dfo = dfe + nin3;
+    double *g = apart ? (double *)dg : dfo + noc3;
+    const int passes = method == FCG_GRAD_GAUSS_CORRECTED ? 1 : nigrad;
+    // old gradient: incoming (grad_gauss_corrected.f90:38-40) or zero (grad_gauss.f90:38-40)
+    const double *gold = method == FCG_GRAD_GAUSS_CORRECTED ? (const double *)dg : nullptr;
     for (int lc = 1; lc <= passes; ++lc) {
-      double *gnew = (gold == gA) ? gB : gA;  // never the buffer the pass reads
       if (m.nin > 0) {
-        k_gauss_faces<<<gf, kTPB, 0, c->stream>>>(m, (const double *)dphi, gold, dfe);
+        auto faces = gold ? k_gauss_faces<false> : k_gauss_faces<true>;
+        faces<<<gf, kTPB, 0, c->stream>>>(m, k, (const double *)dphi, gold, dfe);
         FCG_CHECK_LAUNCH(c, "k_gauss_faces");
       }
       if (m.noc > 0) {
@@ -300,11 +386,11 @@ extern "C" int fcg_grad(fcg_context *c, const double *phi, double *dPhidxi, int 
                                                                          gold, dfo);
         FCG_CHECK_LAUNCH(c, "k_gauss_oc");
       }
-      k_gauss_cells<<<gc, kTPB, 0, c->stream>>>(m, (const double *)dphi, dfe, dfo, gnew);
+      k_gauss_cells<<<gc, kTPB, 0, c->stream>>>(m, k, (const double *)dphi, dfe, dfo, g);
       FCG_CHECK_LAUNCH(c, "k_gauss_cells");
-      gold = gnew;  // :116-120
+      gold = g;
     }
-    FCG_CUDA_TRY(c, cudaMemcpyAsync(dg, gold, n3, cudaMemcpyDeviceToDevice, c->stream));
+    if (!apart) FCG_CUDA_TRY(c, cudaMemcpyAsync(dg, g, n3, cudaMemcpyDeviceToDevice, c->stream));
   }
   if ((rc = stage_out(c, dPhidxi, dg, n3, hg))) return rc;
   if (hg) FCG_CUDA_TRY(c, cudaStreamSynchronize(c->stream));
