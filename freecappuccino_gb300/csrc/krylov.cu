@@ -13,7 +13,8 @@
 //    the stop test) on the device.  No host round trip per sweep.
 //  * One sweep is a fixed chain of kernels captured once into the body of a CUDA-graph
 //    WHILE node; the kernel that evaluates the stop test clears the node's condition.
-//    A whole solve is one graph launch.
+//    A whole solve is one graph launch.  DPCG on a system whose rows the resident threads
+//    can hold is one cooperative launch instead (resident_cg.cuh).
 //  * The DIC/DILU triangular solves run in one launch each: on a lexicographic hex block
 //    as wavefront-tiled sweeps (wave_sweep.cuh), elsewhere with rows waiting on the rows
 //    they read; one launch per level (rows of one level depend only on rows of earlier
@@ -58,7 +59,9 @@ struct Scal {
 };
 
 // Grid of each reduction kernel: one full wave of resident blocks on every SM (from the
-// occupancy calculator), so no kernel runs a partial second wave.
+// occupancy calculator), so no kernel runs a partial second wave, and no more blocks than
+// have rows: an empty block still takes a ticket (a
+// sweep of dpcg_mixed at 24^3: 31 us with full waves, 20 without them).
 struct Grids {
   int init, p, spmv, update, dot, bdot, bp, bspmv1, bupd1, bspmv2, bupd2, fin, plain;
   int mstart, mspmv, mupd, mru1, mru2, mp;
@@ -78,6 +81,7 @@ struct KrylovState {
   // made at the first solve that sweeps
   DBuf wbuf;
   wave::Arrays<double> wv{};
+  DBuf rbuf;  // slots of the resident form's grid-wide sums (resident_cg.cuh)
   DBuf trace;
   // mixed precision: FP32 copy of D^-1/2 A D^-1/2 in the sliced layout, the scaling
   // D^-1/2 in FP64 and the FP32 inner vectors (correction y, residual r, direction p, Ap)
@@ -121,6 +125,7 @@ void destroy_krylov(KrylovState *k) {
   if (k->S) cudaFree(k->S);
   k->vec.release();
   k->wbuf.release();
+  k->rbuf.release();
   k->trace.release();
   k->mixed.release();
   k->sfb.release();
@@ -755,6 +760,11 @@ __global__ void __launch_bounds__(kTPB, 8) k_final(SellView s, int n, const doub
 }
 
 }  // namespace
+}  // namespace fcg
+
+#include "resident_cg.cuh"
+
+namespace fcg {
 
 // ---------------------------------------------------------------------------
 // Host side
@@ -810,7 +820,7 @@ static int ensure_state(fcg_context *c, int nsw) {
         cudaGetLastError();
         b = 1;
       }
-      return c->num_sms * std::max(1, std::min(b, 8));
+      return std::min(c->num_sms * std::max(1, std::min(b, 8)), (c->n + kTPB - 1) / kTPB);
     };
     Grids &g = k->gr;
     g.init = occ((const void *)k_init);
@@ -1097,6 +1107,40 @@ static bool graphs_disabled() {
   return e && e[0] == '1';
 }
 
+// Rows a thread of the resident form (resident_cg.cuh) for this system, 0 where it does not
+// apply: O-C pairs, a system the threads cannot hold, or the host-driven loop.
+static int resident_rows(const fcg_context *c) {
+  if (c->mv.noc || graphs_disabled()) return 0;
+  const int warps = std::min(c->num_sms, kResidentBlocks) * (kResidentThreads / 32);
+  const int rows = (c->sv.nslices + warps - 1) / warps;
+  return rows <= 2 ? rows : rows <= kResidentRows ? kResidentRows : 0;
+}
+
+static int launch_resident(fcg_context *c, int rows) {
+  KrylovState *k = c->ks;
+  const int sms = std::min(c->num_sms, kResidentBlocks);
+  const int warps = std::min(kResidentThreads / 32, (c->sv.nslices + sms - 1) / sms);
+  const int grid = (c->sv.nslices + warps * rows - 1) / (warps * rows);
+  FCG_CUDA_TRY(c, k->rbuf.ensure(sizeof(double) * 5 * (size_t)slot_set(grid)));
+  ResidentCg a{c->sv, c->n, k->sval, k->invd, k->x, k->res, k->zk, k->rtmp,
+               k->pk, k->qk, k->S, k->rbuf.as<double>(), k->trace.as<double>()};
+  k_resident_start<<<grid_for(std::max(c->n, 5 * slot_set(grid)), c->num_sms), kTPB, 0, c->stream>>>(a, grid);
+  FCG_CHECK_LAUNCH(c, "k_resident_start");
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(32 * warps);
+  cfg.stream = c->stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  auto kernel = rows == 1 ? k_resident_dpcg<1> : rows == 2 ? k_resident_dpcg<2>
+                                                           : k_resident_dpcg<kResidentRows>;
+  FCG_CUDA_TRY(c, cudaLaunchKernelEx(&cfg, kernel, a));
+  return FCG_OK;
+}
+
 // Captures the WHILE-node graph of one solver kind.
 static int build_graph(fcg_context *c, int kind) {
   KrylovState *k = c->ks;
@@ -1218,7 +1262,10 @@ static int run_solver(fcg_context *c, int kind, const double *a, const double *s
     }
     FCG_CHECK_LAUNCH(c, "k_factor_level");
   }
-  if (!graphs_disabled()) {
+  const int rows = kind == SK_DPCG ? resident_rows(c) : 0;
+  if (rows) {
+    if ((rc = launch_resident(c, rows))) return rc;
+  } else if (!graphs_disabled()) {
     if ((rc = build_graph(c, kind))) return rc;
     FCG_CUDA_TRY(c, cudaGraphLaunch(k->exec[kind], c->stream));
   } else {
@@ -1262,8 +1309,9 @@ static int run_solver(fcg_context *c, int kind, const double *a, const double *s
   if (S.status) {
     const char *what = S.status == FCG_ERR_PIVOT     ? "zero or non-finite pivot in the factor"
                        : S.status == FCG_ERR_TIMEOUT
-                           ? (S.wait_fail ? "a triangular-sweep dependency wait gave up"
-                                          : "solver loop exceeded nsw + 2 sweeps")
+                           ? (S.wait_fail == 2 ? "a grid-wide sum's wait gave up"
+                              : S.wait_fail    ? "a triangular-sweep dependency wait gave up"
+                                               : "solver loop exceeded nsw + 2 sweeps")
                                                      : "non-finite value in a reduction";
     return set_error(c, S.status, what);
   }
