@@ -106,7 +106,7 @@ __device__ __forceinline__ void for_share(const Split &sp, const BSys *sys, int 
 // This CTA's block sums of system k: part[(k gridDim + CTA) 2 ..].
 template <int NV>
 __device__ __forceinline__ void put_partial(double (&v)[NV], double *part, int k,
-                                            double (*sh)[kWarps]) {
+                                            double (*sh)[kTPB]) {
   block_sum<NV>(v, sh);
   if (threadIdx.x == 0)
 #pragma unroll
@@ -309,7 +309,7 @@ __device__ __noinline__ void close_phase(int phase, BSys *sys, BCtl *ctl, const 
 __global__ void __launch_bounds__(kTPB, kResident)
     k_batch_dpcg(BSys *sys, int nsys, int spi, double *part, BCtl *ctl, int max_loops,
                  long long spin_limit, int absent_block) {
-  __shared__ double sh[2][kWarps];
+  __shared__ double sh[2][kTPB];
   __shared__ Split sp;
   // diagnostics only (fcg_batch_set_wait_test): one CTA never reaches a barrier, so the
   // others' bounded waits run out and the solve ends with FCG_ERR_TIMEOUT

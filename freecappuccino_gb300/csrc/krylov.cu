@@ -286,7 +286,7 @@ __device__ __noinline__ void cg_close_sweep(Scal *S, double resl, double sk_new,
 }
 
 // pk = M^-1 res + bet*pk: Jacobi (dpcg.f90:85-100) or z from the sweeps (iccg.f90:278).
-__global__ void __launch_bounds__(kTPB, 8) k_cg_p(int n, const double *__restrict__ res, const double *__restrict__ invd,
+__global__ void __launch_bounds__(kTPB, 6) k_cg_p(int n, const double *__restrict__ res, const double *__restrict__ invd,
                        const double *__restrict__ z, double *__restrict__ pk, const Scal *S,
                        int kind) {
   if (solve_done(S)) return;
@@ -321,7 +321,7 @@ __global__ void __launch_bounds__(kTPB, 8) k_cg_spmv(SellView s, int n, const do
 
 // fi += alf*pk, res -= alf*qk, resl = sum|res| (dpcg.f90:124-142); DPCG also forms
 // the next sk and beta in the same pass.
-__global__ void __launch_bounds__(kTPB, 8) k_cg_update(int n, double *__restrict__ x, double *__restrict__ res,
+__global__ void __launch_bounds__(kTPB, 5) k_cg_update(int n, double *__restrict__ x, double *__restrict__ res,
                             const double *__restrict__ pk, const double *__restrict__ qk,
                             const double *__restrict__ invd, Scal *S, double *partials,
                             double *trace, cudaGraphConditionalHandle h, int use_cond, int kind) {
@@ -344,7 +344,7 @@ __global__ void __launch_bounds__(kTPB, 8) k_cg_update(int n, double *__restrict
 }
 
 // ICCG: sk = sum res*z, bet = sk/s0 (iccg.f90:268-273).
-__global__ void __launch_bounds__(kTPB, 8) k_cg_dot(int n, const double *__restrict__ res, const double *__restrict__ z,
+__global__ void __launch_bounds__(kTPB, 5) k_cg_dot(int n, const double *__restrict__ res, const double *__restrict__ z,
                          Scal *S, double *partials) {
   if (solve_done(S)) return;
   double v[1] = {0.0};
@@ -415,7 +415,7 @@ __global__ void k_factor_level(const int *__restrict__ rows, int count,
 
 // --- BiCGStab sweep (bicgstab.f90:99-224) -------------------------------------
 // bet = sum res*reso; om = bet*gam/(alf*beto+small); beto = bet
-__global__ void __launch_bounds__(kTPB, 8) k_bi_dot1(int n, const double *__restrict__ res, const double *__restrict__ reso,
+__global__ void __launch_bounds__(kTPB, 5) k_bi_dot1(int n, const double *__restrict__ res, const double *__restrict__ reso,
                           Scal *S, double *partials) {
   if (solve_done(S)) return;
   double v[1] = {0.0};
@@ -429,7 +429,7 @@ __global__ void __launch_bounds__(kTPB, 8) k_bi_dot1(int n, const double *__rest
 }
 
 // pk = res + om*(pk - alf*uk)
-__global__ void __launch_bounds__(kTPB, 8) k_bi_p(int n, const double *__restrict__ res, const double *__restrict__ uk,
+__global__ void __launch_bounds__(kTPB, 6) k_bi_p(int n, const double *__restrict__ res, const double *__restrict__ uk,
                        double *__restrict__ pk, const Scal *S) {
   if (solve_done(S)) return;
   const double om = __ldcg(&S->om), alf = __ldcg(&S->alf);
@@ -457,7 +457,7 @@ __global__ void __launch_bounds__(kTPB, 8) k_bi_spmv1(SellView s, int n, const d
 }
 
 // fi += gam*zk; res -= gam*uk
-__global__ void __launch_bounds__(kTPB, 8) k_bi_upd1(int n, double *__restrict__ x, double *__restrict__ res,
+__global__ void __launch_bounds__(kTPB, 6) k_bi_upd1(int n, double *__restrict__ x, double *__restrict__ res,
                           const double *__restrict__ zk, const double *__restrict__ uk,
                           const Scal *S) {
   if (solve_done(S)) return;
@@ -500,7 +500,7 @@ __device__ __noinline__ void bi_close_sweep(Scal *S, double resl, double *trace,
 }
 
 // fi += alf*zk; res -= alf*vk; resl = sum|res|; stop test
-__global__ void __launch_bounds__(kTPB, 8) k_bi_upd2(int n, double *__restrict__ x, double *__restrict__ res,
+__global__ void __launch_bounds__(kTPB, 5) k_bi_upd2(int n, double *__restrict__ x, double *__restrict__ res,
                           const double *__restrict__ zk, const double *__restrict__ vk, Scal *S,
                           double *partials, double *trace, cudaGraphConditionalHandle h,
                           int use_cond) {
@@ -622,7 +622,7 @@ __device__ __noinline__ void mx_decide(Scal *S, double rrn) {
 
 // y32 += alf p32, r32 -= alf q32, rr' = r32.r32; decides whether a reliable update
 // follows and, inside the graph, arms the IF node that runs it.  float4 accesses.
-__global__ void __launch_bounds__(kTPB, 6)
+__global__ void __launch_bounds__(kTPB, 5)
     k_mx_update(int n, float *__restrict__ y32, float *__restrict__ r32,
                 const float *__restrict__ p32, const float *__restrict__ q32, Scal *S,
                 double *partials, cudaGraphConditionalHandle hif, int use_cond) {
@@ -716,7 +716,7 @@ __global__ void __launch_bounds__(kTPB, 8)
 }
 
 // p32 = r32 + bet p32; closes the loop body (float4 accesses)
-__global__ void __launch_bounds__(kTPB, 6)
+__global__ void __launch_bounds__(kTPB, 5)
     k_mx_p(int n, const float *__restrict__ r32, float *__restrict__ p32, Scal *S,
            cudaGraphConditionalHandle h, int use_cond) {
   if (solve_done(S)) {

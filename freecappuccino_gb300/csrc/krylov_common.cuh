@@ -14,33 +14,49 @@ constexpr int kWarps = kTPB / 32;
 // ---------------------------------------------------------------------------
 // Deterministic reductions
 // ---------------------------------------------------------------------------
+// Rows of the shared array block_sum() works in, kTPB doubles each.
+__host__ __device__ constexpr int sum_rows(int NV) { return NV < 4 ? NV : 4; }
+
+// Sums of v over the block, in every thread.  The threads' values go through shared memory
+// to one warp a value, which adds eight per lane before its lanes: 12 FP64 instructions a
+// value and block.  An FP64 instruction holds an SM's pipe for 16 cycles whatever number of
+// its lanes work, so trees over the lanes of every warp (43 a value) kept a full SM's blocks
+// busy for 5 us at the end of a kernel with two sums (k_cg_update at 64^3: 22 -> 18 us).
 template <int NV>
-__device__ __forceinline__ void block_sum(double (&v)[NV], double (*sh)[kWarps]) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-    for (int k = 0; k < NV; ++k) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
+__device__ __forceinline__ void block_sum(double (&v)[NV], double (*sh)[kTPB]) {
+  constexpr int R = sum_rows(NV);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  if (lane == 0)
 #pragma unroll
-    for (int k = 0; k < NV; ++k) sh[k][w] = v[k];
-  __syncthreads();
-  if (w == 0) {
+  for (int k0 = 0; k0 < NV; k0 += R) {
 #pragma unroll
-    for (int k = 0; k < NV; ++k) v[k] = lane < kWarps ? sh[k][lane] : 0.0;
+    for (int k = 0; k < R; ++k)
+      if (k0 + k < NV) sh[k][threadIdx.x] = v[k0 + k];
+    __syncthreads();
+    if (w < R && k0 + w < NV) {
+      double t = sh[w][lane], u = sh[w][lane + 32];
+#pragma unroll 1
+      for (int i = 64; i < kTPB; i += 64) {
+        t += sh[w][lane + i];
+        u += sh[w][lane + i + 32];
+      }
+      t += u;
 #pragma unroll
-    for (int o = kWarps / 2; o > 0; o >>= 1)
+      for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+      if (lane == 0) sh[w][0] = t;  // the warp has read the row
+    }
+    __syncthreads();
 #pragma unroll
-      for (int k = 0; k < NV; ++k) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
+    for (int k = 0; k < R; ++k)
+      if (k0 + k < NV) v[k0 + k] = sh[k][0];
+    __syncthreads();
   }
-  __syncthreads();
 }
 
 // Stores this block's sums; returns true in the last block to arrive, whose thread 0
 // then holds the grid-wide sums in v (partials added in block-index order).
 template <int NV>
 __device__ __forceinline__ bool reduce_commit(double (&v)[NV], double *partials, unsigned int *ticket) {
-  __shared__ double sh[NV][kWarps];
+  __shared__ double sh[sum_rows(NV)][kTPB];
   __shared__ bool am_last;
   block_sum<NV>(v, sh);
   const int G = gridDim.x;
