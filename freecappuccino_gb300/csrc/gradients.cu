@@ -100,13 +100,6 @@ __global__ void k_gauss_oc(MeshView m, const double *__restrict__ fi,
 
 constexpr int kBatch = 3;
 
-// own ? x : -x on the integer pipe: the compiler's own choice adds an FP64 instruction, of
-// which a cell kernel has none to spare.
-__device__ __forceinline__ double signed_term(bool own, double x) {
-  const unsigned long long flip = own ? 0ULL : 0x8000000000000000ULL;
-  return __longlong_as_double(__double_as_longlong(x) ^ flip);
-}
-
 // Bound by the FP64 pipe: 21 instructions a cell (1/vol is the mesh's, and the sign of a
 // neighbour's term an integer flip).  128^3: 106 us; with a quotient and two signed sums a
 // face 208, with negations in FP64 189.  Batches of 2, 3 and 6 faces differ by 2 %.

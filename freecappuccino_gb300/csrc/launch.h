@@ -21,4 +21,14 @@ inline int grid_for(long long count, int num_sms, int blocks_per_sm = 8) {
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < (count);     \
        i += (long long)gridDim.x * blockDim.x)
 
+#ifdef __CUDACC__
+// own ? x : -x on the integer pipe, for sums whose terms take a sign per face: x - e is
+// x + (-e) to the bit.  A choice between s + e and s - e, or a negation, costs a second FP64
+// instruction a term, and the FP64 pipe is what bounds such a kernel.
+__device__ __forceinline__ double signed_term(bool own, double x) {
+  const unsigned long long flip = own ? 0ULL : 0x8000000000000000ULL;
+  return __longlong_as_double(__double_as_longlong(x) ^ flip);
+}
+#endif
+
 }  // namespace fcg

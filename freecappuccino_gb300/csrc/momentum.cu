@@ -9,6 +9,9 @@
 //      divergence, the volume sources, the face fluxes, the boundary loops,
 //      Crank-Nicolson -- and assembles the three diagonals from its own CSR row.
 // Compiled with --fmad=false: bit-identical to the reference's loops on the same inputs.
+// Both kernels are bound by the FP64 pipe: 216 instructions a face (83 % of the pipe, 1.09
+// ms at 96^3) and 121 a cell (79 %, 215 us; 277 with the faces' terms added or subtracted by
+// choice, which took two instructions a term).
 //
 // MIN and MAX keep the first argument on ties (only the sign of a zero can differ).
 #include "face_geo.h"
@@ -94,14 +97,14 @@ __device__ __forceinline__ double face_value(const MeshView &m, int limiter, int
     }
     return fi[f] + fxp * psi * (fi[s] - fi[f]);
   } else {  // FCG_CONV_MUSCL, :254-320
+    // theta = 1/8; theta * 0.5 is one exact scaling of the central value's sum
     const double theta = 0.125;
     // the reference's central correction repeats the upwind one's three products first,
     // so it continues from the same partial sum
     const double g2 = g[3 * f] * o.dux + g[3 * f + 1] * o.duy + g[3 * f + 2] * o.duz;
     const double gc = g2 + g[3 * s] * o.ddx + g[3 * s + 1] * o.ddy + g[3 * s + 2] * o.ddz;
     const double fv2 = fi[f] + g2;
-    const double fvc = 0.5 * (fi[f] + fi[s] + gc);
-    return theta * fvc + (1.0 - theta) * fv2;
+    return 0.5 * theta * (fi[f] + fi[s] + gc) + (1.0 - theta) * fv2;
   }
 }
 
@@ -164,7 +167,7 @@ __global__ void __launch_bounds__(kTPB)
     const double fvuds = fpos * F.v[p] + fneg * F.v[q];
     const double fwuds = fpos * F.w[p] + fneg * F.w[q];
     // face_value from the upwind side (:129-150): one path for both signs of the flux
-    const bool fwd = flomass >= 0.0;
+    const bool fwd = !(flomass < 0.0);
     const int uc = fwd ? p : q, dc = fwd ? q : p;
     const double lam = fwd ? fxp : fxn;
     Offs o{};
@@ -299,28 +302,16 @@ __global__ void k_uvw_cells(MeshView m, fcg_uvw_params prm, UvwView F, int bst_i
     for (int e = e0; e < e1; ++e) {
       const int ent = m.cf_ent[e];
       const int f = (ent > 0 ? ent : -ent) - 1;
-      if (ent > 0) {
-        s0 = s0 - fdiv[3 * f];
-        s1 = s1 - fdiv[3 * f + 1];
-        s2 = s2 - fdiv[3 * f + 2];
-      } else {
-        s0 = s0 + fdiv[3 * f];
-        s1 = s1 + fdiv[3 * f + 1];
-        s2 = s2 + fdiv[3 * f + 2];
-      }
+      s0 = s0 + signed_term(ent < 0, fdiv[3 * f]);
+      s1 = s1 + signed_term(ent < 0, fdiv[3 * f + 1]);
+      s2 = s2 + signed_term(ent < 0, fdiv[3 * f + 2]);
     }
     if (m.noc)  // the O-C pairs (fieldManipulation.f90:110-125)
       for (int e = m.oc_cptr[c]; e < m.oc_cptr[c + 1]; ++e) {
         const int v = m.oc_vix[e], i = v < m.noc ? v : v - m.noc;
-        if (v < m.noc) {
-          s0 = s0 - odiv[3 * i];
-          s1 = s1 - odiv[3 * i + 1];
-          s2 = s2 - odiv[3 * i + 2];
-        } else {
-          s0 = s0 + odiv[3 * i];
-          s1 = s1 + odiv[3 * i + 1];
-          s2 = s2 + odiv[3 * i + 2];
-        }
+        s0 = s0 + signed_term(v >= m.noc, odiv[3 * i]);
+        s1 = s1 + signed_term(v >= m.noc, odiv[3 * i + 1]);
+        s2 = s2 + signed_term(v >= m.noc, odiv[3 * i + 2]);
       }
     for (int e = b0; e < b1; ++e) {
       const int f = m.cb_face[e];
@@ -363,15 +354,9 @@ __global__ void k_uvw_cells(MeshView m, fcg_uvw_params prm, UvwView F, int bst_i
     for (int e = e0; e < e1; ++e) {
       const int ent = m.cf_ent[e];
       const int f = (ent > 0 ? ent : -ent) - 1;
-      if (ent > 0) {
-        s0 = s0 + fsrc[3 * f];
-        s1 = s1 + fsrc[3 * f + 1];
-        s2 = s2 + fsrc[3 * f + 2];
-      } else {
-        s0 = s0 - fsrc[3 * f];
-        s1 = s1 - fsrc[3 * f + 1];
-        s2 = s2 - fsrc[3 * f + 2];
-      }
+      s0 = s0 + signed_term(ent > 0, fsrc[3 * f]);
+      s1 = s1 + signed_term(ent > 0, fsrc[3 * f + 1]);
+      s2 = s2 + signed_term(ent > 0, fsrc[3 * f + 2]);
     }
     if (m.noc)  // the O-C pairs (:186-215): ar (left cell) or al (right) off sp, the sources
       for (int e = m.oc_cptr[c]; e < m.oc_cptr[c + 1]; ++e) {
@@ -380,15 +365,9 @@ __global__ void k_uvw_cells(MeshView m, fcg_uvw_params prm, UvwView F, int bst_i
         sp0 = sp0 - co;
         sp1 = sp1 - co;
         sp2 = sp2 - co;
-        if (v < m.noc) {
-          s0 = s0 + osrc[3 * i];
-          s1 = s1 + osrc[3 * i + 1];
-          s2 = s2 + osrc[3 * i + 2];
-        } else {
-          s0 = s0 - osrc[3 * i];
-          s1 = s1 - osrc[3 * i + 1];
-          s2 = s2 - osrc[3 * i + 2];
-        }
+        s0 = s0 + signed_term(v < m.noc, osrc[3 * i]);
+        s1 = s1 + signed_term(v < m.noc, osrc[3 * i + 1]);
+        s2 = s2 + signed_term(v < m.noc, osrc[3 * i + 2]);
       }
     // boundary loops (:223-378): inlet, outlet, symmetry, wall
     for (int e = b0; e < b1; ++e) {
@@ -590,7 +569,7 @@ extern "C" int fcg_calcuvw(fcg_context *c, const fcg_uvw_params *prm, const fcg_
       case FCG_CONV_FLUX_LIMITER: faces = k_uvw_faces<FCG_CONV_FLUX_LIMITER>; break;
       default: break;
     }
-    faces<<<grid_for(m.nin, c->num_sms), kTPB, 0, c->stream>>>(m, *prm, V, geo, (double *)da,
+    faces<<<grid_for(m.nin, c->num_sms, 64), kTPB, 0, c->stream>>>(m, *prm, V, geo, (double *)da,
                                                                  fsrc, fdiv);
     FCG_CHECK_LAUNCH(c, "k_uvw_faces");
   }
@@ -598,7 +577,7 @@ extern "C" int fcg_calcuvw(fcg_context *c, const fcg_uvw_params *prm, const fcg_
   if ((rc = bnd_geo(c, &bg))) return rc;
   long long ncb = 0;
   for (int t = 0; t < B_NTYPES; ++t) ncb += c->cnt[t];
-  k_uvw_cells<<<grid_for(m.n, c->num_sms), kTPB, 0, c->stream>>>(
+  k_uvw_cells<<<grid_for(m.n, c->num_sms, 64), kTPB, 0, c->stream>>>(
       m, *prm, V, c->bst[B_INLET], c->bst[B_OUTLET], bg, ncb, (double *)da, fsrc, fdiv, osrc,
       odiv, (double *)ddv, (double *)drhs, (double *)dap);
   FCG_CHECK_LAUNCH(c, "k_uvw_cells");
