@@ -595,7 +595,7 @@ __global__ void __launch_bounds__(kTPB)
 // 64^3, one output and two shared-memory loads for every one or two multiply-adds) was the
 // shared-memory pipe; here a thread holds a 4 x 4 block of the first product and a 4 x 8
 // block of the second (a quarter of the tile's cells; the quarters are added at the end),
-// 16-byte loads, 8 to 11 multiply-adds a load: about 88 us.
+// 16-byte loads, 8 to 11 multiply-adds a load: 84 us.
 __global__ void __launch_bounds__(kTPB, 3)
     k_lp_layer_bwd(int n, const float *__restrict__ dh, const float *__restrict__ z,
                    const __nv_bfloat16 *__restrict__ hin, const float *__restrict__ m,
@@ -615,8 +615,11 @@ __global__ void __launch_bounds__(kTPB, 3)
 #pragma unroll
     for (int k = 0; k < 8; ++k) gw[o][k] = 0.f;
   }
-  const int cg = t & 15, rg = t >> 4;                        // columns 4 cg.., cells 4 rg..
-  const int kg = t >> 6, og = (t >> 3) & 7, xg = t & 7;      // cells 16 kg.., outputs 4 og..
+  // first product: a warp takes 16 cells and 32 columns, a thread the cells rg + 4 r and the
+  // columns 4 cg..: its loads are one bank pass each
+  const int cg = (t & 7) + 8 * ((t >> 5) & 1), rg = 16 * (t >> 6) + ((t >> 3) & 3);
+  // second product: cells 16 kg.., outputs 4 og.., columns 4 xg.. and C + 4 xg..
+  const int kg = t >> 6, og = (t >> 3) & 7, xg = t & 7;
   const long long per = ((long long)n + gridDim.x - 1) / gridDim.x;
   const long long c0 = (long long)blockIdx.x * per, c1 = min((long long)n, c0 + per);
   for (long long base = c0; base < c1; base += B) {
@@ -653,7 +656,7 @@ __global__ void __launch_bounds__(kTPB, 3)
     for (int o = 0; o < C; o += 4) {
       float4 d[4], w[4];
 #pragma unroll
-      for (int r = 0; r < 4; ++r) d[r] = *reinterpret_cast<const float4 *>(&dzs[4 * rg + r][o]);
+      for (int r = 0; r < 4; ++r) d[r] = *reinterpret_cast<const float4 *>(&dzs[rg + 4 * r][o]);
 #pragma unroll
       for (int j = 0; j < 4; ++j)
         w[j] = *reinterpret_cast<const float4 *>(&W[(o + j) * 2 * C + 4 * cg]);
@@ -670,7 +673,7 @@ __global__ void __launch_bounds__(kTPB, 3)
     }
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
-      const int cl = 4 * rg + r;
+      const int cl = rg + 4 * r;
       if (cl >= cnt) break;
       float4 v = make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
       if (cg < C / 4) {
@@ -685,8 +688,8 @@ __global__ void __launch_bounds__(kTPB, 3)
 #pragma unroll 4
     for (int cl = 16 * kg; cl < 16 * kg + 16; ++cl) {
       const float4 d = *reinterpret_cast<const float4 *>(&dzs[cl][4 * og]);
-      const float4 xa = *reinterpret_cast<const float4 *>(&xs[cl][8 * xg]);
-      const float4 xb = *reinterpret_cast<const float4 *>(&xs[cl][8 * xg + 4]);
+      const float4 xa = *reinterpret_cast<const float4 *>(&xs[cl][4 * xg]);
+      const float4 xb = *reinterpret_cast<const float4 *>(&xs[cl][C + 4 * xg]);
       const float dv[4] = {d.x, d.y, d.z, d.w};
 #pragma unroll
       for (int o = 0; o < 4; ++o) {
@@ -711,7 +714,7 @@ __global__ void __launch_bounds__(kTPB, 3)
     for (int o = 0; o < 4; ++o) {
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
-        float *p = &red[(4 * og + o) * 2 * C + 8 * xg + k];
+        float *p = &red[(4 * og + o) * 2 * C + (k < 4 ? 0 : C - 4) + 4 * xg + k];
         *p = g == 0 ? gw[o][k] : *p + gw[o][k];
       }
       if (xg == 0) {
@@ -727,8 +730,8 @@ __global__ void __launch_bounds__(kTPB, 3)
 
 // dh_prev += Ahat dm (Ahat of the pressure system is symmetric); eight lanes a cell, four
 // channels a lane, the loads of a row of at most eight slots in flight together, four blocks
-// an SM: about 71 us at 64^3 (96 with the 68 registers of three blocks, 83 with the spills
-// of five); a lane a channel and a slot at a time took 128.
+// an SM: 66 us at 64^3 (71 with dh_prev read after the sums, 96 with the 68 registers of
+// three blocks, 83 with the spills of five); a lane a channel and a slot at a time took 128.
 __global__ void __launch_bounds__(kTPB, 4)
     k_lp_agg_bwd(SellView s, int n, const float *__restrict__ aval,
                  const float *__restrict__ dm, float *__restrict__ dh_prev) {
@@ -738,6 +741,8 @@ __global__ void __launch_bounds__(kTPB, 4)
     const long long base = __ldg(&s.ptr[slice]) + ln;
     const int w = __ldg(&s.width[slice]), op = __ldg(&s.offp[slice]);
     const bool uni = __ldg(&s.kind[slice]) == 0;
+    float4 *o = reinterpret_cast<float4 *>(dh_prev + r * C + q);
+    float4 v = *o;  // with the first loads, not after the sums
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
     for (int j0 = 0; j0 < w; j0 += 8) {
       float a[8];
@@ -746,11 +751,11 @@ __global__ void __launch_bounds__(kTPB, 4)
       for (int j = 0; j < 8; ++j) {
         a[j] = 0.f;
         if (j0 + j < w) {
-          long long col = uni ? r + __ldg(&s.off[op + j0 + j])
-                              : __ldg(&s.off[op + 32 * (j0 + j) + ln]);
+          int col = uni ? (int)r + __ldg(&s.off[op + j0 + j])
+                        : __ldg(&s.off[op + 32 * (j0 + j) + ln]);
           col = col < 0 ? 0 : (col >= n ? n - 1 : col);
           a[j] = __ldg(&aval[base + (long long)(j0 + j) * 32]);
-          x[j] = __ldg(reinterpret_cast<const float4 *>(dm + col * C + q));
+          x[j] = __ldg(reinterpret_cast<const float4 *>(dm + (long long)col * C + q));
         }
       }
 #pragma unroll
@@ -762,8 +767,6 @@ __global__ void __launch_bounds__(kTPB, 4)
           acc.w += a[j] * x[j].w;
         }
     }
-    float4 *o = reinterpret_cast<float4 *>(dh_prev + r * C + q);
-    float4 v = *o;
     v.x += acc.x;
     v.y += acc.y;
     v.z += acc.z;
@@ -809,12 +812,16 @@ __global__ void __launch_bounds__(kTPB)
   }
 }
 
-// grad[t] = sum over blocks of part[b][t] in FP64: a block takes 32 values, its warps every
-// eighth partial each, and their sums are added in warp order.  One thread adding all of a
-// value's partials, one dependent FP64 sum each, took 62 us for 304.
+// grad[t] = sum over blocks of part[b][t] in FP64, for blockIdx.y of several such sums one
+// after the other: a block takes 32 values, its warps every eighth partial each, and their
+// sums are added in warp order.  One thread adding all of a value's partials, one dependent
+// FP64 sum each, took 62 us for 304; a launch a layer 17 us for 456, bound by the latency of
+// its few blocks, so the six layers' sums are one launch (training step at 64^3: 1.57 -> 1.50 ms).
 __global__ void __launch_bounds__(kTPB)
     k_lp_sum_parts(const float *__restrict__ part, int nblocks, int width,
                    float *__restrict__ grad) {
+  part += (long long)blockIdx.y * nblocks * width;
+  grad += (long long)blockIdx.y * width;
   __shared__ double sums[kTPB / 32][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, t = blockIdx.x * 32 + lane;
   double sacc = 0.0;
@@ -1269,6 +1276,7 @@ int ensure_workspace(fcg_learned *Lp, fcg_context *c, bool train) {
     LP_TRY(Lp, Lp->dh2.ensure(sizeof(float) * nc));
     LP_TRY(Lp, Lp->dm.ensure(sizeof(float) * nc));
     LP_TRY(Lp, Lp->dvec.ensure(sizeof(float) * 6 * Lp->ncap));
+    LP_TRY(Lp, Lp->part.ensure(sizeof(float) * (size_t)Lp->num_sms * 3 * lp::kLayerParams * lp::L));
     Lp->train_cap = true;
   }
   return FCG_OK;
@@ -1539,20 +1547,20 @@ int loss_grad(fcg_learned *Lp, fcg_context *c, const float *r, const float *e) {
   const __nv_bfloat16 *H = Lp->hbuf.as<__nv_bfloat16>();
   float *dh = Lp->dh.as<float>(), *dh2 = Lp->dh2.as<float>();
   k_lp_out_bwd<<<GS, kTPB, 0, st>>>(n, gy, sums, H + (size_t)lp::L * hs, prm, dh, part);
-  auto sum_parts = [&](int blocks, int width, float *out) {
-    k_lp_sum_parts<<<(width + 31) / 32, kTPB, 0, st>>>(part, blocks, width, out);
+  auto sum_parts = [&](int blocks, int width, float *out, int sums = 1) {
+    k_lp_sum_parts<<<dim3((width + 31) / 32, sums), kTPB, 0, st>>>(part, blocks, width, out);
   };
   sum_parts(GS, lp::C + 1, grad + lp::oWout);
   for (int l = lp::L - 1; l >= 0; --l) {
     k_lp_layer_bwd<<<GB, kTPB, 0, st>>>(n, dh, Lp->zbuf.as<float>() + (l + 1) * hs, H + l * hs,
                                         Lp->mbuf.as<float>() + l * hs,
                                         prm + lp::oLayer0 + l * lp::kLayerParams, dh2,
-                                        Lp->dm.as<float>(), part);
-    sum_parts(GB, lp::kLayerParams, grad + lp::oLayer0 + l * lp::kLayerParams);
+                                        Lp->dm.as<float>(), part + (size_t)l * GB * lp::kLayerParams);
     k_lp_agg_bwd<<<grid_for((long long)n * 8, c->num_sms), kTPB, 0, st>>>(
         c->sv, n, scaled32(c), Lp->dm.as<float>(), dh2);
     std::swap(dh, dh2);
   }
+  sum_parts(GB, lp::kLayerParams, grad + lp::oLayer0, lp::L);
   k_lp_embed_bwd<<<GS, kTPB, 0, st>>>(n, dh, Lp->zbuf.as<float>(), Lp->feat.as<float>(), part);
   sum_parts(GS, lp::C * lp::F + lp::C, grad + lp::oWin);
   LP_TRY(Lp, cudaGetLastError());
@@ -1612,7 +1620,6 @@ extern "C" int fcg_lp_create(int device, unsigned long long seed, fcg_learned **
   const size_t pb = sizeof(float) * lp::P;
   if (Lp->params.ensure(pb) || Lp->adam_m.ensure(pb) || Lp->adam_v.ensure(pb) ||
       Lp->grad.ensure(pb) || Lp->wbf.ensure(sizeof(__nv_bfloat16) * lp::L * 2 * lp::C * lp::C) ||
-      Lp->part.ensure(sizeof(float) * (size_t)Lp->num_sms * 3 * lp::kLayerParams) ||
       Lp->red.ensure(sizeof(double) * (lp::kMaxDir * kMaxBlocks + 8)) ||
       Lp->scal.ensure(sizeof(float) * 64) || cudaMalloc(&Lp->S, sizeof(lp::LScal)) ||
       cudaMallocHost(&Lp->hS, sizeof(lp::LScal)) ||
