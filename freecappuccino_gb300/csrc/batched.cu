@@ -712,7 +712,7 @@ extern "C" int fcg_batch_autotune(fcg_batch *b, const double *const *a, const do
   B_TRY(b, cudaSetDevice(b->device));
   const int ns = (int)b->ctx.size();
   std::vector<DBuf> zeros(ns);
-  const int cand_items[] = {4, 8, 16, 32, 64, 128};
+  const int cand_items[] = {4, 8, 16, 32, 64, 128}, cand_bps[] = {1, 2, 4, kResident};
   int best_spi = b->slices_per_item, best_bps = b->blocks_per_sm;
   float best = 1e30f;
   int rc = FCG_OK;
@@ -724,7 +724,8 @@ extern "C" int fcg_batch_autotune(fcg_batch *b, const double *const *a, const do
   }
   bool loaded = false;
   for (int spi : cand_items) {
-    for (int bps = 1; bps <= std::min(b->occ, 4) && !rc; bps *= 2) {
+    for (int bps : cand_bps) {
+      if (rc || bps > b->occ) continue;
       if ((rc = fcg_batch_set_params(b, spi, bps))) break;
       float t = 0.f;
       for (int rep = 0; rep < 2 && !rc; ++rep) {  // first run warms up
