@@ -239,15 +239,16 @@ def learned_launches(stats, ml=None):
     coarsest): per solve one Galerkin launch per coarse level, the dense inverse and, for
     the smoothed first level, the P, transposed-P and A P kernels; per
     iteration the fine residual, restriction and prolongation, per inner level the
-    pre-sweeps, residual, restriction, prolongation and post-sweeps, the coarsest solve,
-    and the dot products the network's output kernel no longer does."""
+    pre-sweeps after the first (the restriction's), residual, restriction, prolongation
+    and post-sweeps, the coarsest solve, and the dot products the network's output kernel
+    no longer does."""
     base = 4 + 1 + 14 * stats["iters"] + 2 * stats["updates"] + 1
     if not ml or len(ml["cells"]) < 2:
         return base
     L, nu = len(ml["cells"]), ml["sweeps"]
     coarse = L - 1
-    last = 1 if ml["dense"] else 2 * nu + 2
-    per_it = 3 + (2 * nu + 3) * (coarse - 1) + last + 1
+    last = 1 if ml["dense"] else 2 * nu + 1
+    per_it = 3 + (2 * nu + 2) * (coarse - 1) + last + 1
     setup = coarse + (1 if ml["dense"] else 0) + (3 if ml["options"]["smoothed"] else 0)
     return base + setup + per_it * stats["iters"]
 
@@ -725,10 +726,17 @@ def main():
     last = reports[-1]
     iters = last.iters
     if method != "learned":
-        ctx_levels = 3 * N - 2  # levels of each triangular sweep on the N^3 hex mesh
-        per_solve = {"dpcg": lambda it: 3 + 3 * it, "dpcg_mixed": lambda it: 6 + 5 * it,
-                     "iccg": lambda it: 3 + (2 * ctx_levels + 4) * it,
-                     "bicgstab": lambda it: 3 + (4 * ctx_levels + 6) * it}
+        # matrix fill, first and last residual; five more for the factor and the records of
+        # the one-launch sweeps (at most kSlab = 512 planes each).  A DPCG whose rows the
+        # resident threads hold is one launch after two.  The mixed solver's residual
+        # replacements (two each) are not counted.
+        sms = torch.cuda.get_device_properties(local).multi_processor_count
+        resident = (N ** 3 + 31) // 32 <= 4 * 16 * min(sms, 160)
+        slabs = (N + 511) // 512
+        per_solve = {"dpcg": lambda it: 5 if resident else 3 + 3 * it,
+                     "dpcg_mixed": lambda it: 11 + 3 * it,
+                     "iccg": lambda it: 7 + slabs + (4 + 2 * slabs) * it,
+                     "bicgstab": lambda it: 7 + slabs + (6 + 4 * slabs) * it}
         launches = sum(per_solve.get(method, lambda it: 3 + 3 * it)(r.iters) for r in reports)
     x_method = last.fi.clone()
     peak, peak_kind = peaks()
