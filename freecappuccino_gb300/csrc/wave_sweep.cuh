@@ -171,10 +171,10 @@ constexpr int kForward = 0, kBackward = 1, kFactor = 2;
 // for DILU), forward y = (b - L y) d from `in`
 // (natural order, system s at s n), or backward z = y rescale - (U z) d into `out`
 // (natural order), rescale = d / (d + small).
-// Measured (GB300, FP64, us forward / backward): 128^3 156 / 155 against 356 / 380 with the
+// Measured (GB300, FP64, us forward / backward): 128^3 143 / 153 against 356 / 380 with the
 // coefficients read in natural order through address arithmetic and validity tests, the
 // scaling on the chain and every hand-over through global memory; 40 ICCG sweeps at 128^3
-// 34.7 -> 18.0 ms, at 256^3 125 -> 68 ms.  One tile alone takes 0.28 us a step (FP32 0.16).
+// 34.7 -> 16.0 ms, at 256^3 125 -> 60 ms.  One tile alone takes 0.28 us a step (FP32 0.16).
 // kD = 4 or 12 measured 189 and 170 us forward at 128^3 and 1217 and 475 us at 256^3
 // (kD = 8: 156 and 473); clusters of 1 x 8, 4 x 2 or 4 x 4 tiles are within 3% of 2 x 4.
 template <class T, int MODE>
@@ -374,14 +374,18 @@ __global__ void __launch_bounds__(kThreads) __cluster_dims__(CX *CY, 1, 1)
           val = W::sub(val, c1, vq);
           val = W::sub(val, c2, prev);
         }
+        // What the next step waits for comes before the barrier, stores to global memory after
+        // it.  The loads: after the barrier in the forward sweep (153 -> 143 us at 128^3),
+        // before it in the backward one, where after it costs 5 %.
         const Cell &next = ring[(u + 1) % kD];
-        load(u + kD, ring[u]);
+        if (BWD) load(u + kD, ring[u]);
         part = FACTOR ? next.c[3] : next.x * next.c[3];
         sm[(u + 1) % kD][dj][di] = val;
         if (act) prev = val;
         if (!BWD) part = W::sub(part, next.c[0], prev);
         if (act && near_p) W::push(push_p + step * u * (int)sizeof(T), val);
         if (act && near_q) W::push(push_q + step * u * (int)sizeof(T), val);
+        asm volatile("bar.sync 1, %0;" ::"n"(NT) : "memory");
         if (BWD) {
           if (act && col_ok) xout[(long long)nxy * kk] = val;
           if (act && far_out) W::st(zw + step * u * NT, val);
@@ -389,8 +393,8 @@ __global__ void __launch_bounds__(kThreads) __cluster_dims__(CX *CY, 1, 1)
         } else {
           if (act) W::st(yw + step * u * NT, val);
           if (act && rearm_z) zw[step * u * NT] = W::sentinel();
+          load(u + kD, ring[u]);
         }
-        asm volatile("bar.sync 1, %0;" ::"n"(NT) : "memory");
       }
       k += step * kD;
       rec += step * kD * (P * NT);
