@@ -29,7 +29,7 @@ namespace ml {
 namespace {
 
 constexpr int kDenseThreads = 1024;
-constexpr int kDenseMaxRows = 160;  // 2 n^2 floats fit the shared memory of a block
+constexpr int kDenseMaxRows = 160;  // 25 elements a thread of the block that inverts
 
 __device__ __forceinline__ bool stopped(const int *done) { return done && __ldcg(done); }
 
@@ -157,56 +157,87 @@ __global__ void __launch_bounds__(kTPB)
 }
 
 // Gauss-Jordan inverse of the (small, symmetric positive definite) coarsest matrix in
-// FP32, one block, the matrix and its inverse in shared memory (2 n^2 floats).  M
-// receives the inverse, row-major.  A pivot below 1e-5 of the largest diagonal entry
-// drops its row (a zero row and column of M), which keeps a singular coarsest matrix (no
-// Dirichlet boundary) from producing infinities.
+// FP32, one block.  M receives the inverse, row-major.  A pivot below 1e-5 of the largest
+// diagonal entry drops its row (a zero row and column of M), which keeps a singular coarsest
+// matrix (no Dirichlet boundary) from producing infinities.
+//
+// In place: after step p the columns up to p hold the inverse's, the others the matrix's.
+// Thread (w, l) of warp w keeps the elements (w + 32 i, l + 32 j) in registers, so row p lies
+// in one warp and column p in one lane of every warp; a step exchanges those two through
+// shared memory (two buffers in turn) and has one barrier.  Bound by the latency of its n
+// steps: 120 rows 60 us; with the matrix and its inverse in shared memory and four
+// barriers a step 360.
+constexpr int kDenseTile = (kDenseMaxRows + 31) / 32;
+static_assert(kDenseThreads == 1024, "32 x 32 threads");
+
 __global__ void __launch_bounds__(kDenseThreads)
     k_ml_dense_inv(int n, const int *__restrict__ ptr, const int *__restrict__ col,
                    const float *__restrict__ a, float *__restrict__ M) {
-  extern __shared__ float dsm[];
-  float *W = dsm, *V = dsm + n * n;
-  __shared__ float fcol[kDenseMaxRows];
-  __shared__ float pinv, tiny;
-  const int tid = threadIdx.x, bs = blockDim.x;
-  const int nn = n * n;
-  for (int i = tid; i < nn; i += bs) {
-    W[i] = 0.f;
-    V[i] = (i / n == i % n) ? 1.f : 0.f;
-  }
+  extern __shared__ float dsm[];  // n^2
+  __shared__ float rowp[2][32 * kDenseTile], colp[2][32 * kDenseTile], diag[32];
+  const int tid = threadIdx.x, w = tid >> 5, l = tid & 31;
+  for (int i = tid; i < n * n; i += kDenseThreads) dsm[i] = 0.f;
   __syncthreads();
-  for (int r = tid; r < n; r += bs)
-    for (int k = ptr[r]; k < ptr[r + 1]; ++k) W[r * n + col[k]] = a[k];
-  __syncthreads();
-  if (tid == 0) {
-    float dmax = 0.f;
-    for (int r = 0; r < n; ++r) dmax = fmaxf(dmax, W[r * n + r]);
-    tiny = 1e-5f * dmax;
-  }
-  __syncthreads();
-  for (int p = 0; p < n; ++p) {
-    if (tid == 0) {
-      const float piv = W[p * n + p];
-      pinv = piv > tiny ? 1.f / piv : 0.f;
+  float dmax = 0.f;
+  for (int r = w; r < n; r += 32)
+    for (int k = ptr[r] + l; k < ptr[r + 1]; k += 32) {
+      dsm[r * n + col[k]] = a[k];
+      if (col[k] == r) dmax = fmaxf(dmax, a[k]);
     }
-    __syncthreads();
-    for (int c = tid; c < n; c += bs) {
-      W[p * n + c] *= pinv;
-      V[p * n + c] *= pinv;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) dmax = fmaxf(dmax, __shfl_xor_sync(0xffffffffu, dmax, o));
+  if (l == 0) diag[w] = dmax;
+  __syncthreads();
+  dmax = diag[l];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) dmax = fmaxf(dmax, __shfl_xor_sync(0xffffffffu, dmax, o));
+  const float tiny = 1e-5f * dmax;
+  float g[kDenseTile][kDenseTile];
+#pragma unroll
+  for (int i = 0; i < kDenseTile; ++i)
+#pragma unroll
+    for (int j = 0; j < kDenseTile; ++j) {
+      const int r = w + 32 * i, c = l + 32 * j;
+      g[i][j] = r < n && c < n ? dsm[r * n + c] : 0.f;
     }
-    for (int r = tid; r < n; r += bs) fcol[r] = (r == p) ? 0.f : W[r * n + p];
-    __syncthreads();
-    for (int i = tid; i < nn; i += bs) {
-      const int r = i / n, c = i - r * n;
-      const float f = fcol[r];
-      if (f != 0.f) {
-        W[i] -= f * W[p * n + c];
-        V[i] -= f * V[p * n + c];
+#pragma unroll
+  for (int pi = 0; pi < kDenseTile; ++pi) {
+    for (int q = 0; q < 32; ++q) {
+      const int p = 32 * pi + q, buf = p & 1;
+      if (p >= n) break;
+      if (w == q) {  // row p, scaled; its own column becomes the inverse's
+        const float piv = __shfl_sync(0xffffffffu, g[pi][pi], q);
+        const float pinv = piv > tiny ? 1.f / piv : 0.f;
+#pragma unroll
+        for (int j = 0; j < kDenseTile; ++j) {
+          g[pi][j] = j == pi && l == q ? pinv : g[pi][j] * pinv;
+          rowp[buf][l + 32 * j] = g[pi][j];
+        }
+      }
+      if (l == q)
+#pragma unroll
+        for (int i = 0; i < kDenseTile; ++i) colp[buf][w + 32 * i] = g[i][pi];
+      __syncthreads();
+      float rv[kDenseTile];
+#pragma unroll
+      for (int j = 0; j < kDenseTile; ++j) rv[j] = rowp[buf][l + 32 * j];
+#pragma unroll
+      for (int i = 0; i < kDenseTile; ++i) {
+        const float f = colp[buf][w + 32 * i];
+        if ((i == pi && w == q) || f == 0.f) continue;  // row p itself; nothing to eliminate
+#pragma unroll
+        for (int j = 0; j < kDenseTile; ++j)
+          g[i][j] = __fmaf_rn(-f, rv[j], j == pi && l == q ? 0.f : g[i][j]);
       }
     }
-    __syncthreads();
   }
-  for (int i = tid; i < nn; i += bs) M[i] = V[i];
+#pragma unroll
+  for (int i = 0; i < kDenseTile; ++i)
+#pragma unroll
+    for (int j = 0; j < kDenseTile; ++j) {
+      const int r = w + 32 * i, c = l + 32 * j;
+      if (r < n && c < n) M[r * n + c] = g[i][j];
+    }
 }
 
 // x = M b, one warp per row
@@ -942,7 +973,7 @@ int values(Hierarchy &H, fcg_context *c, cudaStream_t st) {
   }
   if (H.has_dense) {
     const DevLevel &L = H.lv.back();
-    const size_t smem = sizeof(float) * 2 * L.n * L.n;
+    const size_t smem = sizeof(float) * L.n * L.n;
     if (smem > 48 * 1024 &&
         cudaFuncSetAttribute(k_ml_dense_inv, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)smem) != cudaSuccess)
