@@ -64,3 +64,33 @@ def test_resident_dpcg_stops_and_fails_as_the_loop():
             run(lambda: c.dpcg(a, bad, zero, 1e-6, 10))
     assert c.dpcg(a, su, zero, 1e-6, 500).iters == r.iters  # the state is usable afterwards
     c.close()
+
+
+def test_resident_dpcg_of_two_threads():
+    """Two contexts, each in its own thread and stream, solve at the same time: the launches
+    are cooperative, so the blocks of one never wait for blocks that cannot run."""
+    import threading
+
+    ctx, sys_, ref = [], [], []
+    for ext in ((24, 24, 24), (43, 43, 43)):
+        m = box_mesh(*ext)
+        c = fcg.Context(m)
+        a, su = c.laplacian(*poisson_system(m))
+        ctx.append(c)
+        sys_.append((a, su, np.zeros(m.numCells)))
+        ref.append(c.dpcg(*sys_[-1], 1e-30, 25).fi)
+    bad = []
+
+    def run(k):
+        for _ in range(20):
+            if not np.array_equal(ctx[k].dpcg(*sys_[k], 1e-30, 25).fi, ref[k]):
+                bad.append(k)
+
+    threads = [threading.Thread(target=run, args=(k,)) for k in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
+    for c in ctx:
+        c.close()
