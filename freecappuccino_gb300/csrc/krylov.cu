@@ -22,10 +22,14 @@
 //    reference's order: the reference's M = (D+L) D^-1 (D+U).
 // Deviations kept on purpose (FP64 division is slow on this part and every FP64
 // operation of a sweep lengthens its chain of dependent rows): DPCG's z = r / a(diag) is
-// computed as r * (1/a(diag)); a sweep's row (b - sum a_k z_k) d as b d - sum (a_k d) z_k
-// with fused multiply-adds; the rescale zk/(d+small) between the sweeps (iccg.f90:102)
-// as a product with d/(d+small), formed once per solve with the factor.  Each rounds an
-// entry by at most an ulp differently.
+// computed as r * (1/a(diag)); an ICCG sweep's row (b - sum a_k z_k) d as
+// b d - sum (a_k d) z_k with fused multiply-adds; the rescale zk/(d+small) between the
+// sweeps (iccg.f90:102) as a product with d/(d+small), formed once per solve with the
+// factor.  Each rounds an entry by at most an ulp differently.  BiCGStab keeps the
+// reference's operations, but for the rescale as a product with 1/(d+small), and the order
+// of its sums: on a pressure system its iterates magnify an ulp of the right-hand side to
+// 1e-9 .. 1e-4 of the solution in 20 to 60 sweeps, so that another rounding is another
+// answer.
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
@@ -227,7 +231,7 @@ __global__ void __launch_bounds__(kTPB, 8) k_init(SellView s, int n, const doubl
       if (kind == SK_DPCG) v[1] += rr * (rr * invd[r]);
     }
   }
-  if (reduce_commit<2>(v, partials, &S->ticket[0]) && threadIdx.x == 0) {
+  if (reduce_commit_tree<2>(v, partials, &S->ticket[0]) && threadIdx.x == 0) {
     S->res0 = v[0];
     S->resl = v[0];
     S->iter = 0;
@@ -364,15 +368,16 @@ __global__ void k_fwd_level(const int *__restrict__ rows, int count,
                             const int *__restrict__ ioffset, const int *__restrict__ ja,
                             const int *__restrict__ diag, const double *__restrict__ a,
                             const double *__restrict__ d, const double *__restrict__ b,
-                            double *__restrict__ z, const Scal *S) {
+                            double *__restrict__ z, const Scal *S, bool plain) {
   if (solve_done(S)) return;
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= count) return;
   int i = rows[t];
   const double di = d[i];
-  double zi = b[i] * di;
-  for (int k = ioffset[i]; k < diag[i]; ++k) zi = __fma_rn(-(a[k] * di), z[ja[k]], zi);
-  z[i] = zi;
+  double zi = plain ? b[i] : b[i] * di;
+  for (int k = ioffset[i]; k < diag[i]; ++k)
+    zi = plain ? __dsub_rn(zi, __dmul_rn(a[k], z[ja[k]])) : __fma_rn(-(a[k] * di), z[ja[k]], zi);
+  z[i] = plain ? zi * di : zi;
 }
 
 // backward with the reference's rescale zk/(d+small) folded in (iccg.f90:256-265), as a
@@ -381,15 +386,16 @@ __global__ void k_bwd_level(const int *__restrict__ rows, int count,
                             const int *__restrict__ ioffset, const int *__restrict__ ja,
                             const int *__restrict__ diag, const double *__restrict__ a,
                             const double *__restrict__ d, const double *__restrict__ rdi,
-                            double *__restrict__ z, const Scal *S) {
+                            double *__restrict__ z, const Scal *S, bool plain) {
   if (solve_done(S)) return;
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= count) return;
   int i = rows[t];
   double di = d[i];
   double zi = z[i] * rdi[i];
-  for (int k = diag[i] + 1; k < ioffset[i + 1]; ++k) zi = __fma_rn(-(a[k] * di), z[ja[k]], zi);
-  z[i] = zi;
+  for (int k = diag[i] + 1; k < ioffset[i + 1]; ++k)
+    zi = plain ? __dsub_rn(zi, __dmul_rn(a[k], z[ja[k]])) : __fma_rn(-(a[k] * di), z[ja[k]], zi);
+  z[i] = plain ? zi * di : zi;
 }
 
 // Factor diagonals, level by level: DIC d_i = 1/(a_ii - sum a_ik^2 d_k) (iccg.f90:
@@ -405,22 +411,25 @@ __global__ void k_factor_level(const int *__restrict__ rows, int count,
   int i = rows[t];
   double di = a[diag[i]];
   for (int k = ioffset[i]; k < diag[i]; ++k) {
-    di = __fma_rn(-(a[k] * (dilu ? a[tpos[k]] : a[k])), d[ja[k]], di);
+    if (dilu)  // BiCGStab: every operation rounded (k_wave_sweep's PLAIN)
+      di = __dsub_rn(di, __dmul_rn(__dmul_rn(a[k], d[ja[k]]), a[tpos[k]]));
+    else
+      di = __fma_rn(-(a[k] * a[k]), d[ja[k]], di);
   }
   double inv = 1.0 / di;
   d[i] = inv;
-  rdi[i] = inv / (inv + S->small);
+  rdi[i] = (dilu ? 1.0 : inv) / (inv + S->small);
   if (!isfinite(inv) || di == 0.0) fail_status(S, FCG_ERR_PIVOT);
 }
 
 // --- BiCGStab sweep (bicgstab.f90:99-224) -------------------------------------
 // bet = sum res*reso; om = bet*gam/(alf*beto+small); beto = bet
-__global__ void __launch_bounds__(kTPB, 5) k_bi_dot1(int n, const double *__restrict__ res, const double *__restrict__ reso,
+__global__ void __launch_bounds__(kTPB, 8) k_bi_dot1(int n, const double *__restrict__ res, const double *__restrict__ reso,
                           Scal *S, double *partials) {
   if (solve_done(S)) return;
   double v[1] = {0.0};
   FCG_GRID_STRIDE(i, n) v[0] += res[i] * reso[i];
-  if (reduce_commit<1>(v, partials, &S->ticket[3]) && threadIdx.x == 0) {
+  if (reduce_commit_tree<1>(v, partials, &S->ticket[3]) && threadIdx.x == 0) {
     double bet = v[0];
     S->bbet = bet;
     S->om = bet * S->gam / (S->alf * S->beto + S->small);
@@ -450,7 +459,7 @@ __global__ void __launch_bounds__(kTPB, 8) k_bi_spmv1(SellView s, int n, const d
       v[0] += u * reso[r];
     }
   }
-  if (reduce_commit<1>(v, partials, &S->ticket[4]) && threadIdx.x == 0) {
+  if (reduce_commit_tree<1>(v, partials, &S->ticket[4]) && threadIdx.x == 0) {
     S->gam = S->bbet / v[0];
     if (!isfinite(S->gam)) fail_status(S, FCG_ERR_NONFINITE);
   }
@@ -483,7 +492,7 @@ __global__ void __launch_bounds__(kTPB, 8) k_bi_spmv2(SellView s, int n, const d
       v[1] += q * q;
     }
   }
-  if (reduce_commit<2>(v, partials, &S->ticket[5]) && threadIdx.x == 0) {
+  if (reduce_commit_tree<2>(v, partials, &S->ticket[5]) && threadIdx.x == 0) {
     S->alf = v[0] / (v[1] + S->small);
     if (!isfinite(S->alf)) fail_status(S, FCG_ERR_NONFINITE);
   }
@@ -500,7 +509,7 @@ __device__ __noinline__ void bi_close_sweep(Scal *S, double resl, double *trace,
 }
 
 // fi += alf*zk; res -= alf*vk; resl = sum|res|; stop test
-__global__ void __launch_bounds__(kTPB, 5) k_bi_upd2(int n, double *__restrict__ x, double *__restrict__ res,
+__global__ void __launch_bounds__(kTPB, 8) k_bi_upd2(int n, double *__restrict__ x, double *__restrict__ res,
                           const double *__restrict__ zk, const double *__restrict__ vk, Scal *S,
                           double *partials, double *trace, cudaGraphConditionalHandle h,
                           int use_cond) {
@@ -517,7 +526,7 @@ __global__ void __launch_bounds__(kTPB, 5) k_bi_upd2(int n, double *__restrict__
     res[i] = r;
     v[0] += fabs(r);
   }
-  if (reduce_commit<1>(v, partials, &S->ticket[6]) && threadIdx.x == 0)
+  if (reduce_commit_tree<1>(v, partials, &S->ticket[6]) && threadIdx.x == 0)
     bi_close_sweep(S, v[0], trace, h, use_cond);
 }
 
@@ -968,23 +977,28 @@ static int start_sweeps(fcg_context *c, bool dilu) {
   int rc;
   if (!wave_sweeps(c)) {
     if (!k->lv.y && (rc = level::allocate(c, 1, k->lbuf, k->lv))) return rc;
-    return level::start(c, 1, c->nnz, k->a, dilu, k->small, k->lv, wave_control(k));
+    return dilu ? level::start<double, true>(c, 1, c->nnz, k->a, true, k->small, k->lv,
+                                             wave_control(k))
+                : level::start<double>(c, 1, c->nnz, k->a, false, k->small, k->lv,
+                                       wave_control(k));
   }
   if (!k->wv.fwd && (rc = wave::allocate(c, 1, k->wbuf, k->wv))) return rc;
-  return wave::start(c, 1, c->nnz, k->a, dilu, k->small, k->wv, wave_control(k));
+  return dilu ? wave::start<double, true>(c, 1, c->nnz, k->a, true, k->small, k->wv, wave_control(k))
+              : wave::start<double>(c, 1, c->nnz, k->a, false, k->small, k->wv, wave_control(k));
 }
 
+template <bool PLAIN>
 static void launch_sweeps(fcg_context *c, cudaStream_t st, const Level &lv, bool forward,
                           const double *b, double *z) {
   KrylovState *k = c->ks;
   if (k->sf_on) {
     if (wave_sweeps(c)) {
-      wave::launch<double>(c, st, 1, forward ? wave::kForward : wave::kBackward, k->wv, b, z,
-                           wave_control(k));
+      wave::launch<double, PLAIN>(c, st, 1, forward ? wave::kForward : wave::kBackward, k->wv, b,
+                                  z, wave_control(k));
       return;
     }
-    level::launch<double>(c, st, 1, forward ? wave::kForward : wave::kBackward, k->lv, b, z,
-                          wave_control(k), k->sf_absent_row);
+    level::launch<double, PLAIN>(c, st, 1, forward ? wave::kForward : wave::kBackward, k->lv, b,
+                                 z, wave_control(k), k->sf_absent_row);
     return;
   }
   for (int l = 0; l < lv.count; ++l) {
@@ -992,10 +1006,10 @@ static void launch_sweeps(fcg_context *c, cudaStream_t st, const Level &lv, bool
     int g = (cnt + kTPB - 1) / kTPB;
     if (forward)
       k_fwd_level<<<g, kTPB, 0, st>>>(lv.rows + start, cnt, c->mv.ioffset, c->mv.ja, c->mv.diag,
-                                      k->a, k->d, b, z, k->S);
+                                      k->a, k->d, b, z, k->S, PLAIN);
     else
       k_bwd_level<<<g, kTPB, 0, st>>>(lv.rows + start, cnt, c->mv.ioffset, c->mv.ja, c->mv.diag,
-                                      k->a, k->d, k->rdi, z, k->S);
+                                      k->a, k->d, k->rdi, z, k->S, PLAIN);
   }
 }
 
@@ -1038,8 +1052,8 @@ static void enqueue_unit(fcg_context *c, cudaStream_t st, int kind, int u,
   if (kind == SK_DPCG || kind == SK_ICCG) {
     int v = kind == SK_DPCG ? u + 3 : u;
     switch (v) {
-      case 0: launch_sweeps(c, st, c->lf, true, k->res, k->zk); break;
-      case 1: launch_sweeps(c, st, c->lb, false, nullptr, k->zk); break;
+      case 0: launch_sweeps<false>(c, st, c->lf, true, k->res, k->zk); break;
+      case 1: launch_sweeps<false>(c, st, c->lb, false, nullptr, k->zk); break;
       case 2: k_cg_dot<<<k->gr.dot, kTPB, 0, st>>>(n, k->res, k->zk, k->S, k->partials); break;
       case 3:
         k_cg_p<<<k->gr.p, kTPB, 0, st>>>(n, k->res, k->invd, k->zk, k->pk, k->S, kind);
@@ -1075,15 +1089,15 @@ static void enqueue_unit(fcg_context *c, cudaStream_t st, int kind, int u,
     switch (u) {
       case 0: k_bi_dot1<<<k->gr.bdot, kTPB, 0, st>>>(n, k->res, k->reso, k->S, k->partials); break;
       case 1: k_bi_p<<<k->gr.bp, kTPB, 0, st>>>(n, k->res, k->uk, k->pk, k->S); break;
-      case 2: launch_sweeps(c, st, c->lf, true, k->pk, k->zk); break;
-      case 3: launch_sweeps(c, st, c->lb, false, nullptr, k->zk); break;
+      case 2: launch_sweeps<true>(c, st, c->lf, true, k->pk, k->zk); break;
+      case 3: launch_sweeps<true>(c, st, c->lb, false, nullptr, k->zk); break;
       case 4:
         k_bi_spmv1<<<k->gr.bspmv1, kTPB, 0, st>>>(s, n, k->sval, k->zk, k->reso, k->uk, k->S,
                                                    k->partials);
         break;
       case 5: k_bi_upd1<<<k->gr.bupd1, kTPB, 0, st>>>(n, k->x, k->res, k->zk, k->uk, k->S); break;
-      case 6: launch_sweeps(c, st, c->lf, true, k->res, k->zk); break;
-      case 7: launch_sweeps(c, st, c->lb, false, nullptr, k->zk); break;
+      case 6: launch_sweeps<true>(c, st, c->lf, true, k->res, k->zk); break;
+      case 7: launch_sweeps<true>(c, st, c->lb, false, nullptr, k->zk); break;
       case 8:
         k_bi_spmv2<<<k->gr.bspmv2, kTPB, 0, st>>>(s, n, k->sval, k->zk, k->res, k->vk, k->S,
                                                    k->partials);

@@ -52,13 +52,36 @@ __device__ __forceinline__ void block_sum(double (&v)[NV], double (*sh)[kTPB]) {
   }
 }
 
+// The same through trees over the lanes of every warp, then over the warps.
+template <int NV>
+__device__ __forceinline__ void block_sum_tree(double (&v)[NV], double (*sh)[kWarps]) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int k = 0; k < NV; ++k) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if (lane == 0)
+#pragma unroll
+    for (int k = 0; k < NV; ++k) sh[k][w] = v[k];
+  __syncthreads();
+  if (w == 0) {
+#pragma unroll
+    for (int k = 0; k < NV; ++k) v[k] = lane < kWarps ? sh[k][lane] : 0.0;
+#pragma unroll
+    for (int o = kWarps / 2; o > 0; o >>= 1)
+#pragma unroll
+      for (int k = 0; k < NV; ++k) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
+  }
+  __syncthreads();
+}
+
 // Stores this block's sums; returns true in the last block to arrive, whose thread 0
 // then holds the grid-wide sums in v (partials added in block-index order).
-template <int NV>
-__device__ __forceinline__ bool reduce_commit(double (&v)[NV], double *partials, unsigned int *ticket) {
-  __shared__ double sh[sum_rows(NV)][kTPB];
+template <int NV, class Sum, class Shared>
+__device__ __forceinline__ bool commit_sums(double (&v)[NV], double *partials,
+                                            unsigned int *ticket, Shared sh, Sum &&sum) {
   __shared__ bool am_last;
-  block_sum<NV>(v, sh);
+  sum(v, sh);
   const int G = gridDim.x;
   if (threadIdx.x == 0) {
 #pragma unroll
@@ -76,13 +99,30 @@ __device__ __forceinline__ bool reduce_commit(double (&v)[NV], double *partials,
   for (int i = threadIdx.x; i < G; i += blockDim.x)
 #pragma unroll
     for (int k = 0; k < NV; ++k) s[k] += __ldcg(&partials[k * G + i]);
-  block_sum<NV>(s, sh);
+  sum(s, sh);
   if (threadIdx.x == 0) {
 #pragma unroll
     for (int k = 0; k < NV; ++k) v[k] = s[k];
     *ticket = 0u;
   }
   return true;
+}
+
+template <int NV>
+__device__ __forceinline__ bool reduce_commit(double (&v)[NV], double *partials, unsigned int *ticket) {
+  __shared__ double sh[sum_rows(NV)][kTPB];
+  return commit_sums<NV>(v, partials, ticket, sh,
+                         [](double (&x)[NV], double (*p)[kTPB]) { block_sum<NV>(x, p); });
+}
+
+// The order that FP64 BiCGStab's sums keep (its iterates on a pressure system magnify an ulp
+// by ten orders of magnitude in 50 sweeps, so another order is another answer).
+template <int NV>
+__device__ __forceinline__ bool reduce_commit_tree(double (&v)[NV], double *partials,
+                                                   unsigned int *ticket) {
+  __shared__ double sh[NV][kWarps];
+  return commit_sums<NV>(v, partials, ticket, sh,
+                         [](double (&x)[NV], double (*p)[kWarps]) { block_sum_tree<NV>(x, p); });
 }
 
 // Row sum of A x for lane `lane` of slice `slice` (one warp per slice).  Uniform

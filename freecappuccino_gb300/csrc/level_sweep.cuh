@@ -52,17 +52,18 @@ struct Arrays {
 template <class T>
 struct Item {
   int p, off, w;
-  T x, s;
+  T x, s, d;  // d: the backward sweep's factor (PLAIN)
   int dep[kW];
-  T v[kW];
+  T v[kW], t[kW];  // t: a_ji of the factor (PLAIN)
 };
 
 // One sweep of ns systems: the factor, y = (b - L y) d from `in` (natural order), or
 // z = y rescale - (U z) d into `out` (natural order); see wave_sweep.cuh.
-template <class T, int MODE>
+// PLAIN as there; its factor takes the CSR values in `in` and their transposes' places.
+template <class T, int MODE, bool PLAIN>
 __global__ void __launch_bounds__(kThreads)
     k_level_sweep(LevelSide lo, LevelSide up, int n, int ns, Arrays<T> A,
-                  const T *__restrict__ in, T *__restrict__ out, int *ctl, int *fail, int *status,
+                  const T *__restrict__ in, const int *__restrict__ tpos, T *__restrict__ out, int *ctl, int *fail, int *status,
                   const int *done, int spin, int absent) {
   using W = Word<T>;
   constexpr bool BWD = MODE == kBackward, FACTOR = MODE == kFactor;
@@ -105,18 +106,21 @@ __global__ void __launch_bounds__(kThreads)
     it.w = m.w;
     it.x = T(0);
     it.s = T(0);
+    it.d = T(0);
 #pragma unroll
     for (int e = 0; e < kW; ++e) {
       it.dep[e] = -1;
-      it.v[e] = T(0);
+      it.v[e] = it.t[e] = T(0);
       if (e < m.w) {
         const long long q = 32LL * (m.off + e) + lane;
         it.dep[e] = sd.dep[q];
         it.v[e] = val[s * elen + q];
+        if (PLAIN && FACTOR && sd.src[q] >= 0) it.t[e] = in[tpos[sd.src[q]]];
       }
     }
     if (m.row >= 0) {
       it.s = dd[s * len + it.p];
+      if (PLAIN && BWD) it.d = A.fd[s * ylen + m.xp];
       if (BWD)
         it.x = A.y[s * ylen + m.xp];
       else if (!FACTOR)
@@ -137,7 +141,7 @@ __global__ void __launch_bounds__(kThreads)
     if (!BWD && c < up.chunks) A.z[s * zlen + 32 * c + lane] = W::sentinel();
     const T *r = res + s * len;
     bool ok = true;
-    T acc = FACTOR ? it.s : it.x * it.s;
+    T acc = FACTOR ? it.s : PLAIN && !BWD ? it.x : it.x * it.s;
     for (int e0 = 0; e0 < it.w; e0 += kW) {
       if (e0 > 0) {  // rows of more than kW entries
 #pragma unroll
@@ -145,6 +149,8 @@ __global__ void __launch_bounds__(kThreads)
           const long long q = 32LL * (it.off + e0 + e) + lane;
           it.dep[e] = e0 + e < it.w ? sd.dep[q] : -1;
           it.v[e] = e0 + e < it.w ? val[s * elen + q] : T(0);
+          if (PLAIN && FACTOR)
+            it.t[e] = e0 + e < it.w && sd.src[q] >= 0 ? in[tpos[sd.src[q]]] : T(0);
         }
       }
       T v[kW];
@@ -163,7 +169,12 @@ __global__ void __launch_bounds__(kThreads)
         }
       }
 #pragma unroll
-      for (int e = 0; e < kW; ++e) acc = W::sub(acc, it.v[e], v[e]);
+      for (int e = 0; e < kW; ++e) {
+        if (PLAIN && FACTOR)
+          acc = W::sub_rounded(acc, it.v[e] * v[e], it.t[e]);
+        else
+          acc = PLAIN ? W::sub_rounded(acc, it.v[e], v[e]) : W::sub(acc, it.v[e], v[e]);
+      }
     }
     if (!ok && atomicExch(&ctl[3], 1) == 0) {
       if (fail) *fail = 1;
@@ -171,6 +182,7 @@ __global__ void __launch_bounds__(kThreads)
     }
     if (m0.row >= 0) {
       if (FACTOR) acc = T(1) / acc;
+      if (PLAIN && !FACTOR) acc = acc * (BWD ? it.d : it.s);
       if (BWD || m0.row != absent || FACTOR) W::st(&res[s * len + it.p], acc);
       if (BWD) {
         out[(long long)s * n + m0.row] = acc;
@@ -184,7 +196,7 @@ __global__ void __launch_bounds__(kThreads)
 }
 
 // The factor's coefficients a_ij^2 (DIC) or a_ij a_ji (DILU) and a_ii from the CSR values.
-template <class T>
+template <class T, bool PLAIN>
 __global__ void k_level_pack_factor(LevelSide lo, int ns, long long nnz,
                                     const int *__restrict__ diag, const int *__restrict__ tpos,
                                     const T *__restrict__ a, int dilu, Arrays<T> A) {
@@ -195,7 +207,7 @@ __global__ void k_level_pack_factor(LevelSide lo, int ns, long long nnz,
       const long long q = 32LL * e + lane;
       const int k = lo.src[q], kt = k >= 0 && dilu ? tpos[k] : k;
       for (int s = 0; s < ns; ++s)
-        A.fval[s * elen + q] = k >= 0 ? a[s * nnz + k] * a[s * nnz + kt] : T(0);
+        A.fval[s * elen + q] = k < 0 ? T(0) : PLAIN ? a[s * nnz + k] : a[s * nnz + k] * a[s * nnz + kt];
     }
     for (int s = 0; s < ns; ++s) A.fd[s * len + p] = row >= 0 ? a[s * nnz + diag[row]] : T(0);
   }
@@ -203,7 +215,7 @@ __global__ void k_level_pack_factor(LevelSide lo, int ns, long long nnz,
 
 // The sweeps' coefficients from the CSR values and the factor, which the factor sweep left
 // in A.y; a pivot that is not finite is recorded.
-template <class T, bool BWD>
+template <class T, bool BWD, bool PLAIN>
 __global__ void k_level_pack(LevelSide sd, long long ylen, int ns, long long nnz,
                              const T *__restrict__ a, T small, Arrays<T> A, int *status,
                              const int *done) {
@@ -216,10 +228,10 @@ __global__ void k_level_pack(LevelSide sd, long long ylen, int ns, long long nnz
       for (int e = sd.ptr[c]; e < sd.ptr[c + 1]; ++e) {
         const long long q = 32LL * e + lane;
         const int k = sd.src[q];
-        (BWD ? A.bval : A.fval)[s * elen + q] = k >= 0 ? a[s * nnz + k] * d : T(0);
+        (BWD ? A.bval : A.fval)[s * elen + q] = k < 0 ? T(0) : PLAIN ? a[s * nnz + k] : a[s * nnz + k] * d;
       }
       if (BWD)
-        A.bd[s * len + p] = row >= 0 ? d / (d + small) : T(0);
+        A.bd[s * len + p] = row >= 0 ? (PLAIN ? T(1) : d) / (d + small) : T(0);
       else
         A.fd[s * len + p] = d;
       if (!BWD && !isfinite(d)) atomicCAS(status, 0, FCG_ERR_PIVOT);
@@ -252,30 +264,30 @@ int allocate(fcg_context *c, int ns, DBuf &buf, Arrays<T> &A) {
   return FCG_OK;
 }
 
-template <class T>
+template <class T, bool PLAIN = false>
 void launch(fcg_context *c, cudaStream_t st, int ns, int mode, const Arrays<T> &A, const T *in,
             T *out, const Control &w, int absent = -1) {
-  auto kernel = mode == kForward    ? k_level_sweep<T, kForward>
-                : mode == kBackward ? k_level_sweep<T, kBackward>
-                                    : k_level_sweep<T, kFactor>;
+  auto kernel = mode == kForward    ? k_level_sweep<T, kForward, PLAIN>
+                : mode == kBackward ? k_level_sweep<T, kBackward, PLAIN>
+                                    : k_level_sweep<T, kFactor, PLAIN>;
   kernel<<<c->num_sms * kBlocksPerSM, kThreads, 0, st>>>(c->order.lo, c->order.up, c->n, ns, A, in,
-                                                         out, w.ctl, w.fail, w.status, w.done,
+                                                         c->tpos, out, w.ctl, w.fail, w.status, w.done,
                                                          w.spin, absent);
 }
 
 // The factor, the coefficients and armed results: before the first sweep of a solve.
-template <class T>
+template <class T, bool PLAIN = false>
 int start(fcg_context *c, int ns, long long nnz, const T *a, bool dilu, T small,
           const Arrays<T> &A, const Control &w) {
   const LevelSide &lo = c->order.lo, &up = c->order.up;
   const long long lf = 32LL * lo.chunks, lb = 32LL * up.chunks;
   const int gf = grid_for(lf, c->num_sms), gb = grid_for(lb, c->num_sms);
   const int ga = grid_for(ns * std::max(lf, lb), c->num_sms);
-  k_level_pack_factor<T><<<gf, kTPB, 0, c->stream>>>(lo, ns, nnz, c->mv.diag, c->tpos, a, dilu, A);
+  k_level_pack_factor<T, PLAIN><<<gf, kTPB, 0, c->stream>>>(lo, ns, nnz, c->mv.diag, c->tpos, a, dilu, A);
   k_level_arm<T><<<ga, kTPB, 0, c->stream>>>(ns * lf, A.y, ns * lb, A.z, w.ctl);
-  launch<T>(c, c->stream, ns, kFactor, A, nullptr, nullptr, w);
-  k_level_pack<T, false><<<gf, kTPB, 0, c->stream>>>(lo, lf, ns, nnz, a, small, A, w.status, w.done);
-  k_level_pack<T, true><<<gb, kTPB, 0, c->stream>>>(up, lf, ns, nnz, a, small, A, w.status, w.done);
+  launch<T, PLAIN>(c, c->stream, ns, kFactor, A, PLAIN ? a : nullptr, nullptr, w);
+  k_level_pack<T, false, PLAIN><<<gf, kTPB, 0, c->stream>>>(lo, lf, ns, nnz, a, small, A, w.status, w.done);
+  k_level_pack<T, true, PLAIN><<<gb, kTPB, 0, c->stream>>>(up, lf, ns, nnz, a, small, A, w.status, w.done);
   k_level_arm<T><<<ga, kTPB, 0, c->stream>>>(ns * lf, A.y, ns * lb, A.z, w.ctl);
   FCG_CHECK_LAUNCH(c, "level-order factor and coefficients");
   return FCG_OK;

@@ -91,6 +91,10 @@ struct Word<double> {
   static __device__ __forceinline__ double sub(double acc, double a, double v) {
     return __fma_rn(-a, v, acc);
   }
+  // ... and rounded
+  static __device__ __forceinline__ double sub_rounded(double acc, double a, double v) {
+    return __dsub_rn(acc, __dmul_rn(a, v));
+  }
 };
 template <>
 struct Word<float> {
@@ -119,6 +123,9 @@ struct Word<float> {
   static __device__ __forceinline__ float sentinel() { return __uint_as_float(kSent); }
   static __device__ __forceinline__ float sub(float acc, float a, float v) {
     return __fmaf_rn(-a, v, acc);
+  }
+  static __device__ __forceinline__ float sub_rounded(float acc, float a, float v) {
+    return __fsub_rn(acc, __fmul_rn(a, v));
   }
 };
 
@@ -177,7 +184,13 @@ constexpr int kForward = 0, kBackward = 1, kFactor = 2;
 // 34.7 -> 16.0 ms, at 256^3 125 -> 60 ms.  One tile alone takes 0.28 us a step (FP32 0.16).
 // kD = 4 or 12 measured 189 and 170 us forward at 128^3 and 1217 and 475 us at 256^3
 // (kD = 8: 156 and 473); clusters of 1 x 8, 4 x 2 or 4 x 4 tiles are within 3% of 2 x 4.
-template <class T, int MODE>
+//
+// PLAIN: every operation of a row rounded on its own, in the reference's form: the factor
+// a_ii - (a_ij y) a_ji (the a_ji in the backward records), y = (b - L y) d and
+// z = (y / (d + small) - U z) d with unscaled coefficients.  For BiCGStab, whose iterates on
+// a pressure system magnify an ulp by ten orders of magnitude in 50 sweeps.  Two operations
+// a neighbour instead of one and the scaling on the chain: 191 / 223 us at 128^3.
+template <class T, int MODE, bool PLAIN>
 __global__ void __launch_bounds__(kThreads) __cluster_dims__(CX *CY, 1, 1)
     k_wave_sweep(int nx, int ny, int nz, int k0, int k1, int ns, Arrays<T> A,
                  const T *__restrict__ in, T *out, int *ctl, int *fail, int *status,
@@ -311,6 +324,16 @@ __global__ void __launch_bounds__(kThreads) __cluster_dims__(CX *CY, 1, 1)
                       (uint32_t)(k * (int)sizeof(T));
     struct Cell {
       T c[P], x;
+      T e[PLAIN ? (FACTOR ? 3 : 1) : 1];  // PLAIN: factor a_ji, backward d
+    };
+    const long long other = FACTOR ? A.bwd - A.fwd : A.fwd - A.bwd;  // to the other record
+    auto sub = [](T acc, T a, T v) {
+      return PLAIN ? W::sub_rounded(acc, a, v) : W::sub(acc, a, v);
+    };
+    // acc less the factor's term of neighbour q
+    auto term = [&](T acc, const Cell &cl, int q, T v) {
+      if constexpr (PLAIN && FACTOR) return W::sub_rounded(acc, cl.c[q] * v, cl.e[q]);
+      return sub(acc, cl.c[q], v);
     };
     Cell ring[kD];
     // The inputs of step u (of this round or, from kD on, the next).  Only loads: an
@@ -318,6 +341,12 @@ __global__ void __launch_bounds__(kThreads) __cluster_dims__(CX *CY, 1, 1)
     auto load = [&](int u, Cell &cl) {
 #pragma unroll
       for (int p = 0; p < P; ++p) cl.c[p] = __ldg(rec + step * u * (P * NT) + p * NT);
+      if constexpr (PLAIN && FACTOR) {
+#pragma unroll
+        for (int p = 0; p < 3; ++p) cl.e[p] = __ldg(rec + other + step * u * (P * NT) + p * NT);
+      } else if constexpr (PLAIN && BWD) {
+        cl.e[0] = __ldg(rec + other + step * u * (P * NT) + 3 * NT);
+      }
       if (BWD) {
         cl.x = yw[step * u * NT];
       } else if (!FACTOR) {
@@ -335,8 +364,12 @@ __global__ void __launch_bounds__(kThreads) __cluster_dims__(CX *CY, 1, 1)
     T prev = T(0);
     if (col_ok && !BWD && k0 > 0) prev = A.y[sys * vl + lay.at(i, j, k0 - 1)];
     if (col_ok && BWD && k1 < nz) prev = xout[(long long)nxy * depth];
-    part = FACTOR ? ring[0].c[3] : ring[0].x * ring[0].c[3];
-    if (!BWD) part = W::sub(part, ring[0].c[0], prev);
+    auto first = [&](const Cell &cl) {  // the input, scaled where the row is
+      if (FACTOR) return cl.c[3];
+      return PLAIN && !BWD ? cl.x : cl.x * cl.c[3];
+    };
+    part = first(ring[0]);
+    if (!BWD) part = term(part, ring[0], 0, prev);
     const int steps = depth + TX + TY - 2;
     for (int s0 = 0; s0 < steps; s0 += kD) {
 #pragma unroll
@@ -366,23 +399,27 @@ __global__ void __launch_bounds__(kThreads) __cluster_dims__(CX *CY, 1, 1)
         }
         T val;
         if (!BWD) {  // lower entries in CSR order: k, j, i
-          val = W::sub(part, c1, vq);
-          val = W::sub(val, c2, vp);
-          if (FACTOR) val = T(1) / val;
+          val = term(part, ring[u], 1, vq);
+          val = term(val, ring[u], 2, vp);
+          if (FACTOR)
+            val = T(1) / val;
+          else if (PLAIN)
+            val = val * ring[u].c[3];
         } else {  // upper entries in CSR order: i, j, k
-          val = W::sub(part, c0, vp);
-          val = W::sub(val, c1, vq);
-          val = W::sub(val, c2, prev);
+          val = sub(part, c0, vp);
+          val = sub(val, c1, vq);
+          val = sub(val, c2, prev);
+          if (PLAIN) val = val * ring[u].e[0];
         }
         // What the next step waits for comes before the barrier, stores to global memory after
         // it.  The loads: after the barrier in the forward sweep (153 -> 143 us at 128^3),
         // before it in the backward one, where after it costs 5 %.
         const Cell &next = ring[(u + 1) % kD];
         if (BWD) load(u + kD, ring[u]);
-        part = FACTOR ? next.c[3] : next.x * next.c[3];
+        part = first(next);
         sm[(u + 1) % kD][dj][di] = val;
         if (act) prev = val;
-        if (!BWD) part = W::sub(part, next.c[0], prev);
+        if (!BWD) part = term(part, next, 0, prev);
         if (act && near_p) W::push(push_p + step * u * (int)sizeof(T), val);
         if (act && near_q) W::push(push_q + step * u * (int)sizeof(T), val);
         asm volatile("bar.sync 1, %0;" ::"n"(NT) : "memory");
@@ -433,7 +470,7 @@ __device__ __forceinline__ void for_cells(const Layout &lay, F &&f) {
 }
 
 // Records of the factor of system blockIdx.y from the CSR values a (system s at s nnz).
-template <class T>
+template <class T, bool PLAIN>
 __global__ void __launch_bounds__(kTPB)
     k_wave_pack_factor(int nx, int ny, int nz, long long nnz, const int *__restrict__ ioffset,
                        const int *__restrict__ diag, const int *__restrict__ tpos,
@@ -441,14 +478,20 @@ __global__ void __launch_bounds__(kTPB)
   const Layout lay(nx, ny, nz);
   const int s = blockIdx.y;
   const T *as = a + s * nnz;
-  T *fwd = A.fwd + s * lay.rec_len();
+  T *fwd = A.fwd + s * lay.rec_len(), *bwd = A.bwd + s * lay.rec_len();
   for_cells(lay, [&](long long r, long long q, int i, int j, int k) {
-    T *f = fwd + q / NT * kPlanes * NT + q % NT;
+    const long long at = q / NT * kPlanes * NT + q % NT;
+    T *f = fwd + at, *b = bwd + at;
     int e = ioffset[r];
     const bool has[3] = {k > 0, j > 0, i > 0};
 #pragma unroll
     for (int p = 0; p < 3; ++p) {
-      f[p * NT] = has[p] ? as[e] * (dilu ? as[tpos[e]] : as[e]) : T(0);
+      if (PLAIN) {
+        f[p * NT] = has[p] ? as[e] : T(0);
+        b[p * NT] = has[p] ? as[dilu ? tpos[e] : e] : T(0);
+      } else {
+        f[p * NT] = has[p] ? as[e] * (dilu ? as[tpos[e]] : as[e]) : T(0);
+      }
       e += has[p];
     }
     f[3 * NT] = as[diag[r]];
@@ -457,7 +500,7 @@ __global__ void __launch_bounds__(kTPB)
 
 // Records of the sweeps of system blockIdx.y from the CSR values a (system s at s nnz) and
 // the factor, which the factor sweep left in A.y; a pivot that is not finite is recorded.
-template <class T>
+template <class T, bool PLAIN>
 __global__ void __launch_bounds__(kTPB)
     k_wave_pack(int nx, int ny, int nz, long long nnz, const int *__restrict__ ioffset,
                 const int *__restrict__ diag, const T *__restrict__ a, T small, Arrays<T> A,
@@ -474,14 +517,18 @@ __global__ void __launch_bounds__(kTPB)
     const bool u0 = i < nx - 1, u1 = j < ny - 1, u2 = k < nz - 1;
     T *f = fwd + at, *b = bwd + at;
     const T dd = y[q];
-    f[0] = l0 ? as[lo] * dd : T(0);
-    f[NT] = l1 ? as[lo + l0] * dd : T(0);
-    f[2 * NT] = l2 ? as[lo + l0 + l1] * dd : T(0);
+    auto coef = [&](bool has, int e) {
+      if (!has) return T(0);
+      return PLAIN ? as[e] : as[e] * dd;
+    };
+    f[0] = coef(l0, lo);
+    f[NT] = coef(l1, lo + l0);
+    f[2 * NT] = coef(l2, lo + l0 + l1);
     f[3 * NT] = dd;
-    b[0] = u0 ? as[up] * dd : T(0);
-    b[NT] = u1 ? as[up + u0] * dd : T(0);
-    b[2 * NT] = u2 ? as[up + u0 + u1] * dd : T(0);
-    b[3 * NT] = dd / (dd + small);
+    b[0] = coef(u0, up);
+    b[NT] = coef(u1, up + u0);
+    b[2 * NT] = coef(u2, up + u0 + u1);
+    b[3 * NT] = (PLAIN ? T(1) : dd) / (dd + small);
     if (!isfinite(dd)) atomicCAS(status, 0, FCG_ERR_PIVOT);
   });
 }
@@ -498,6 +545,16 @@ __global__ void k_wave_arm(long long len, T *y, T *ze, int *ctl) {
 }
 
 // The arrays of ns systems on c's block, zeroed, and the kernels' shared-memory opt-in.
+template <class T, bool PLAIN = false>
+int allow_shared(fcg_context *c) {
+  const int smem = (TX + TY) * kSlab * (int)sizeof(T);
+  for (const void *f : {(const void *)k_wave_sweep<T, kForward, PLAIN>,
+                        (const void *)k_wave_sweep<T, kBackward, PLAIN>,
+                        (const void *)k_wave_sweep<T, kFactor, PLAIN>})
+    FCG_CUDA_TRY(c, cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  return FCG_OK;
+}
+
 template <class T>
 int allocate(fcg_context *c, int ns, DBuf &buf, Arrays<T> &A) {
   const Layout lay(c->hex.nx, c->hex.ny, c->hex.nz);
@@ -505,11 +562,9 @@ int allocate(fcg_context *c, int ns, DBuf &buf, Arrays<T> &A) {
   const size_t bytes = sizeof(T) * (size_t)ns * (size_t)(2 * rl + 2 * vl);
   FCG_CUDA_TRY(c, buf.ensure(bytes));
   FCG_CUDA_TRY(c, cudaMemsetAsync(buf.p, 0, bytes, c->stream));
-  const int smem = (TX + TY) * kSlab * (int)sizeof(T);
-  for (const void *f : {(const void *)k_wave_sweep<T, kForward>,
-                        (const void *)k_wave_sweep<T, kBackward>,
-                        (const void *)k_wave_sweep<T, kFactor>})
-    FCG_CUDA_TRY(c, cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  int rc = allow_shared<T>(c);
+  if (!rc && sizeof(T) == 8) rc = allow_shared<T, sizeof(T) == 8>(c);
+  if (rc) return rc;
   T *p = buf.as<T>();
   A.fwd = p + g;
   A.bwd = p + ns * rl + g;
@@ -528,7 +583,7 @@ struct Control {
 };
 
 // One sweep, in launches of at most kSlab planes (each a whole sweep over its planes).
-template <class T>
+template <class T, bool PLAIN = false>
 void launch(fcg_context *c, cudaStream_t st, int ns, int mode, const Arrays<T> &A, const T *in,
             T *out, const Control &w) {
   const HexBlock &h = c->hex;
@@ -539,9 +594,9 @@ void launch(fcg_context *c, cudaStream_t st, int ns, int mode, const Arrays<T> &
     const int k0 = (int)((long long)h.nz * b / slabs), k1 = (int)((long long)h.nz * (b + 1) / slabs);
     const size_t smem = (size_t)(TX + TY) * (k1 - k0) * sizeof(T);
     if (s > 0) cudaMemsetAsync(w.ctl, 0, 2 * sizeof(int), st);
-    auto kernel = mode == kForward    ? k_wave_sweep<T, kForward>
-                  : mode == kBackward ? k_wave_sweep<T, kBackward>
-                                      : k_wave_sweep<T, kFactor>;
+    auto kernel = mode == kForward    ? k_wave_sweep<T, kForward, PLAIN>
+                  : mode == kBackward ? k_wave_sweep<T, kBackward, PLAIN>
+                                      : k_wave_sweep<T, kFactor, PLAIN>;
     kernel<<<g, kThreads, smem, st>>>(h.nx, h.ny, h.nz, k0, k1, ns, A, in, out, w.ctl, w.fail,
                                       w.status, w.done, w.spin);
   }
@@ -550,7 +605,7 @@ void launch(fcg_context *c, cudaStream_t st, int ns, int mode, const Arrays<T> &
 // The factor and the records of ns systems, and armed vectors: before the first sweep of
 // a solve.  128^3, FP64: about 0.2 ms; a factor that read the CSR at every step, with every
 // hand-over through global memory, took 1.08 ms.
-template <class T>
+template <class T, bool PLAIN = false>
 int start(fcg_context *c, int ns, long long nnz, const T *a, bool dilu, T small,
           const Arrays<T> &A, const Control &w) {
   const HexBlock &h = c->hex;
@@ -559,11 +614,11 @@ int start(fcg_context *c, int ns, long long nnz, const T *a, bool dilu, T small,
   const int chunks = (lay.nlev + kPackLevels - 1) / kPackLevels;
   const int gv = grid_for(vl, c->num_sms);
   const dim3 gc(std::min(lay.ntx * lay.nty * chunks, c->num_sms * 8), ns);
-  k_wave_pack_factor<T><<<gc, kTPB, 0, c->stream>>>(h.nx, h.ny, h.nz, nnz, c->mv.ioffset,
+  k_wave_pack_factor<T, PLAIN><<<gc, kTPB, 0, c->stream>>>(h.nx, h.ny, h.nz, nnz, c->mv.ioffset,
                                                     c->mv.diag, c->tpos, a, dilu, A);
   k_wave_arm<T><<<gv, kTPB, 0, c->stream>>>(vl, A.y - g, A.ze - g, w.ctl);
-  launch<T>(c, c->stream, ns, kFactor, A, nullptr, nullptr, w);
-  k_wave_pack<T><<<gc, kTPB, 0, c->stream>>>(h.nx, h.ny, h.nz, nnz, c->mv.ioffset, c->mv.diag, a,
+  launch<T, PLAIN>(c, c->stream, ns, kFactor, A, nullptr, nullptr, w);
+  k_wave_pack<T, PLAIN><<<gc, kTPB, 0, c->stream>>>(h.nx, h.ny, h.nz, nnz, c->mv.ioffset, c->mv.diag, a,
                                              small, A, w.status, w.done);
   k_wave_arm<T><<<gv, kTPB, 0, c->stream>>>(vl, A.y - g, A.ze - g, w.ctl);
   FCG_CHECK_LAUNCH(c, "wavefront factor and records");
