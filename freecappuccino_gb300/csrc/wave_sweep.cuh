@@ -210,15 +210,19 @@ __global__ void __launch_bounds__(kThreads) __cluster_dims__(CX *CY, 1, 1)
   const int rank = (int)cluster.block_rank();
   const int tid = threadIdx.x;
   if (rank == 0 && tid == 0) {
-    const int c = atomicAdd(&ctl[BWD ? 1 : 0], 1);
-    for (int r = 0; r < CX * CY; ++r)
-      asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(peer_addr(smem_addr(&claim), r)),
-                   "r"(c)
-                   : "memory");
-    if (c == 0) ctl[BWD ? 0 : 1] = 0;  // the other sweep's counter, which is not running
+    claim = atomicAdd(&ctl[BWD ? 1 : 0], 1);
+    if (claim == 0) ctl[BWD ? 0 : 1] = 0;  // the other sweep's counter, which is not running
   }
+  // Another block's shared memory may be touched only once every block of the cluster has
+  // started, so the claim is read after this barrier, not handed out before it.  Rank 0 leaves
+  // after the last cluster.sync() below, its copy is there as long as it is read.
   cluster.sync();
-  const int c = claim / ns, sys = claim - c * ns;
+  int claimed;
+  asm volatile("ld.shared::cluster.b32 %0, [%1];"
+               : "=r"(claimed)
+               : "r"(peer_addr(smem_addr(&claim), 0))
+               : "memory");
+  const int c = claimed / ns, sys = claimed - c * ns;
   const int sc = BWD ? lay.clusters() - 1 - c : c;
   const int cx = rank % CX, cy = rank / CX;
   const int ti = (sc % lay.nsx) * CX + cx, tj = (sc / lay.nsx) * CY + cy;
