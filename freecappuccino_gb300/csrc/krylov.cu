@@ -113,6 +113,7 @@ struct KrylovState {
   bool sf_on = true;
   int sf_spin = 1 << 20;     // polls before a dependency wait gives up
   int sf_absent_row = -1;    // test hook: this row never publishes its flag
+  int test_polls = 0;        // test hook: polls of the resident form's waits (0: the default)
   bool wave_on = true;       // wavefront-tiled sweeps on lexicographic hex blocks
 };
 
@@ -1137,7 +1138,9 @@ static int launch_resident(fcg_context *c, int rows) {
   const int grid = (c->sv.nslices + warps * rows - 1) / (warps * rows);
   FCG_CUDA_TRY(c, k->rbuf.ensure(sizeof(double) * 5 * (size_t)slot_set(grid)));
   ResidentCg a{c->sv, c->n, k->sval, k->invd, k->x, k->res, k->zk, k->rtmp,
-               k->pk, k->qk, k->S, k->rbuf.as<double>(), k->trace.as<double>()};
+               k->pk, k->qk, k->S, k->rbuf.as<double>(), k->trace.as<double>(),
+               k->test_polls > 0 ? k->test_polls : kResidentPolls,
+               k->sf_absent_row < 0 ? -1 : k->sf_absent_row / 32 % (grid * warps) / warps};
   k_resident_start<<<grid_for(std::max(c->n, 5 * slot_set(grid)), c->num_sms), kTPB, 0, c->stream>>>(a, grid);
   FCG_CHECK_LAUNCH(c, "k_resident_start");
   cudaLaunchConfig_t cfg = {};
@@ -1377,6 +1380,7 @@ extern "C" int fcg_set_sweep_wait_test(fcg_context *c, int polls, int absent_row
   if (rc) return rc;
   KrylovState *k = c->ks;
   k->sf_spin = polls > 0 ? polls : (1 << 20);
+  k->test_polls = polls > 0 ? polls : 0;
   k->sf_absent_row = absent_row - 1;
   for (int i = 0; i < SK_N; ++i) {  // both values are kernel arguments of the graphs
     if (k->exec[i]) cudaGraphExecDestroy(k->exec[i]);

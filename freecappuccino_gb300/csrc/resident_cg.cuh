@@ -35,6 +35,9 @@ struct ResidentCg {
   Scal *S;
   double *slots;  // five sets (grid_sums)
   double *trace;
+  int polls;    // of a wait before it gives up
+  int quitter;  // diagnostics (fcg_set_sweep_wait_test): the block whose first wait for the
+                // update's sums counts as given up; -1: none
 };
 
 // A slot that is not written yet: a signalling NaN, which no sum of doubles results in.
@@ -120,7 +123,7 @@ __device__ __forceinline__ bool grid_sums(const ResidentCg &a, int sweep, double
     }
     // all of a lane's slots are read together, again until none is empty
     double t[M][NV];
-    int left = kResidentPolls;
+    int left = a.polls;
     bool wait;
     do {
       wait = false;
@@ -135,6 +138,7 @@ __device__ __forceinline__ bool grid_sums(const ResidentCg &a, int sweep, double
 #pragma unroll
         for (int k = 0; k < NV; ++k) wait |= __double_as_longlong(t[m][k]) == kEmpty;
     } while (wait && --left > 0);
+    if (NV == 2 && (int)blockIdx.x == a.quitter) wait = true;
 #pragma unroll
     for (int m = 0; m < M; ++m)
       if (lane + 32 * m < G) {
@@ -198,7 +202,7 @@ __device__ __forceinline__ double direction_row(const ResidentCg &a, const doubl
 
 template <int R>
 __global__ void __launch_bounds__(kResidentThreads, 1) k_resident_dpcg(ResidentCg a) {
-  __shared__ Scal sc;  // the block's copy of the scalars; block 0's goes back
+  __shared__ Scal sc;  // the block's copy of the scalars; block 0 returns the solve's
   __shared__ double sh[2][kResidentThreads / 32];
   __shared__ int failed;
   if (solve_done(a.S)) return;
@@ -275,7 +279,24 @@ __global__ void __launch_bounds__(kResidentThreads, 1) k_resident_dpcg(ResidentC
       a.p0[r] = p[i];
     }
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) *a.S = sc;
+  // Only what the sweeps change, and a status of this block's beside one that is there:
+  // another block may have given up on the last sums, which this one saw complete, and left
+  // without storing its rows.
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    Scal *S = a.S;
+    S->resl = sc.resl;
+    S->resor = sc.resor;
+    S->rsm = sc.rsm;
+    S->s0 = sc.s0;
+    S->sk = sc.sk;
+    S->bet = sc.bet;
+    S->pkapk = sc.pkapk;
+    S->alf = sc.alf;
+    S->iter = sc.iter;
+    S->done = sc.done;
+    S->converged = sc.converged;
+    if (sc.status) fail_status(S, sc.status);
+  }
 }
 
 }  // namespace

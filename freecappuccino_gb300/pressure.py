@@ -441,7 +441,8 @@ class Context:
     def set_sweep_wait_test(self, polls: int = 0, absent_row: int = 0):
         """Timeout diagnostics of the one-launch DIC/DILU sweeps: every dependency wait
         gives up after `polls` polls and row `absent_row` (1-based) never announces its
-        forward result.  (0, 0) restores normal runs."""
+        forward result; in a DPCG that runs as one launch the block of that row leaves after
+        the first sweep.  (0, 0) restores normal runs."""
         self._check(self.lib.fcg_set_sweep_wait_test(self.h, int(polls), int(absent_row)),
                     "fcg_set_sweep_wait_test")
 
