@@ -179,6 +179,7 @@ _PROTOS = {
     "fcg_lp_load": (C.c_int, [_LP, C.c_char_p]),
     "fcg_lp_set_matrix": (C.c_int, [_LP, _CTX, _vp]),
     "fcg_lp_features": (C.c_int, [_LP, _CTX, _vp]),
+    "fcg_lp_set_prepare_test": (C.c_int, [_LP, C.c_int]),
     "fcg_lp_apply": (C.c_int, [_LP, _CTX, _vp, _vp]),
     "fcg_lp_loss_grad": (C.c_int, [_LP, _CTX, _vp, _vp, C.POINTER(C.c_float), _vp]),
     "fcg_lp_train_step": (C.c_int, [_LP, _CTX, _vp, _vp, C.c_float, C.POINTER(C.c_float)]),

@@ -129,6 +129,7 @@ struct fcg_learned {
   unsigned long long hex_uid = 0;
   unsigned hex_gen = 0;
   DBuf hexval;
+  int prepare_fails = 0;  // diagnostics (fcg_lp_set_prepare_test)
 };
 
 namespace fcg {
@@ -1260,12 +1261,13 @@ int reduction_grid(const fcg_context *c) {
 int ensure_workspace(fcg_learned *Lp, fcg_context *c, bool train) {
   const size_t n = (size_t)c->n;
   if (n > Lp->ncap) {
-    Lp->ncap = n;
+    Lp->fuid = 0;  // features must be recomputed into the new buffer
+    Lp->ncap = 0;  // no size before its buffers are there
     Lp->train_cap = false;
     LP_TRY(Lp, Lp->feat.ensure(sizeof(float) * n * lp::F));
     LP_TRY(Lp, Lp->y.ensure(sizeof(float) * n));
     LP_TRY(Lp, Lp->hbuf.ensure(sizeof(__nv_bfloat16) * 3 * n * lp::C));  // h ping-pong + m
-    Lp->fuid = 0;  // features must be recomputed into the new buffer
+    Lp->ncap = n;
   }
   if (train && !Lp->train_cap) {
     const size_t nc = Lp->ncap * lp::C;
@@ -1342,10 +1344,17 @@ bool hex_on(const fcg_learned *Lp, const fcg_context *c) {
 int hex_prepare(fcg_learned *Lp, fcg_context *c) {
   if (Lp->hex_uid != c->uid || Lp->hex_gen != c->bind_gen) {
     fcg::lphex::HexGrid g;
+    Lp->hex = g;  // no mesh's until its planes are there: a failed ensure() has freed the old
+    Lp->hex_uid = 0;
     int rc = fcg::lphex::detect(c, &g);
     if (rc) return lp_fail(Lp, rc, fcg_last_error(c));
     if (g.ok) {
       const size_t bytes = sizeof(float) * fcg::lphex::value_count(g);
+      if (Lp->prepare_fails > 0) {
+        --Lp->prepare_fails;
+        Lp->hexval.release();
+        return lp_cuda(Lp, cudaErrorMemoryAllocation, "stencil value planes (planted failure)");
+      }
       LP_TRY(Lp, Lp->hexval.ensure(bytes));
       LP_TRY(Lp, cudaMemsetAsync(Lp->hexval.p, 0, bytes, c->stream));  // padding columns
     }
@@ -1373,7 +1382,9 @@ int hex_status(fcg_learned *Lp, fcg_context *c) {
 int compute_features(fcg_learned *Lp, fcg_context *c) {
   int rc = ensure_workspace(Lp, c, false);
   if (rc) return rc;
-  if (Lp->fuid != c->uid || Lp->fgen != c->bind_gen) {
+  const bool mesh_done = Lp->fuid == c->uid && Lp->fgen == c->bind_gen;
+  Lp->fuid = 0;  // the buffer is no mesh's until every step has succeeded
+  if (!mesh_done) {
     double *red = Lp->red.as<double>();
     k_lp_volsum<<<reduction_grid(c), kTPB, 0, c->stream>>>(
         c->n, c->mv.vol, red, Lp->scal.as<unsigned>() + 16, red + lp::kMaxDir * kMaxBlocks);
@@ -1920,6 +1931,12 @@ extern "C" int fcg_lp_train_step(fcg_learned *Lp, fcg_context *c, const float *r
   LP_TRY(Lp, cudaGetLastError());
   if ((rc = mark_done(Lp, c))) return rc;
   return read_loss(Lp, c, loss);
+}
+
+extern "C" int fcg_lp_set_prepare_test(fcg_learned *Lp, int fails) {
+  if (!Lp || fails < 0) return FCG_ERR_ARG;
+  Lp->prepare_fails = fails;
+  return FCG_OK;
 }
 
 extern "C" int fcg_lp_set_loss(fcg_learned *Lp, int kind) {

@@ -98,6 +98,11 @@ class LearnedPreconditioner:
         ctx._follow(a)
         self._check(self.lib.fcg_lp_set_matrix(self.h, ctx.h, _ptr(_host(a))), "fcg_lp_set_matrix")
 
+    def set_prepare_test(self, fails: int = 0):
+        """Diagnostics: the next `fails` set_matrix calls that would allocate the stencil
+        values of a hex block fail as without memory."""
+        self._check(self.lib.fcg_lp_set_prepare_test(self.h, int(fails)), "fcg_lp_set_prepare_test")
+
     def features(self, ctx: Context) -> np.ndarray:
         """Per-cell inputs of the network as (numCells, FEATURES)."""
         out = np.zeros((FEATURES, ctx.n), np.float32)

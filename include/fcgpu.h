@@ -541,6 +541,9 @@ int fcg_lp_set_matrix(fcg_learned *lp, fcg_context *ctx, const double *a);
 /* Features of the last fcg_lp_set_matrix, feature-major: out[FCG_LP_FEATURES][numCells]
  * (feature 0 is the residual input of the last forward pass). */
 int fcg_lp_features(fcg_learned *lp, fcg_context *ctx, float *out);
+/* Diagnostics of a failed fcg_lp_set_matrix: on the next `fails` meshes that form a hex
+ * block the allocation of its stencil values fails (FCG_ERR_CUDA), as without memory. */
+int fcg_lp_set_prepare_test(fcg_learned *lp, int fails);
 /* z = N(r). */
 int fcg_lp_apply(fcg_learned *lp, fcg_context *ctx, const float *r, float *z);
 /* The loss chosen by fcg_lp_set_loss (default: residual norm, |Ahat N(r) - r|^2 / |r|^2)
