@@ -217,9 +217,7 @@ __global__ void k_level_pack_factor(LevelSide lo, int ns, long long nnz,
 // in A.y; a pivot that is not finite is recorded.
 template <class T, bool BWD, bool PLAIN>
 __global__ void k_level_pack(LevelSide sd, long long ylen, int ns, long long nnz,
-                             const T *__restrict__ a, T small, Arrays<T> A, int *status,
-                             const int *done) {
-  if (__ldcg(done) != 0) return;  // the factor sweep has not run
+                             const T *__restrict__ a, T small, Arrays<T> A, int *status) {
   const long long len = 32LL * sd.chunks, elen = 32LL * sd.entries;
   FCG_GRID_STRIDE(p, len) {
     const int c = (int)(p >> 5), lane = (int)(p & 31), row = sd.row[p];
@@ -278,7 +276,8 @@ void launch(fcg_context *c, cudaStream_t st, int ns, int mode, const Arrays<T> &
 // The factor, the coefficients and armed results: before the first sweep of a solve.
 template <class T, bool PLAIN = false>
 int start(fcg_context *c, int ns, long long nnz, const T *a, bool dilu, T small,
-          const Arrays<T> &A, const Control &w) {
+          const Arrays<T> &A, const Control &solver) {
+  const Control w = solver.unstopped();
   const LevelSide &lo = c->order.lo, &up = c->order.up;
   const long long lf = 32LL * lo.chunks, lb = 32LL * up.chunks;
   const int gf = grid_for(lf, c->num_sms), gb = grid_for(lb, c->num_sms);
@@ -286,8 +285,8 @@ int start(fcg_context *c, int ns, long long nnz, const T *a, bool dilu, T small,
   k_level_pack_factor<T, PLAIN><<<gf, kTPB, 0, c->stream>>>(lo, ns, nnz, c->mv.diag, c->tpos, a, dilu, A);
   k_level_arm<T><<<ga, kTPB, 0, c->stream>>>(ns * lf, A.y, ns * lb, A.z, w.ctl);
   launch<T, PLAIN>(c, c->stream, ns, kFactor, A, PLAIN ? a : nullptr, nullptr, w);
-  k_level_pack<T, false, PLAIN><<<gf, kTPB, 0, c->stream>>>(lo, lf, ns, nnz, a, small, A, w.status, w.done);
-  k_level_pack<T, true, PLAIN><<<gb, kTPB, 0, c->stream>>>(up, lf, ns, nnz, a, small, A, w.status, w.done);
+  k_level_pack<T, false, PLAIN><<<gf, kTPB, 0, c->stream>>>(lo, lf, ns, nnz, a, small, A, w.status);
+  k_level_pack<T, true, PLAIN><<<gb, kTPB, 0, c->stream>>>(up, lf, ns, nnz, a, small, A, w.status);
   k_level_arm<T><<<ga, kTPB, 0, c->stream>>>(ns * lf, A.y, ns * lb, A.z, w.ctl);
   FCG_CHECK_LAUNCH(c, "level-order factor and coefficients");
   return FCG_OK;

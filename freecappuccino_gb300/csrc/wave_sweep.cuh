@@ -508,8 +508,7 @@ template <class T, bool PLAIN>
 __global__ void __launch_bounds__(kTPB)
     k_wave_pack(int nx, int ny, int nz, long long nnz, const int *__restrict__ ioffset,
                 const int *__restrict__ diag, const T *__restrict__ a, T small, Arrays<T> A,
-                int *status, const int *done) {
-  if (__ldcg(done) != 0) return;  // the factor sweep has not run
+                int *status) {
   const Layout lay(nx, ny, nz);
   const int s = blockIdx.y;
   const T *as = a + s * nnz, *y = A.y + s * lay.vec_len();
@@ -584,6 +583,8 @@ struct Control {
   int *ctl, *fail, *status;
   const int *done;
   int spin;
+  // the same without the solver's stop flag: the control word that stays zero
+  Control unstopped() const { return Control{ctl, fail, status, ctl + 2, spin}; }
 };
 
 // One sweep, in launches of at most kSlab planes (each a whole sweep over its planes).
@@ -607,11 +608,13 @@ void launch(fcg_context *c, cudaStream_t st, int ns, int mode, const Arrays<T> &
 }
 
 // The factor and the records of ns systems, and armed vectors: before the first sweep of
-// a solve.  128^3, FP64: about 0.2 ms; a factor that read the CSR at every step, with every
+// a solve.  A pivot that breaks down is reported whether or not the first residual has
+// already met the stop test.  128^3, FP64: about 0.2 ms; a factor that read the CSR at every step, with every
 // hand-over through global memory, took 1.08 ms.
 template <class T, bool PLAIN = false>
 int start(fcg_context *c, int ns, long long nnz, const T *a, bool dilu, T small,
-          const Arrays<T> &A, const Control &w) {
+          const Arrays<T> &A, const Control &solver) {
+  const Control w = solver.unstopped();
   const HexBlock &h = c->hex;
   const Layout lay(h.nx, h.ny, h.nz);
   const long long vl = ns * lay.vec_len(), g = Layout::guard();
@@ -623,7 +626,7 @@ int start(fcg_context *c, int ns, long long nnz, const T *a, bool dilu, T small,
   k_wave_arm<T><<<gv, kTPB, 0, c->stream>>>(vl, A.y - g, A.ze - g, w.ctl);
   launch<T, PLAIN>(c, c->stream, ns, kFactor, A, nullptr, nullptr, w);
   k_wave_pack<T, PLAIN><<<gc, kTPB, 0, c->stream>>>(h.nx, h.ny, h.nz, nnz, c->mv.ioffset, c->mv.diag, a,
-                                             small, A, w.status, w.done);
+                                             small, A, w.status);
   k_wave_arm<T><<<gv, kTPB, 0, c->stream>>>(vl, A.y - g, A.ze - g, w.ctl);
   FCG_CHECK_LAUNCH(c, "wavefront factor and records");
   return FCG_OK;
