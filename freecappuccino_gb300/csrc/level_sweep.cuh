@@ -60,10 +60,11 @@ struct Item {
 // One sweep of ns systems: the factor, y = (b - L y) d from `in` (natural order), or
 // z = y rescale - (U z) d into `out` (natural order); see wave_sweep.cuh.
 // PLAIN as there; its factor takes the CSR values in `in` and their transposes' places.
+// `in` holds in_len values a system.
 template <class T, int MODE, bool PLAIN>
 __global__ void __launch_bounds__(kThreads)
     k_level_sweep(LevelSide lo, LevelSide up, int n, int ns, Arrays<T> A,
-                  const T *__restrict__ in, const int *__restrict__ tpos, T *__restrict__ out, int *ctl, int *fail, int *status,
+                  const T *__restrict__ in, long long in_len, const int *__restrict__ tpos, T *__restrict__ out, int *ctl, int *fail, int *status,
                   const int *done, int spin, int absent) {
   using W = Word<T>;
   constexpr bool BWD = MODE == kBackward, FACTOR = MODE == kFactor;
@@ -115,7 +116,7 @@ __global__ void __launch_bounds__(kThreads)
         const long long q = 32LL * (m.off + e) + lane;
         it.dep[e] = sd.dep[q];
         it.v[e] = val[s * elen + q];
-        if (PLAIN && FACTOR && sd.src[q] >= 0) it.t[e] = in[tpos[sd.src[q]]];
+        if (PLAIN && FACTOR && sd.src[q] >= 0) it.t[e] = in[s * in_len + tpos[sd.src[q]]];
       }
     }
     if (m.row >= 0) {
@@ -124,7 +125,7 @@ __global__ void __launch_bounds__(kThreads)
       if (BWD)
         it.x = A.y[s * ylen + m.xp];
       else if (!FACTOR)
-        it.x = in[(long long)s * n + m.row];
+        it.x = in[s * in_len + m.row];
     }
   };
   Meta m0 = meta(__shfl_sync(0xffffffffu, claim(), 0));
@@ -150,7 +151,7 @@ __global__ void __launch_bounds__(kThreads)
           it.dep[e] = e0 + e < it.w ? sd.dep[q] : -1;
           it.v[e] = e0 + e < it.w ? val[s * elen + q] : T(0);
           if (PLAIN && FACTOR)
-            it.t[e] = e0 + e < it.w && sd.src[q] >= 0 ? in[tpos[sd.src[q]]] : T(0);
+            it.t[e] = e0 + e < it.w && sd.src[q] >= 0 ? in[s * in_len + tpos[sd.src[q]]] : T(0);
         }
       }
       T v[kW];
@@ -267,9 +268,10 @@ void launch(fcg_context *c, cudaStream_t st, int ns, int mode, const Arrays<T> &
             T *out, const Control &w, int absent = -1) {
   auto kernel = mode == kForward    ? k_level_sweep<T, kForward, PLAIN>
                 : mode == kBackward ? k_level_sweep<T, kBackward, PLAIN>
-                                    : k_level_sweep<T, kFactor, PLAIN>;
+                                    : k_level_sweep<T, kFactor, wave::kPlainFactor<T, PLAIN>>;
+  const long long in_len = mode == kFactor ? c->nnz : c->n;
   kernel<<<c->num_sms * kBlocksPerSM, kThreads, 0, st>>>(c->order.lo, c->order.up, c->n, ns, A, in,
-                                                         c->tpos, out, w.ctl, w.fail, w.status, w.done,
+                                                         in_len, c->tpos, out, w.ctl, w.fail, w.status, w.done,
                                                          w.spin, absent);
 }
 
@@ -282,9 +284,10 @@ int start(fcg_context *c, int ns, long long nnz, const T *a, bool dilu, T small,
   const long long lf = 32LL * lo.chunks, lb = 32LL * up.chunks;
   const int gf = grid_for(lf, c->num_sms), gb = grid_for(lb, c->num_sms);
   const int ga = grid_for(ns * std::max(lf, lb), c->num_sms);
-  k_level_pack_factor<T, PLAIN><<<gf, kTPB, 0, c->stream>>>(lo, ns, nnz, c->mv.diag, c->tpos, a, dilu, A);
+  constexpr bool PF = wave::kPlainFactor<T, PLAIN>;
+  k_level_pack_factor<T, PF><<<gf, kTPB, 0, c->stream>>>(lo, ns, nnz, c->mv.diag, c->tpos, a, dilu, A);
   k_level_arm<T><<<ga, kTPB, 0, c->stream>>>(ns * lf, A.y, ns * lb, A.z, w.ctl);
-  launch<T, PLAIN>(c, c->stream, ns, kFactor, A, PLAIN ? a : nullptr, nullptr, w);
+  launch<T, PLAIN>(c, c->stream, ns, kFactor, A, PF ? a : nullptr, nullptr, w);
   k_level_pack<T, false, PLAIN><<<gf, kTPB, 0, c->stream>>>(lo, lf, ns, nnz, a, small, A, w.status);
   k_level_pack<T, true, PLAIN><<<gb, kTPB, 0, c->stream>>>(up, lf, ns, nnz, a, small, A, w.status);
   k_level_arm<T><<<ga, kTPB, 0, c->stream>>>(ns * lf, A.y, ns * lb, A.z, w.ctl);

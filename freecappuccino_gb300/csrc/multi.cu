@@ -121,7 +121,7 @@ __global__ void k_m_factor(const int *__restrict__ rows, int count, long long nn
     float *d = d32 + (long long)k * n;
     float di = a[dg[i]];
     for (int q = io[i]; q < dg[i]; ++q)
-      di = __fmaf_rn(-(a[q] * a[tpos[q]]), d[ja[q]], di);
+      di = __fsub_rn(di, __fmul_rn(__fmul_rn(a[q], d[ja[q]]), a[tpos[q]]));
     const float inv = 1.0f / di;
     d[i] = inv;
     if (!isfinite(inv)) atomicCAS(&S->status, 0, FCG_ERR_PIVOT);

@@ -189,7 +189,9 @@ constexpr int kForward = 0, kBackward = 1, kFactor = 2;
 // a_ii - (a_ij y) a_ji (the a_ji in the backward records), y = (b - L y) d and
 // z = (y / (d + small) - U z) d with unscaled coefficients.  For BiCGStab, whose iterates on
 // a pressure system magnify an ulp by ten orders of magnitude in 50 sweeps.  Two operations
-// a neighbour instead of one and the scaling on the chain: 191 / 223 us at 128^3.
+// a neighbour instead of one and the scaling on the chain: 191 / 223 us at 128^3.  The FP32
+// factor is the PLAIN one whatever the sweeps: a_ij a_ji leaves FP32's range for coefficients
+// above 1.8e19 or below 1e-19, (a_ij y) a_ji does not.
 template <class T, int MODE, bool PLAIN>
 __global__ void __launch_bounds__(kThreads) __cluster_dims__(CX *CY, 1, 1)
     k_wave_sweep(int nx, int ny, int nz, int k0, int k1, int ns, Arrays<T> A,
@@ -547,13 +549,17 @@ __global__ void k_wave_arm(long long len, T *y, T *ze, int *ctl) {
   }
 }
 
+// Is the factor formed in the PLAIN way?
+template <class T, bool PLAIN>
+constexpr bool kPlainFactor = PLAIN || sizeof(T) == 4;
+
 // The arrays of ns systems on c's block, zeroed, and the kernels' shared-memory opt-in.
 template <class T, bool PLAIN = false>
 int allow_shared(fcg_context *c) {
   const int smem = (TX + TY) * kSlab * (int)sizeof(T);
   for (const void *f : {(const void *)k_wave_sweep<T, kForward, PLAIN>,
                         (const void *)k_wave_sweep<T, kBackward, PLAIN>,
-                        (const void *)k_wave_sweep<T, kFactor, PLAIN>})
+                        (const void *)k_wave_sweep<T, kFactor, kPlainFactor<T, PLAIN>>})
     FCG_CUDA_TRY(c, cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   return FCG_OK;
 }
@@ -601,7 +607,7 @@ void launch(fcg_context *c, cudaStream_t st, int ns, int mode, const Arrays<T> &
     if (s > 0) cudaMemsetAsync(w.ctl, 0, 2 * sizeof(int), st);
     auto kernel = mode == kForward    ? k_wave_sweep<T, kForward, PLAIN>
                   : mode == kBackward ? k_wave_sweep<T, kBackward, PLAIN>
-                                      : k_wave_sweep<T, kFactor, PLAIN>;
+                                      : k_wave_sweep<T, kFactor, kPlainFactor<T, PLAIN>>;
     kernel<<<g, kThreads, smem, st>>>(h.nx, h.ny, h.nz, k0, k1, ns, A, in, out, w.ctl, w.fail,
                                       w.status, w.done, w.spin);
   }
@@ -621,7 +627,7 @@ int start(fcg_context *c, int ns, long long nnz, const T *a, bool dilu, T small,
   const int chunks = (lay.nlev + kPackLevels - 1) / kPackLevels;
   const int gv = grid_for(vl, c->num_sms);
   const dim3 gc(std::min(lay.ntx * lay.nty * chunks, c->num_sms * 8), ns);
-  k_wave_pack_factor<T, PLAIN><<<gc, kTPB, 0, c->stream>>>(h.nx, h.ny, h.nz, nnz, c->mv.ioffset,
+  k_wave_pack_factor<T, kPlainFactor<T, PLAIN>><<<gc, kTPB, 0, c->stream>>>(h.nx, h.ny, h.nz, nnz, c->mv.ioffset,
                                                     c->mv.diag, c->tpos, a, dilu, A);
   k_wave_arm<T><<<gv, kTPB, 0, c->stream>>>(vl, A.y - g, A.ze - g, w.ctl);
   launch<T, PLAIN>(c, c->stream, ns, kFactor, A, nullptr, nullptr, w);
