@@ -965,7 +965,7 @@ const double *sliced64(const fcg_context *c) { return c->ks ? c->ks->sval : null
 // never publishes (only the row-claiming form has one).
 static bool wave_sweeps(const fcg_context *c) {
   const KrylovState *k = c->ks;
-  return k->sf_on && k->wave_on && c->hex.ok && k->sf_absent_row < 0;
+  return k->sf_on && k->wave_on && wave::applies<double>(c, 1) && k->sf_absent_row < 0;
 }
 
 static wave::Control wave_control(KrylovState *k) {

@@ -664,7 +664,8 @@ int ensure_multi(fcg_context *c, int ns) {
   {
     const char *e = std::getenv("FCG_SWEEP");
     m->sf_on = !(e && std::string(e) == "levels");
-    m->wave_on = c->hex.ok && !(e && (std::string(e) == "levels" || std::string(e) == "rows"));
+    m->wave_on = wave::applies<float>(c, ns) &&
+                 !(e && (std::string(e) == "levels" || std::string(e) == "rows"));
   }
   m->wbuf.release();
   m->lbuf.release();

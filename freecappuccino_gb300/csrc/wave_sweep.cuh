@@ -565,10 +565,33 @@ int allow_shared(fcg_context *c) {
 }
 
 template <class T>
+size_t array_bytes(const Layout &lay, int ns) {
+  return sizeof(T) * (size_t)ns * (size_t)(2 * lay.rec_len() + 2 * lay.vec_len());
+}
+
+// Does c's block take the wavefront form for ns systems?  The records hold a tile's whole
+// wavefront, nz + 22 levels of 128 columns, which on a thin block is many times its cells:
+// 12 times with two planes, 8 with two cells in i (2000 x 2000 x 2: 7.7 GB; level order,
+// level_sweep.cuh, about 1.2).  Such a block goes over to level order where that is also the
+// faster form, as its tiles, claimed row by row, number several times what the chip holds at
+// once, and where the records would take more than 4 GB.  40 ICCG sweeps, ms, wavefront /
+// level order: 512 x 512 x 2 (2048 tiles) 52 / 58; 724 x 724 x 2 (4186) 120 / 83; 2000 x 2000
+// x 2 (31250) 1548 / 244; 2 x 2000 x 2000 (5.2 GB) 346 / 240.  Below both lines the wavefront
+// form is up to twice as fast (128 x 128 x 2: 7.7 / 14.9; 2 x 1024 x 512: 53 / 83).
+template <class T>
+bool applies(const fcg_context *c, int ns) {
+  if (!c->hex.ok) return false;
+  const Layout lay(c->hex.nx, c->hex.ny, c->hex.nz);
+  const bool thin = lay.len() > 4LL * c->n;
+  return !thin || ((long long)lay.ntx * lay.nty * ns <= 16LL * c->num_sms &&
+                   array_bytes<T>(lay, ns) <= (size_t)4 << 30);
+}
+
+template <class T>
 int allocate(fcg_context *c, int ns, DBuf &buf, Arrays<T> &A) {
   const Layout lay(c->hex.nx, c->hex.ny, c->hex.nz);
   const long long g = Layout::guard(), rl = lay.rec_len(), vl = lay.vec_len();
-  const size_t bytes = sizeof(T) * (size_t)ns * (size_t)(2 * rl + 2 * vl);
+  const size_t bytes = array_bytes<T>(lay, ns);
   FCG_CUDA_TRY(c, buf.ensure(bytes));
   FCG_CUDA_TRY(c, cudaMemsetAsync(buf.p, 0, bytes, c->stream));
   int rc = allow_shared<T>(c);
