@@ -772,6 +772,10 @@ def main():
             dom = "k_mx_spmv"
             dom_bytes = 8 * nnz + 4 * (n + 1) + 8 * n  # FP32 values + int32 columns, FP32 x/y
             dom_desc = "k_mx_spmv (FP32 sliced-ELL SpMV of the scaled matrix + p.Ap, 256^3)"
+        elif "k_resident_dpcg" in prof:
+            dom = "k_resident_dpcg"  # a small system: every sweep in one launch
+            dom_bytes = spmv_bytes(n, nnz) + 24 * n  # z read beside p, both written
+            dom_desc = "k_resident_dpcg (one sweep of the cooperative DPCG launch)"
         else:
             dom = "k_cg_spmv"
             dom_bytes = spmv_bytes(n, nnz)

@@ -102,6 +102,7 @@ struct KrylovState {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   bool matrix_loaded = false;
   int last_kind = -1;
+  int last_rows = 0;  // rows a thread of the last solve's resident form, 0: the loop of kernels
   double small = (double)1e-20f;  // parameters::small (modules_allocatable.f90:27)
   int early_exit = 1;
   // one-launch triangular sweeps: the control words {forward claim counter, backward claim
@@ -1131,7 +1132,8 @@ static int resident_rows(const fcg_context *c) {
   return rows <= 2 ? rows : rows <= kResidentRows ? kResidentRows : 0;
 }
 
-static int launch_resident(fcg_context *c, int rows) {
+// `timed` (may be null): recorded right before the launch of the sweeps.
+static int launch_resident(fcg_context *c, int rows, cudaEvent_t timed = nullptr) {
   KrylovState *k = c->ks;
   const int sms = std::min(c->num_sms, kResidentBlocks);
   const int warps = std::min(kResidentThreads / 32, (c->sv.nslices + sms - 1) / sms);
@@ -1143,6 +1145,7 @@ static int launch_resident(fcg_context *c, int rows) {
                k->sf_absent_row < 0 ? -1 : k->sf_absent_row / 32 % (grid * warps) / warps};
   k_resident_start<<<grid_for(std::max(c->n, 5 * slot_set(grid)), c->num_sms), kTPB, 0, c->stream>>>(a, grid);
   FCG_CHECK_LAUNCH(c, "k_resident_start");
+  if (timed) FCG_CUDA_TRY(c, cudaEventRecord(timed, c->stream));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(32 * warps);
@@ -1312,6 +1315,7 @@ static int run_solver(fcg_context *c, int kind, const double *a, const double *s
   FCG_CUDA_TRY(c, cudaStreamSynchronize(c->stream));
   const Scal &S = *k->hS;
   k->last_kind = kind;
+  k->last_rows = rows;
   if (resor && S.iter > 0) *resor = S.res0;  // dpcg.f90:139
   if (rep) {
     rep->res0 = S.res0;
@@ -1392,8 +1396,8 @@ extern "C" int fcg_set_sweep_wait_test(fcg_context *c, int polls, int absent_row
 }
 
 // Re-opens the last solve for profiling: clears the stop flag, the reliable-update
-// flag and the sweep counters, and lifts the sweep cap.
-__global__ void k_prof_reopen(Scal *S) {
+// flag and the sweep counters, and sets the sweep cap.
+__global__ void k_prof_reopen(Scal *S, int nsw) {
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     S->done = 0;
     S->ru = 0;
@@ -1402,7 +1406,7 @@ __global__ void k_prof_reopen(Scal *S) {
     S->converged = 0;
     S->iter = 0;
     S->body_count = 0;
-    S->nsw = 0x3fffffff;
+    S->nsw = nsw;
     S->resmax = 0.0;  // never converges: every profiled sweep does its full work
   }
 }
@@ -1410,16 +1414,31 @@ __global__ void k_prof_reopen(Scal *S) {
 extern "C" int fcg_profile_sweeps(fcg_context *c, int reps, double *ms, int max_units,
                                   int *units) {
   if (!c || reps < 1) return FCG_ERR_ARG;
-  if (!c->ks || c->ks->last_kind < 0)
+  if (!c->ks || c->ks->last_kind < 0 || c->ks->bind_gen != c->bind_gen)
     return set_error(c, FCG_ERR_STATE, "fcg_profile_sweeps before any solve");
   FCG_CUDA_TRY(c, cudaSetDevice(c->device));
   KrylovState *k = c->ks;
+  if (k->last_rows) {  // one launch for all sweeps
+    if (units) *units = 1;
+    k_prof_reopen<<<1, 32, 0, c->stream>>>(k->S, reps);
+    int rc = launch_resident(c, k->last_rows, k->ev0);
+    if (rc) return rc;
+    FCG_CUDA_TRY(c, cudaEventRecord(k->ev1, c->stream));
+    int iter = 0;  // fewer than reps when the iteration breaks down
+    FCG_CUDA_TRY(c, cudaMemcpyAsync(&iter, &k->S->iter, sizeof iter, cudaMemcpyDeviceToHost,
+                                    c->stream));
+    FCG_CUDA_TRY(c, cudaStreamSynchronize(c->stream));
+    float t = 0.f;
+    FCG_CUDA_TRY(c, cudaEventElapsedTime(&t, k->ev0, k->ev1));
+    if (ms && max_units > 0) ms[0] = t / std::max(iter, 1);
+    return FCG_OK;
+  }
   const int kind = k->last_kind, nu = sweep_units(kind);
   if (units) *units = nu;
   std::vector<cudaEvent_t> ev(2 * nu);
   for (auto &e : ev) FCG_CUDA_TRY(c, cudaEventCreate(&e));
   std::vector<double> acc(nu, 0.0);
-  k_prof_reopen<<<1, 32, 0, c->stream>>>(k->S);
+  k_prof_reopen<<<1, 32, 0, c->stream>>>(k->S, 0x3fffffff);
   for (int r = 0; r < reps; ++r) {
     for (int u = 0; u < nu; ++u) {
       cudaEventRecord(ev[2 * u], c->stream);
@@ -1442,6 +1461,7 @@ extern "C" int fcg_profile_sweeps(fcg_context *c, int reps, double *ms, int max_
 
 extern "C" const char *fcg_profile_unit_name(const fcg_context *c, int unit) {
   if (!c || !c->ks || c->ks->last_kind < 0) return "";
+  if (c->ks->last_rows) return unit == 0 ? "k_resident_dpcg" : "";
   return sweep_unit_name(c->ks->last_kind, unit);
 }
 

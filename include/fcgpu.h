@@ -460,7 +460,8 @@ int fcg_dpcg_noalloc(int numCells, const int *ioffset, const int *ja, const int 
 /* Diagnostics (no reference counterpart; the reference times whole outer iterations
  * with cpu_time, main.f90:127-148).  Runs `reps` more sweeps of the last solve's method
  * kernel by kernel, outside the CUDA graph, with CUDA events around every kernel (a
- * triangular sweep counts as one unit), and writes the mean milliseconds of each unit
+ * triangular sweep counts as one unit, and so does a whole sweep of a DPCG that ran as
+ * one launch), and writes the mean milliseconds of each unit
  * to ms[0..*units-1].  It continues the last solve's iteration and so changes its
  * state: solve again before using results.  fcg_profile_unit_name names unit i. */
 int fcg_profile_sweeps(fcg_context *ctx, int reps, double *ms, int max_units, int *units);
