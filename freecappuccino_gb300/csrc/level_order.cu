@@ -55,10 +55,13 @@ int build_side(fcg_context *c, const Level &lv, bool upper, LevelSide &s, int **
   const MeshView &m = c->mv;
   const int len = lv.pad_len, chunks = len / 32, g = grid_for(len, c->num_sms);
   DBuf tmp, width, own;  // own: the side's arrays, kept with the bound mesh
-  auto fail = [&](cudaError_t e, const char *what) {
+  auto drop = [&] {
     tmp.release();
     width.release();
     own.release();
+  };
+  auto fail = [&](cudaError_t e, const char *what) {
+    drop();
     return cuda_fail(c, e, what);
   };
   cudaError_t e;
@@ -68,7 +71,7 @@ int build_side(fcg_context *c, const Level &lv, bool upper, LevelSide &s, int **
   k_widths<<<g, kTPB, 0, c->stream>>>(len, lv.pad, m.ioffset, m.diag, upper, w);
   int rc = scan_ints(c, w, wp, chunks, tmp);
   if (rc) {
-    fail(cudaSuccess, "");
+    drop();  // the scan has described its error
     return rc;
   }
   int total = 0;
