@@ -962,15 +962,18 @@ const float *scaled32(const fcg_context *c) { return c->ks ? c->ks->sval32 : nul
 const double *scale64(const fcg_context *c) { return c->ks ? c->ks->s64 : nullptr; }
 const double *sliced64(const fcg_context *c) { return c->ks ? c->ks->sval : nullptr; }
 
-// The wavefront-tiled form runs on hex blocks, unless a test hook asks for a row that
-// never publishes (only the row-claiming form has one).
+// The wavefront-tiled form runs on hex blocks, unless a test hook asks for a row that never
+// publishes and no block of another cluster waits for it (in level order each row has waits).
 static bool wave_sweeps(const fcg_context *c) {
   const KrylovState *k = c->ks;
-  return k->sf_on && k->wave_on && wave::applies<double>(c, 1) && k->sf_absent_row < 0;
+  return k->sf_on && k->wave_on && wave::applies<double>(c, 1) &&
+         (k->sf_absent_row < 0 || wave::awaited_column(c->hex, k->sf_absent_row) >= 0);
 }
 
-static wave::Control wave_control(KrylovState *k) {
-  return wave::Control{k->sf_ctl, &k->S->wait_fail, &k->S->status, &k->S->done, k->sf_spin};
+static wave::Control wave_control(const fcg_context *c) {
+  KrylovState *k = c->ks;
+  return wave::Control{k->sf_ctl, &k->S->wait_fail, &k->S->status, &k->S->done, k->sf_spin,
+                       c->hex.ok ? wave::awaited_column(c->hex, k->sf_absent_row) : -1};
 }
 
 // Factor, coefficients and armed vectors of a solve with one-launch sweeps.
@@ -980,13 +983,13 @@ static int start_sweeps(fcg_context *c, bool dilu) {
   if (!wave_sweeps(c)) {
     if (!k->lv.y && (rc = level::allocate(c, 1, k->lbuf, k->lv))) return rc;
     return dilu ? level::start<double, true>(c, 1, c->nnz, k->a, true, k->small, k->lv,
-                                             wave_control(k))
+                                             wave_control(c))
                 : level::start<double>(c, 1, c->nnz, k->a, false, k->small, k->lv,
-                                       wave_control(k));
+                                       wave_control(c));
   }
   if (!k->wv.fwd && (rc = wave::allocate(c, 1, k->wbuf, k->wv))) return rc;
-  return dilu ? wave::start<double, true>(c, 1, c->nnz, k->a, true, k->small, k->wv, wave_control(k))
-              : wave::start<double>(c, 1, c->nnz, k->a, false, k->small, k->wv, wave_control(k));
+  return dilu ? wave::start<double, true>(c, 1, c->nnz, k->a, true, k->small, k->wv, wave_control(c))
+              : wave::start<double>(c, 1, c->nnz, k->a, false, k->small, k->wv, wave_control(c));
 }
 
 template <bool PLAIN>
@@ -996,11 +999,11 @@ static void launch_sweeps(fcg_context *c, cudaStream_t st, const Level &lv, bool
   if (k->sf_on) {
     if (wave_sweeps(c)) {
       wave::launch<double, PLAIN>(c, st, 1, forward ? wave::kForward : wave::kBackward, k->wv, b,
-                                  z, wave_control(k));
+                                  z, wave_control(c));
       return;
     }
     level::launch<double, PLAIN>(c, st, 1, forward ? wave::kForward : wave::kBackward, k->lv, b,
-                                 z, wave_control(k), k->sf_absent_row);
+                                 z, wave_control(c), k->sf_absent_row);
     return;
   }
   for (int l = 0; l < lv.count; ++l) {

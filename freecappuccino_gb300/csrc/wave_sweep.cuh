@@ -196,7 +196,7 @@ template <class T, int MODE, bool PLAIN>
 __global__ void __launch_bounds__(kThreads) __cluster_dims__(CX *CY, 1, 1)
     k_wave_sweep(int nx, int ny, int nz, int k0, int k1, int ns, Arrays<T> A,
                  const T *__restrict__ in, T *out, int *ctl, int *fail, int *status,
-                 const int *done, int spin) {
+                 const int *done, int spin, int absent) {
   using W = Word<T>;
   constexpr int P = kPlanes;
   constexpr bool BWD = MODE == kBackward, FACTOR = MODE == kFactor;
@@ -253,6 +253,9 @@ __global__ void __launch_bounds__(kThreads) __cluster_dims__(CX *CY, 1, 1)
     // cell k of the upstream tile's last (backward: first) column at that row
     const long long nb = BWD ? (is_p ? 1LL : (long long)lay.ntx) : (is_p ? -1LL : -(long long)lay.ntx);
     const int ndi = is_p ? (BWD ? 0 : TX - 1) : row, ndj = is_p ? row : (BWD ? 0 : TY - 1);
+    // diagnostics: what this column leaves for other clusters never arrives
+    const int from = is_p ? ti * TX - 1 + nx * (tj * TY + row) : ti * TX + row + nx * (tj * TY - 1);
+    const bool lost = MODE == kForward && from == absent;
     const T *src = E + tile0 + nb * nlev * NT + (long long)(ndi + ndj) * NT + ndj * TX + ndi;
     constexpr int B = 8;  // cells asked for together
     int at = 0, idle = 0;
@@ -261,7 +264,7 @@ __global__ void __launch_bounds__(kThreads) __cluster_dims__(CX *CY, 1, 1)
 #pragma unroll
       for (int u = 0; u < B; ++u) {
         v[u] = W::sentinel();
-        if (mine && at + u < depth) {
+        if (mine && !lost && at + u < depth) {
           const int k = BWD ? k1 - 1 - at - u : k0 + at + u;
           v[u] = W::ld(src + (long long)k * NT);
         }
@@ -587,6 +590,16 @@ bool applies(const fcg_context *c, int ns) {
                    array_bytes<T>(lay, ns) <= (size_t)4 << 30);
 }
 
+// The column of a row that a block of another cluster waits for in the forward sweep, -1
+// when there is none.
+inline int awaited_column(const HexBlock &h, int row) {
+  if (row < 0) return -1;
+  const int i = row % h.nx, j = row / h.nx % h.ny;
+  const bool p = i % (CX * TX) == CX * TX - 1 && i + 1 < h.nx;
+  const bool q = j % (CY * TY) == CY * TY - 1 && j + 1 < h.ny;
+  return p || q ? i + h.nx * j : -1;
+}
+
 template <class T>
 int allocate(fcg_context *c, int ns, DBuf &buf, Arrays<T> &A) {
   const Layout lay(c->hex.nx, c->hex.ny, c->hex.nz);
@@ -612,6 +625,9 @@ struct Control {
   int *ctl, *fail, *status;
   const int *done;
   int spin;
+  // diagnostics (fcg_set_sweep_wait_test): the column i + nx j whose forward results never
+  // reach the clusters that wait for them; -1: none
+  int absent = -1;
   // the same without the solver's stop flag: the control word that stays zero
   Control unstopped() const { return Control{ctl, fail, status, ctl + 2, spin}; }
 };
@@ -632,7 +648,7 @@ void launch(fcg_context *c, cudaStream_t st, int ns, int mode, const Arrays<T> &
                   : mode == kBackward ? k_wave_sweep<T, kBackward, PLAIN>
                                       : k_wave_sweep<T, kFactor, kPlainFactor<T, PLAIN>>;
     kernel<<<g, kThreads, smem, st>>>(h.nx, h.ny, h.nz, k0, k1, ns, A, in, out, w.ctl, w.fail,
-                                      w.status, w.done, w.spin);
+                                      w.status, w.done, w.spin, w.absent);
   }
 }
 

@@ -416,7 +416,9 @@ int fcg_set_solver_options(fcg_context *ctx, double small, int early_exit);
  * each row waiting on the rows it reads: every wait gives up after `polls` polls (<= 0:
  * the default, about 0.4 s), and row absent_row (1-based; 0: none) never announces its
  * result in forward sweeps, so the waits of the rows that read it run out and the solve
- * returns FCG_ERR_TIMEOUT with the device still usable.  In a DPCG that runs as one launch
+ * returns FCG_ERR_TIMEOUT with the device still usable.  In the wavefront form on a hex
+ * block the row's whole (i, j) column never arrives at the blocks of another cluster (columns
+ * at a cluster's upper edge; for other rows the level order runs).  In a DPCG that runs as one launch
  * the block that holds the row gives up on the first sweep's residual sum and leaves, so the
  * other blocks' waits for the next sum run out.  (0, 0) restores normal runs. */
 int fcg_set_sweep_wait_test(fcg_context *ctx, int polls, int absent_row);

@@ -8,6 +8,7 @@ import numpy as np
 import pytest
 
 import freecappuccino_gb300 as fcg
+from freecappuccino_gb300 import _lib
 from tests.meshes import poisson_system
 from tests.test_wave_blocks import _context, box_mesh
 
@@ -73,3 +74,24 @@ def test_clusters_hand_over_in_every_slab_multi_rhs(tall):
     (x1, r1), (x2, r2) = out
     assert np.array_equal(x1, x2) and [r.iters for r in r1] == [r.iters for r in r2]
     assert all(r.converged for r in r1)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("i,j", [(31, 10), (5, 31), (31, 31)])
+def test_wait_for_another_cluster_runs_out(i, j):
+    """A column at a cluster's edge never arrives: the polling warp's wait, the waits of the
+    cells behind it and of the clusters after it end, and the next solve is as before."""
+    m = box_mesh(35, 37, 6)
+    c = _context(m)
+    a, su = c.laplacian(*poisson_system(m))
+    x0 = np.zeros(m.numCells)
+    before = {s: getattr(c, s)(a, su, x0, 0.0, 6).fi for s in ("iccg", "bicgstab")}
+    c.set_sweep_wait_test(polls=4096, absent_row=1 + i + 35 * (j + 37 * 2))
+    for solver in before:
+        with pytest.raises(_lib.FcgError) as ei:
+            getattr(c, solver)(a, su, x0, 0.0, 6)
+        assert ei.value.status == _lib.FCG_ERR_TIMEOUT and "dependency wait" in str(ei.value)
+    c.set_sweep_wait_test(0, 0)
+    for solver, fi in before.items():
+        assert np.array_equal(getattr(c, solver)(a, su, x0, 0.0, 6).fi, fi)
+    c.close()
