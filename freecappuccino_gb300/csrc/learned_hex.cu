@@ -298,17 +298,20 @@ __global__ void __launch_bounds__(kCons * 32, 1)
 
 // ---------------------------------------------------------------------------
 // The same layer with the tile product on the fifth-generation tensor cores (selected by
-// FCG_LP_HEX_MMA=tc; the mma.sync form above stays the default: this one measured 1.17
-// against 0.94 ms per layer at 256^3 -- the per-plane barrier of all consumers and the
+// FCG_LP_HEX_MMA=tc; the mma.sync form above stays the default: this one measured 1.21
+// against 0.657 ms per layer at 256^3 -- the per-plane barrier of all consumers and the
 // bank conflicts of writing the canonical operand layout, whose K-chunks of a row share
-// banks, cost more than the product it moves off the consumers).  The
+// banks, cost more than the product it moves off the consumers).  The rows are stored in the
+// fragments' channel order and the operand holds the channels' own, so a quad of lanes
+// exchanges words before its 16-byte stores, and a warp of the epilogue takes the channels of
+// two stored quarters (1.81 ms with 4-byte stores of both).  The
 // consumers write each plane's 256 rows [h; m] into a shared-memory operand in the
 // canonical K-major layout without swizzle (8-row x 16-byte core matrices; 128 bytes
 // between core matrices along K, 1024 between 8-row groups); after a barrier one thread
 // issues two 128 x 32 x 64 products (four K = 16 steps each, `tcgen05.mma.kind::f16`,
 // BF16 operands, FP32 accumulation in tensor memory) and commits them to an mbarrier.
 // While they run, the consumers aggregate the next plane into the second operand buffer;
-// then every warp reads its 32 rows x 16 columns of the accumulator (`tcgen05.ld`), adds
+// then every warp reads 16 columns of its 32 rows of the accumulator (`tcgen05.ld`), adds
 // the bias, applies the ReLU and the skip connection and stores h'.  Operands and
 // accumulators are double buffered (2 x 32 KB of shared memory, 2 x 64 of the 128 tensor
 // memory columns the block allocates).
@@ -341,6 +344,20 @@ __device__ __forceinline__ uint32_t tc_off(int r, int kc) {
 __device__ __forceinline__ uint64_t tc_desc(uint32_t addr) {
   return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)(128u >> 4) << 16) |
          ((uint64_t)(1024u >> 4) << 32) | (1ull << 46);
+}
+// Word j of the result in lane tg of a quad: word tg of lane j.
+__device__ __forceinline__ uint4 quad_transpose(uint4 w, int lane) {
+  const bool a = lane & 1, b = lane & 2;
+  auto swap = [](uint32_t &lo, uint32_t &hi, bool upper, int x) {
+    const uint32_t r = __shfl_xor_sync(0xffffffffu, upper ? lo : hi, x);
+    lo = upper ? r : lo;
+    hi = upper ? hi : r;
+  };
+  swap(w.x, w.y, a, 1);
+  swap(w.z, w.w, a, 1);
+  swap(w.x, w.z, b, 2);
+  swap(w.y, w.w, b, 2);
+  return w;
 }
 // OR of `v` over the consumer warps, which also wait for each other here (named barrier 1).
 __device__ __forceinline__ bool cons_sync_or(bool v, int nthreads) {
@@ -430,31 +447,35 @@ __global__ void __launch_bounds__(kThreads, 1)
     auto epilogue = [&](int k, int buf, int ph, int st) {
       bool ok = mbar_wait(&sm.mma_done[buf], ph & 1, abort);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      uint32_t v[16];
-      const uint32_t ta = tmem + ((uint32_t)(32 * eq) << 16) + (uint32_t)(64 * buf + 32 * et + 16 * ech);
-      asm volatile(
-          "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,"
-          "%14,%15}, [%16];"
-          : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
-            "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
-            "=r"(v[14]), "=r"(v[15])
-          : "r"(ta)
-          : "memory");
+      // the channels of the stored quarters 2 ech and 2 ech + 1: 8 i + 4 ech .. + 3
+      uint32_t v[4][4];
+      const uint32_t ta = tmem + ((uint32_t)(32 * eq) << 16) + (uint32_t)(64 * buf + 32 * et + 4 * ech);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+                     : "=r"(v[i][0]), "=r"(v[i][1]), "=r"(v[i][2]), "=r"(v[i][3])
+                     : "r"(ta + 8 * i)
+                     : "memory");
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
       const int il = erow & 15, jrow = erow >> 4;
       const int ig = i0 + il, jg = j0 + jrow;
 #pragma unroll
-      for (int c = 0; c < 16; c += 2) {
-        const int col = 16 * ech + c, at = lp::hpos(col);
-        const __nv_bfloat162 hold =
-            *reinterpret_cast<const __nv_bfloat162 *>(&sm.h[st][jrow + 1][il + 1][at]);
-        const float z0 = __uint_as_float(v[c]) + sm.b[col];
-        const float z1 = __uint_as_float(v[c + 1]) + sm.b[col + 1];
-        const __nv_bfloat162 o = __floats2bfloat162_rn(lp::bf(hold.x) + fmaxf(z0, 0.f),
-                                                       lp::bf(hold.y) + fmaxf(z1, 0.f));
+      for (int t = 0; t < 2; ++t) {
+        const int at = 8 * (2 * ech + t);  // the quarter's place in a stored row
+        const uint4 hold = *reinterpret_cast<const uint4 *>(&sm.h[st][jrow + 1][il + 1][at]);
+        uint4 out;
+        const __nv_bfloat162 *hp = reinterpret_cast<const __nv_bfloat162 *>(&hold);
+        __nv_bfloat162 *o = reinterpret_cast<__nv_bfloat162 *>(&out);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int col = 8 * i + 4 * ech + 2 * t;
+          const float z0 = __uint_as_float(v[i][2 * t]) + sm.b[col];
+          const float z1 = __uint_as_float(v[i][2 * t + 1]) + sm.b[col + 1];
+          o[i] = __floats2bfloat162_rn(lp::bf(hp[i].x) + fmaxf(z0, 0.f),
+                                       lp::bf(hp[i].y) + fmaxf(z1, 0.f));
+        }
         if (ok && ig < nx && jg < ny)
-          *reinterpret_cast<__nv_bfloat162 *>(
-              hout + (((long long)k * ny + jg) * nx + ig) * C + at) = o;
+          *reinterpret_cast<uint4 *>(hout + (((long long)k * ny + jg) * nx + ig) * C + at) = out;
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       return ok;
@@ -464,6 +485,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       const int idx = k - k0 + 1;  // ring index of plane k
       const int buf = (k - k0) & 1;
       bad = bad || !mbar_wait(&sm.full[(idx + 1) % S], ((idx + 1) / S) & 1, abort);
+      bad = __any_sync(0xffffffffu, bad);
       if (!bad) {
         const int sP = (idx - 1) % S, sC = idx % S, sN = (idx + 1) % S;
         unsigned char *ab = sm.a[buf];
@@ -492,12 +514,8 @@ __global__ void __launch_bounds__(kThreads, 1)
           const uint4 mq = lp::round8(acc);
           const int row = jr * 16 + il;
           // the operand is in channel order: pair i of quarter tg is channels 8 i + 2 tg, + 1
-          const unsigned hw[4] = {own.x, own.y, own.z, own.w}, mw[4] = {mq.x, mq.y, mq.z, mq.w};
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            *reinterpret_cast<unsigned *>(ab + tc_off(row, i) + qc / 2) = hw[i];
-            *reinterpret_cast<unsigned *>(ab + tc_off(row, 4 + i) + qc / 2) = mw[i];
-          }
+          *reinterpret_cast<uint4 *>(ab + tc_off(row, lane & 3)) = quad_transpose(own, lane);
+          *reinterpret_cast<uint4 *>(ab + tc_off(row, 4 + (lane & 3))) = quad_transpose(mq, lane);
         }
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -709,7 +727,7 @@ cudaError_t layer(const HexGrid &g, int num_sms, const __nv_bfloat16 *hin, __nv_
   const int kc = chunk_planes(ntx * nty, g.nz, num_sms);
   const dim3 grid((unsigned)(ntx * nty), (unsigned)((g.nz + kc - 1) / kc));
   // the tile product on mma.sync (default) or on tcgen05 (FCG_LP_HEX_MMA=tc: the same bits,
-  // measured 1.17 against 0.94 ms per layer at 256^3)
+  // measured 1.21 against 0.657 ms per layer at 256^3)
   const char *mm = std::getenv("FCG_LP_HEX_MMA");
   if (mm && std::strcmp(mm, "tc") == 0)
     k_lp_layer_hex_tc<<<grid, kThreads, kSmemTcBytes, st>>>(th, tv, g.nx, g.ny, g.nz, kc, hout, wl,
