@@ -160,34 +160,39 @@ __device__ __forceinline__ bool grid_sync(BCtl *ctl, long long limit) {
   return grid_sync(ctl, limit, [] {});
 }
 
-// In the last CTA of a barrier: every system's partials added in CTA order (one warp a
-// system), then fin(k, sums) by one lane.
+// In the last CTA of a barrier: every system's partials added in CTA order, then fin(k, sums)
+// by one lane.  A system has `width` lanes, a warp while eight systems or fewer are there and
+// less of one for more, so that all systems are closed at the same time: what a close costs is
+// latency (the loads, the FP64 sums' and quotients' chains), and a warp a system took 48
+// systems of 12^3 six rounds of it (90 us a sweep).
+static_assert(kMaxBatch * 4 <= kTPB, "four lanes a system at least");
 template <class F>
 __device__ __forceinline__ void sum_systems(const Split &sp, int nsys, const double *part, F &&fin) {
-  const int lane = threadIdx.x & 31;
-  for (int k = threadIdx.x >> 5; k < nsys; k += kWarps) {
-    if (sp.n[k] == 0) continue;
-    const int b0 = sp.cta_of(sp.base[k]), b1 = sp.cta_of(sp.base[k + 1] - 1);
-    const double *pk = part + (long long)k * gridDim.x * 2;
-    double v[2] = {0.0, 0.0};
-    for (int b = b0 + lane; b <= b1; b += 8 * 32) {
-      double2 t[8];  // the loads of eight partials in flight together
+  int width = 32;
+  while (width * nsys > kTPB) width >>= 1;
+  const int k = threadIdx.x / width, lane = threadIdx.x & (width - 1);
+  const bool on = k < nsys && sp.n[k] > 0;
+  const int b0 = on ? sp.cta_of(sp.base[k]) : 0, b1 = on ? sp.cta_of(sp.base[k + 1] - 1) : -1;
+  const double *pk = part + (long long)k * gridDim.x * 2;
+  double v[2] = {0.0, 0.0};
+  for (int b = b0 + lane; b <= b1; b += 8 * width) {
+    double2 t[8];  // the loads of eight partials in flight together
 #pragma unroll
-      for (int u = 0; u < 8; ++u)
-        t[u] = b + 32 * u <= b1 ? __ldcg(reinterpret_cast<const double2 *>(pk + 2 * (b + 32 * u)))
-                                : make_double2(0.0, 0.0);
+    for (int u = 0; u < 8; ++u)
+      t[u] = b + width * u <= b1
+                 ? __ldcg(reinterpret_cast<const double2 *>(pk + 2 * (b + width * u)))
+                 : make_double2(0.0, 0.0);
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        v[0] += t[u].x;
-        v[1] += t[u].y;
-      }
+    for (int u = 0; u < 8; ++u) {
+      v[0] += t[u].x;
+      v[1] += t[u].y;
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-      for (int q = 0; q < 2; ++q) v[q] += __shfl_down_sync(0xffffffffu, v[q], o);
-    if (lane == 0) fin(k, v);
   }
+  __syncwarp();
+  for (int o = width >> 1; o > 0; o >>= 1)
+#pragma unroll
+    for (int q = 0; q < 2; ++q) v[q] += __shfl_down_sync(0xffffffffu, v[q], o, width);
+  if (on && lane == 0) fin(k, v);
 }
 
 // Row sum of A x for lane `lane` of slice `slice` (FP64, slot order = CSR column order).
