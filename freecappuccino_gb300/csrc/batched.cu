@@ -594,12 +594,15 @@ extern "C" int fcg_batch_create(fcg_context *const *ctxs, int nsys, fcg_batch **
     return FCG_ERR_CUDA;
   }
   b->occ = occ;
-  // two slices a warp before another CTA an SM: two systems of 16^3 take 18 us a sweep with
-  // four CTAs an SM and 26 with six, 12 systems of 5.9 M cells 330 and 295
+  // Six slices a warp before another CTA an SM: a barrier's polls and a phase's partial sums
+  // cost more with every CTA.  100 sweeps, ms, with 1, 2, 3, 4 and 6 CTAs an SM: one system of
+  // 48^3 (2.8 slices a warp) 2.9, 3.0, 3.0, 3.2, 3.8; of 64^3 (6.7) 3.8, 3.5, 3.6, 3.9, 4.7; of
+  // 80^3 (13) 5.1, 4.3, 4.2, 4.4, 5.5; of 100^3 (26) 12.5, 8.1, 7.1, 6.9, 7.4.  12 systems of 7.9
+  // M cells in all (204) are fastest with six.
   long long slices = 0;
   for (int k = 0; k < nsys; ++k) slices += ctxs[k]->sv.nslices;
   const long long warps = (long long)b->num_sms * kWarps;
-  b->blocks_per_sm = (int)std::min<long long>(occ, 1 + slices / (2 * warps));
+  b->blocks_per_sm = (int)std::min<long long>(occ, 1 + slices / (6 * warps));
   std::memset(b->hsys, 0, sizeof(BSys) * nsys);
   if (build_items(b)) {
     fcg_batch_destroy(b);
