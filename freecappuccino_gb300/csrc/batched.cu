@@ -15,7 +15,7 @@
 //
 // What bounds it: memory latency in the phases, hidden by resident warps (the kernel is held
 // to 40 registers, six CTAs an SM), and three barriers of 2 to 5 us a sweep.  12 systems of
-// 5.9 M cells, a sweep: p 47, SpMV 147, update 101 us.  With one partial sum, block barrier
+// 7.9 M cells in all, a sweep: p 47, SpMV 147, update 101 us.  With one partial sum, block barrier
 // and ticket per item and two CTAs an SM a sweep took 811 us, and at its best setting
 // (five CTAs, items of 128 slices) 360; rows of eight loads issued together, which need 64
 // registers, 444.

@@ -362,9 +362,10 @@ __global__ void __launch_bounds__(kTPB, 5) k_cg_dot(int n, const double *__restr
 }
 
 // --- triangular sweeps, one launch per level -----------------------------------
-// The row arithmetic is explicit -- the sweeps' coefficient a_k d_i rounded, then a fused
-// multiply-add per entry; the factors' product a_k^2 or a_k a_k^T likewise -- so that every
-// kernel form (per level, one launch, wavefront tiles) gives the same bits.
+// The row arithmetic is explicit -- ICCG's coefficient a_k d_i rounded, then a fused
+// multiply-add per entry, and in its factor the product a_k^2 likewise; BiCGStab's (plain)
+// every operation rounded -- so that every kernel form (per level, one launch, wavefront
+// tiles) gives the same bits.
 // forward: z_i = b_i d_i - sum_{k<diag} (a_k d_i) z_{ja_k}        (iccg.f90:248-254)
 __global__ void k_fwd_level(const int *__restrict__ rows, int count,
                             const int *__restrict__ ioffset, const int *__restrict__ ja,

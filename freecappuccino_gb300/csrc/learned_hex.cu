@@ -24,7 +24,7 @@
 //   - each warp releases plane k's stage, and the issuing thread refills what all have.
 //
 // What bounds it: the warps' instruction issue and shared-memory wavefronts (one block an
-// SM, 57% issue activity).  A lane therefore keeps its own column's planes k-1, k and k+1 in
+// SM, 50% issue activity at 160^3).  A lane therefore keeps its own column's planes k-1, k and k+1 in
 // FP32 registers (each converted once, not three times) and takes two cells that follow
 // one another in j, each the other's neighbour: four shared-memory loads and conversions a
 // cell instead of seven.  The rows' stored channel order is that of the product's

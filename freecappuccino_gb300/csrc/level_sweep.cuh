@@ -17,9 +17,9 @@
 // the first unfinished chunk is always being worked on and the waits end; each is bounded.
 // The sentinels of one sweep's result are restored by the other sweep.
 //
-// Measured (GB300): on 93 x 81 x 77 cells less a step (588 k rows, 249 levels) the FP64
-// forward and backward sweeps take 177 and 179 us, 0.7 us a level, against about 890 us each
-// with warps claiming rows in the natural order; 40 ICCG sweeps 70.9 -> 16.9 ms.  On
+// Measured (GB300): on 93 x 81 x 77 cells less a step (532 k rows, 249 levels) the FP64
+// forward and backward sweeps take 179 us each, 0.7 us a level, against about 890 us each
+// with warps claiming rows in the natural order; 40 ICCG sweeps 70.9 -> 16.5 ms.  On
 // 150 x 140 x 130 cells, us forward: 351, 319, 310, 319 with 1, 2, 4 and 8 blocks an SM.
 #pragma once
 

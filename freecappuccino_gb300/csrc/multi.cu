@@ -64,7 +64,7 @@ struct MultiState {
   level::Arrays<float> lv{};
   bool sf_on = true;
   // the wavefront-tiled sweeps on hex blocks (wave_sweep.cuh), every system's tiles in one
-  // launch: five transport systems at 128^3 to 1e-10 take 9.4 ms, 76.3 with row-claiming
+  // launch: five transport systems at 128^3 to 1e-10 take 7.3 ms, 76.3 with row-claiming
   // sweeps in the natural order
   bool wave_on = false;
   DBuf wbuf;
